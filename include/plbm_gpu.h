@@ -49,15 +49,18 @@ extern "C" {
 
 /* ---- arithmetic of the fused step --------------------------------------
  * PLBM_F64 storage:
- *   FMA    binary64, FMA contraction allowed (default)
+ *   FMA    binary64 accuracy (default).  BGK, TRT and RR: exact integer
+ *          moments, fixed-point products, one binary64 FMA per population; the
+ *          error per step is no larger than that of the binary64 operators
+ *          with FMA contraction, which a cell outside the fixed point's range
+ *          (as for HYBRID) and the improved BGK take
  *   STRICT binary64, no contraction: the Fortran's operations in its order,
  *          bit-identical to it
- *   HYBRID BGK, TRT and RR: exact integer moments, double-float for the
- *          small terms, binary64 only for the final combination (FP64
- *          instructions per cell: BGK 18, TRT 10, RR 9, instead of 60-150).
- *          A cell with |f_0| >= 2, |f_axis| >= 1/2 or |f_diagonal| >= 1/4
- *          is evaluated with the FMA binary64 operator instead (see
- *          plbm_hybrid_range_flag)
+ *   HYBRID BGK, TRT and RR: the same step, and integer forms of the moments
+ *          and equilibria (plbm_update_macros below).  A cell out of range
+ *          (f_0 outside [0, 1), f_axis [0, 1/4), f_diagonal [0, 1/8), density
+ *          <= 1/4, or too fast) is evaluated with the binary64 operator
+ *          instead (see plbm_hybrid_range_flag)
  * Deviation storage (PLBM_F32DEV / PLBM_F16DEV):
  *   FMA    binary32 collision (default)
  *   STRICT binary64 collision on the stored deviations
@@ -257,7 +260,7 @@ int plbm_read_npy_header(const char *path, int *ndim, long long *shape, int *for
 int plbm_synchronize(plbm_grid_t *g);
 
 /* PLBM_MATH_HYBRID with PLBM_F64 storage evaluates a cell outside its range
- * (|f_0| >= 2, |f_axis| >= 1/2 or |f_diagonal| >= 1/4) with the binary64
+ * (see PLBM_MATH_* above) with the binary64
  * operator and sets a device flag: results stay valid, the flag only reports
  * that the slower path ran.  Reads it (after synchronising the device) and
  * clears it when reset != 0.  No reference counterpart (the reference has no

@@ -29,6 +29,7 @@ UNITS = [
     ("step_f64.cu", "step_f64_strict.o", ["--fmad=false", "-DPLBM_STRICT"]),
     ("step_dev.cu", "step_dev.o", ["--fmad=true"]),
     ("step_df64.cu", "step_df64.o", ["--fmad=false"]),
+    ("step_hybrid.cu", "step_hybrid.o", ["--fmad=true"]),
     ("fields.cu", "fields.o", ["--fmad=false"]),
     ("noalloc.cu", "noalloc.o", ["--fmad=false"]),
     ("batched.cu", "batched.o", ["--fmad=true"]),

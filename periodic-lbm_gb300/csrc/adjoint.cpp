@@ -68,7 +68,7 @@ void* lat(char* base, const plbm_adjoint_t* a, int i) { return base + (size_t)i 
 cudaError_t fwd_step(const plbm_adjoint_t* a, const void* src, void* dst, const CollParams& p,
                      cudaStream_t stream) {
   Sweep s{a->nx, a->ny, a->ld, src, dst, stream};
-  if (a->storage == PLBM_F64) return fma::step_pull_f64(K_BGK, s, p);
+  if (a->storage == PLBM_F64) return step_pull_f64(K_BGK, s, p);
   return step_pull_dev(ST_F32DEV, K_BGK, s, p);
 }
 

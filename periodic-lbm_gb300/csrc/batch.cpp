@@ -136,7 +136,6 @@ BatchLaunch launch_of(const plbm_batch_t* b) {
   L.tile_xy = b->d_tile_xy;
   L.tile_grid = b->d_tile_grid;
   L.nt_bgk = b->nt_bgk;
-  L.hybrid = b->math == PLBM_MATH_HYBRID;
   L.small_index = b->small_index;
   L.ngrids = b->ngrids;
   L.ntiles = b->ntiles;
@@ -306,7 +305,6 @@ extern "C" int plbm_batch_set_math(plbm_batch_t* b, int math) {
     return fail(PLBM_E_UNSUPPORTED, "PLBM_MATH_HYBRID needs PLBM_F64 storage");
   CUDA_TRY(cudaSetDevice(b->device), "cudaSetDevice");
   CUDA_TRY(cudaStreamSynchronize(b->stream), "synchronize");
-  for (BatchGrid& g : b->grids) g.hybrid = math == PLBM_MATH_HYBRID ? 1 : 0;
   b->math = math;
   return apply_schedule(b);
 }

@@ -69,12 +69,13 @@ __device__ __noinline__ void fallback_cell(const double* __restrict__ src, doubl
 
 // Process one tile of one grid for one step.  I: index type inside one grid's
 // lattice pair (32-bit when every grid's pair has fewer than 2^32 elements).
-// KIND: K_BGK or K_TRT, or -1 for the grid's own (read at run time); HY: 1
-// hybrid binary64, 0 the binary64 operator, -1 the grid's flag.  gp is the
-// grid's table entry; its relaxation constants are read where they are used
-// (through the read-only path) rather than held in registers.  (x0, y0) is
-// the tile's first cell; its TY = 2^lty rows run along y.
-template <class S, bool CG, typename I, int KIND = -1, int HY = -1>
+// KIND: K_BGK or K_TRT, or (deviation storage) -1 for the grid's own, read at
+// run time.  Binary64 grids take the fixed-point collisions of
+// hybrid.cuh in either arithmetic (their error is no larger than the binary64
+// operator's).  gp is the grid's table entry; its relaxation constants are read
+// where they are used (through the read-only path) rather than held in
+// registers.  xy is the tile's first cell; its TY = 2^lty rows run along y.
+template <class S, bool CG, typename I, int KIND>
 __device__ __forceinline__ void do_tile(const BatchGrid* __restrict__ gp, int2 xy, int parity,
                                         typename S::elem* __restrict__ base) {
   const int nx = __ldg(&gp->nx), ny = __ldg(&gp->ny), ld = __ldg(&gp->ld);
@@ -82,7 +83,6 @@ __device__ __forceinline__ void do_tile(const BatchGrid* __restrict__ gp, int2 x
   const int y = xy.y + (int)(threadIdx.x & ((1u << lty) - 1u));
   const int x = xy.x + (int)(threadIdx.x >> lty);
   if (x >= nx || y >= ny) return;
-  const int kind = KIND >= 0 ? KIND : __ldg(&gp->kind);
   const long long goff = __ldg(&gp->off);
   const I L = (I)ld, P = (I)ld * (I)nx, lat = 9 * P;
   const typename S::elem* src = base + goff + (parity ? lat : 0);
@@ -104,21 +104,15 @@ __device__ __forceinline__ void do_tile(const BatchGrid* __restrict__ gp, int2 x
 #pragma unroll
   for (int q = 0; q < 9; q++) f[q] = (typename S::real)e[q];
   if constexpr (S::ddf) {
-    if (kind == K_TRT) collide_shift<K_TRT, typename S::real>(f, gp->p);
+    if (KIND == K_TRT || (KIND < 0 && __ldg(&gp->kind) == K_TRT)) collide_shift<K_TRT, typename S::real>(f, gp->p);
     else collide_shift<K_BGK, typename S::real>(f, gp->p);
   } else {
-    if (HY > 0 || (HY < 0 && __ldg(&gp->hybrid))) {
-      bool bad = false;
-      if (kind == K_TRT) hy::trt_fma(f, gp->ht, bad);
-      else hy::bgk_fma(f, gp->hp, bad);
-      if (bad) {  // outside the hybrid range: the binary64 operator on the same inputs
-        fallback_cell<CG>(src, dst, x, y, gp);
-        return;
-      }
-    } else if (kind == K_TRT) {
-      collide_ref<K_TRT>(f, gp->p);
-    } else {
-      collide_ref<K_BGK>(f, gp->p);
+    bool bad = false;
+    if constexpr (KIND == K_TRT) hy::trt_fma(f, gp->ht, bad);
+    else hy::bgk_fma(f, gp->hp, bad);
+    if (bad) {  // outside the fixed point's range: the binary64 operator on the same inputs
+      fallback_cell<CG>(src, dst, x, y, gp);
+      return;
     }
   }
   const I o = c0 + y0;
@@ -126,14 +120,15 @@ __device__ __forceinline__ void do_tile(const BatchGrid* __restrict__ gp, int2 x
   for (int q = 0; q < 9; q++) S::store(dst, (size_t)((I)q * P + o), f[q]);
 }
 
-// Tiles t = blockIdx.x, blockIdx.x + gridDim.x, ...; the grid of tile t is
-// tile_grid[t], its first cell tile_xy[t] (both precomputed).
-template <class S, bool CG, typename I>
+// Tiles t = first + blockIdx.x, + gridDim.x, ... below last, all of one
+// collision kind; the grid of tile t is tile_grid[t], its first cell
+// tile_xy[t] (both precomputed).
+template <class S, bool CG, typename I, int KIND>
 __device__ __forceinline__ void sweep(const BatchGrid* __restrict__ grids, const int2* __restrict__ tile_xy,
-                                      const int* __restrict__ tile_grid, int ntiles, int parity,
+                                      const int* __restrict__ tile_grid, int first, int last, int parity,
                                       typename S::elem* base) {
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x)
-    do_tile<S, CG, I>(grids + __ldg(tile_grid + t), __ldg(tile_xy + t), parity, base);
+  for (int t = first; t < last; t += gridDim.x)
+    do_tile<S, CG, I, KIND>(grids + __ldg(tile_grid + t), __ldg(tile_xy + t), parity, base);
 }
 
 // Grid-wide barrier with a bounded wait.  Returns false when the wait ran out
@@ -169,53 +164,79 @@ __device__ __forceinline__ bool barrier(Ctrl* ctrl, int step) {
   return ok != 0;
 }
 
-template <class S, typename I>
-__global__ void __launch_bounds__(kBatchMaxThreads) k_batch_persistent(const BatchGrid* __restrict__ grids,
-                                                                      const int2* __restrict__ tile_xy,
-                                                                      const int* __restrict__ tile_grid,
-                                                                      int ntiles, int nsteps, int parity0,
-                                                                      typename S::elem* base, Ctrl* ctrl) {
+// CTAs per SM the kernels are compiled for: binary64 1024 resident threads (64
+// registers), deviation storage 1536 (40; uncapped the persistent kernel takes
+// 52 and runs 48 grids at 0.062 ms per step instead of 0.057).
+template <class S>
+constexpr int batch_min_blocks(int max_threads) {
+  return (S::ddf ? 1536 : 1024) / max_threads;
+}
+
+// Binary64: the BGK tiles (t < nt_bgk) and the TRT tiles run in loops of their own, each
+// compiled for its kind: with the kind read per tile inside one loop the
+// binary64 kernel took 114 registers, 2 CTAs of 256 per SM (48 grids, 4.0 M
+// cells: 0.204 ms per step against 0.163).  A CTA that ends its BGK
+// tiles early goes on with its share of the TRT tiles: tile t of either kind
+// belongs to CTA t mod gridDim.x.  Deviation storage reads the kind per tile:
+// both collisions fit in the registers of one, and the shared loads are the
+// faster form (0.0566 ms per step, 0.0571 in two loops).
+template <class S, typename I, int MAXT>
+__global__ void __launch_bounds__(MAXT, batch_min_blocks<S>(MAXT))
+    k_batch_persistent(const BatchGrid* __restrict__ grids, const int2* __restrict__ tile_xy,
+                       const int* __restrict__ tile_grid, int nt_bgk, int ntiles, int nsteps, int parity0,
+                       typename S::elem* base, Ctrl* ctrl) {
+  const int r = nt_bgk % (int)gridDim.x;
+  const int trt0 = nt_bgk + ((int)blockIdx.x >= r ? (int)blockIdx.x - r : (int)blockIdx.x + (int)gridDim.x - r);
   for (int s = 0; s < nsteps; s++) {
-    sweep<S, true, I>(grids, tile_xy, tile_grid, ntiles, (parity0 + s) & 1, base);
+    const int parity = (parity0 + s) & 1;
+    if constexpr (S::ddf) {
+      sweep<S, true, I, -1>(grids, tile_xy, tile_grid, blockIdx.x, ntiles, parity, base);
+    } else {
+      sweep<S, true, I, K_BGK>(grids, tile_xy, tile_grid, blockIdx.x, nt_bgk, parity, base);
+      sweep<S, true, I, K_TRT>(grids, tile_xy, tile_grid, trt0, ntiles, parity, base);
+    }
     if (s + 1 < nsteps && !barrier(ctrl, s)) return;
   }
 }
 
+// Per-step launch over the tiles of one collision kind (tile t0 + blockIdx.x),
+// compiled for that kind alone: the binary64 BGK tiles take 64 registers and
+// the TRT tiles 72.  One kernel for both kinds needed far more registers than
+// either (97 for the earlier forms, 80 under a cap with spills, 20.9k MLUPS on
+// the 512-grid batch against 24.5k split by kind).
+template <class S, typename I, int KIND, int MAXT, int MINB>
+__global__ void __launch_bounds__(MAXT, MINB) k_batch_kind(const BatchGrid* __restrict__ grids,
+                                                          const int2* __restrict__ tile_xy,
+                                                          const int* __restrict__ tile_grid, int t0, int parity,
+                                                          typename S::elem* base) {
+  const int t = t0 + (int)blockIdx.x;
+  do_tile<S, false, I, KIND>(grids + __ldg(tile_grid + t), __ldg(tile_xy + t), parity, base);
+}
+
+// Per-step launch over all tiles, for deviation storage in CTAs other than 128
+// threads (48 grids, 256 threads: 0.0645 ms per step, 0.070 as a launch per
+// kind).
 template <class S, typename I>
 __global__ void __launch_bounds__(kBatchMaxThreads) k_batch_step(const BatchGrid* __restrict__ grids,
                                                                 const int2* __restrict__ tile_xy,
-                                                                const int* __restrict__ tile_grid, int ntiles,
-                                                                int parity, typename S::elem* base) {
-  sweep<S, false, I>(grids, tile_xy, tile_grid, ntiles, parity, base);
+                                                                const int* __restrict__ tile_grid, int parity,
+                                                                typename S::elem* base) {
+  const int t = (int)blockIdx.x;
+  do_tile<S, false, I, -1>(grids + __ldg(tile_grid + t), __ldg(tile_xy + t), parity, base);
 }
 
-// Per-step launch of 128-thread CTAs over the tiles of one collision kind
-// (tile t0 + blockIdx.x), compiled for that kind and arithmetic alone with
-// MINB resident CTAs per SM: the binary64 hybrid BGK tiles (bgk_fma) take 64
-// registers (8 CTAs) and the TRT tiles (trt_fma) 72 (7).  One kernel for both
-// kinds needed far more registers than either (97 for the earlier forms, 80
-// under a cap with spills, 20.9k MLUPS on the 512-grid batch against 24.5k
-// split by kind).
-template <class S, typename I, int KIND, int HY, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_batch_kind(const BatchGrid* __restrict__ grids,
-                                                         const int2* __restrict__ tile_xy,
-                                                         const int* __restrict__ tile_grid, int t0, int parity,
-                                                         typename S::elem* base) {
-  const int t = t0 + (int)blockIdx.x;
-  do_tile<S, false, I, KIND, HY>(grids + __ldg(tile_grid + t), __ldg(tile_xy + t), parity, base);
-}
-
-template <class S, typename I, int HY>
+template <class S, typename I, int MAXT>
 cudaError_t launch_kinds(const BatchLaunch& L, int parity) {
   typedef typename S::elem E;
   E* base = static_cast<E*>(L.base);
   const int ntrt = L.ntiles - L.nt_bgk;
+  constexpr int trt_blocks = MAXT == 128 ? 7 : batch_min_blocks<S>(MAXT);
   if (L.nt_bgk > 0)
-    k_batch_kind<S, I, K_BGK, HY, 8><<<L.nt_bgk, 128, 0, L.stream>>>(L.grids, L.tile_xy, L.tile_grid,
-                                                                                    0, parity, base);
+    k_batch_kind<S, I, K_BGK, MAXT, MAXT == 128 ? 8 : batch_min_blocks<S>(MAXT)>
+        <<<L.nt_bgk, L.threads, 0, L.stream>>>(L.grids, L.tile_xy, L.tile_grid, 0, parity, base);
   if (ntrt > 0)
-    k_batch_kind<S, I, K_TRT, HY, 7><<<ntrt, 128, 0, L.stream>>>(L.grids, L.tile_xy, L.tile_grid, L.nt_bgk, parity,
-                                                                 base);
+    k_batch_kind<S, I, K_TRT, MAXT, trt_blocks>
+        <<<ntrt, L.threads, 0, L.stream>>>(L.grids, L.tile_xy, L.tile_grid, L.nt_bgk, parity, base);
   return cudaGetLastError();
 }
 
@@ -234,19 +255,21 @@ cudaError_t launch_batch(const BatchLaunch& L, int nsteps, int parity0) {
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_batch_persistent<S, I>, L.grids, L.tile_xy, L.tile_grid, L.ntiles, nsteps,
-                              parity0, base, ctrl);
+    auto kernel = !S::ddf && L.threads <= 256 ? k_batch_persistent<S, I, 256> : k_batch_persistent<S, I, kBatchMaxThreads>;
+    return cudaLaunchKernelEx(&cfg, kernel, L.grids, L.tile_xy, L.tile_grid, L.nt_bgk, L.ntiles, nsteps, parity0,
+                              base, ctrl);
   }
-  // one tile per CTA; 128-thread CTAs run one kernel per collision kind
+  // one tile per CTA
   for (int s = 0; s < nsteps; s++) {
     const int parity = (parity0 + s) & 1;
     cudaError_t e;
-    if (L.threads == 128) {
-      e = (!S::ddf && L.hybrid) ? launch_kinds<S, I, 1>(L, parity) : launch_kinds<S, I, 0>(L, parity);
-    } else {
-      k_batch_step<S, I><<<L.ntiles, L.threads, 0, L.stream>>>(L.grids, L.tile_xy, L.tile_grid, L.ntiles, parity,
-                                                               base);
+    if (L.threads <= 128 && (!S::ddf || L.threads == 128)) {
+      e = launch_kinds<S, I, 128>(L, parity);
+    } else if constexpr (S::ddf) {
+      k_batch_step<S, I><<<L.ntiles, L.threads, 0, L.stream>>>(L.grids, L.tile_xy, L.tile_grid, parity, base);
       e = cudaGetLastError();
+    } else {
+      e = L.threads <= 256 ? launch_kinds<S, I, 256>(L, parity) : launch_kinds<S, I, kBatchMaxThreads>(L, parity);
     }
     if (e != cudaSuccess) return e;
   }
@@ -263,16 +286,20 @@ cudaError_t launch_batch_i(const BatchLaunch& L, int nsteps, int parity0) {
 
 size_t batch_ctrl_bytes() { return sizeof(Ctrl); }
 
+namespace {
+template <class S, typename I>
+cudaError_t persistent_ctas(int threads, int* per_sm) {
+  auto kernel = !S::ddf && threads <= 256 ? k_batch_persistent<S, I, 256> : k_batch_persistent<S, I, kBatchMaxThreads>;
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, threads, 0);
+}
+}  // namespace
+
 cudaError_t batch_max_ctas(int storage, int threads, int small_index, int* per_sm) {
   if (storage == ST_F64)
-    return small_index ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_batch_persistent<StoreF64, uint32_t>,
-                                                                     threads, 0)
-                       : cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_batch_persistent<StoreF64, size_t>,
-                                                                     threads, 0);
-  return small_index ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_batch_persistent<StoreF32Dev, uint32_t>,
-                                                                   threads, 0)
-                     : cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_batch_persistent<StoreF32Dev, size_t>,
-                                                                   threads, 0);
+    return small_index ? persistent_ctas<StoreF64, uint32_t>(threads, per_sm)
+                       : persistent_ctas<StoreF64, size_t>(threads, per_sm);
+  return small_index ? persistent_ctas<StoreF32Dev, uint32_t>(threads, per_sm)
+                     : persistent_ctas<StoreF32Dev, size_t>(threads, per_sm);
 }
 
 cudaError_t batch_run(int storage, const BatchLaunch& L, int nsteps, int parity0) {

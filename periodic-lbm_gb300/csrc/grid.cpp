@@ -458,7 +458,7 @@ cudaError_t fused_step(plbm_grid_t* g, const void* a, void* b, const CollParams&
     // collision; strict: the reference's two passes, expression by expression
     if (g->math == PLBM_MATH_FMA && !(g->kind == PLBM_BGKI && g->ld != g->ny))
       return fma::step_scheme_f64(g->streaming, g->kind, s, g->dt, p);
-    if (g->math == PLBM_MATH_HYBRID) return step_scheme_hybrid(g->streaming, g->kind, s, g->dt, p);
+    if (g->math == PLBM_MATH_HYBRID) return step_scheme_fixed(g->streaming, g->kind, s, g->dt, p, true);
     cudaError_t e = stream_scheme(g, s);
     if (e != cudaSuccess) return e;
     return g->math == PLBM_MATH_STRICT ? strict::collide_f64(g->kind, s, p) : fma::collide_f64(g->kind, s, p);
@@ -476,8 +476,8 @@ cudaError_t fused_step(plbm_grid_t* g, const void* a, void* b, const CollParams&
   }
   switch (g->math) {
     case PLBM_MATH_STRICT: return strict::step_pull_f64(g->kind, s, p);
-    case PLBM_MATH_HYBRID: return step_pull_df64(g->kind, s, p);
-    default: return fma::step_pull_f64(g->kind, s, p);
+    case PLBM_MATH_HYBRID: return step_pull_fixed(g->kind, s, p, true);
+    default: return step_pull_f64(g->kind, s, p);
   }
 }
 
@@ -857,8 +857,8 @@ extern "C" int plbm_launch_step(int storage, int math, int kind, int nx, int ny,
     if (math == PLBM_MATH_HYBRID && kind == PLBM_BGKI)
       return fail(PLBM_E_UNSUPPORTED, "PLBM_MATH_HYBRID is not offered for collide_bgk_improved");
     if (math == PLBM_MATH_STRICT) e = strict::step_pull_f64(kind, s, p);
-    else if (math == PLBM_MATH_HYBRID) e = step_pull_df64(kind, s, p);
-    else e = fma::step_pull_f64(kind, s, p);
+    else if (math == PLBM_MATH_HYBRID) e = step_pull_fixed(kind, s, p, true);
+    else e = step_pull_f64(kind, s, p);
   } else if (storage == PLBM_F32DEV || storage == PLBM_F16DEV) {
     if (kind == PLBM_BGKI) return fail(PLBM_E_UNSUPPORTED, "collide_bgk_improved needs PLBM_F64 storage");
     e = step_pull_dev(storage, kind, s, p);

@@ -21,19 +21,29 @@
 //
 //   BGK (bgk_fma, src/collision_bgk.F90:58-71 with the equilibrium of
 //     src/fvm_bardow.F90:99-126): the nonlinear terms of all nine populations
-//     are integer combinations of three double-float products.
+//     are integer combinations of three products j_a u_b.
 //   TRT (trt_fma, incompressible, src/collision_trt.F90:98-152): symmetric
 //     and antisymmetric brackets of each pair, joined by one exact 128-bit
-//     product r D (r = lambda_d / lambda_e scaled); |j|^2 and jx jy exact.
+//     product r D (r = lambda_d / lambda_e scaled).
 //   RR (rr_fma, src/collision_regularized.F90:72-194): the six merged Hermite
-//     coefficients of the equilibrium and the regularized part in
-//     double-float, taken to the fixed point at half scale.
+//     coefficients of the equilibrium and the regularized part.
+// The products are fixed-point (mulh64, recip_fixed of fixed.cuh), each within
+// ~2^-60: the error of a collision is the nine final roundings, below that of
+// the straight binary64 operators (random cells at |u| <= 0.05, against 113-bit
+// arithmetic, norm-wise: BGK 1.3e-16 against 1.4e-16, TRT 1.3e-16 / 1.4e-16, RR
+// 1.2e-16 / 1.2e-16; largest error of a population over its weight 3e-16 against
+// 1e-15).  Products in double-float, with conversions to and from the fixed
+// point, erred by 1e-15 of the weight at |u| = 0.05 and took 720 (BGK) and 1173
+// (RR) instructions per cell instead of 644 and 894; at 8192^2 a BGK step took
+// 1.762 ms instead of 1.700, RR 2.60 instead of 2.34, the plugin's BGK step 2.08
+// instead of 1.85.
 // Each states its range; a cell outside it reports `bad`, and the kernels then
 // evaluate that cell with the binary64 operator of the reference instead.
 // Populations stored shifted (h = f - w, the plugin's storage) take the same
 // forms with DH = sum h = rho - 1 in place of R in the linear brackets.
 #pragma once
-#include "df64.cuh"
+#include <math.h>
+#include "fixed.cuh"
 
 namespace plbm {
 namespace hy {
@@ -175,8 +185,14 @@ DF_HD double fixed_to_double_any(int64_t T) {
 
 constexpr int64_t kOne = (int64_t)1 << kScale;  // 1.0 in fixed point
 
-
-
+DF_HD int64_t shl(int64_t a, int s) { return (int64_t)((uint64_t)a << s); }
+// a / 2^s rounded to nearest (ties toward +infinity).
+DF_HD int64_t round_shr(int64_t a, int s) { return (a + ((int64_t)1 << (s - 1))) >> s; }
+// |a| / 2^32, within one unit.
+DF_HD uint32_t uabs_hi(int64_t a) {
+  const int32_t h = (int32_t)(a >> 32);
+  return (uint32_t)(h ^ (h >> 31));
+}
 
 // a k / 2^64 rounded to nearest, for the constant corrections below
 // (|a| < 2^63, |k| < 2^31; a's low 32 bits do not take part).
@@ -288,7 +304,7 @@ DF_HD df64 fixed_to_df_x(int64_t T) {
 // of all nine populations are integer combinations of three products,
 //   A = 1.5 jx^2 / rho,  B = 1.5 jy^2 / rho,  X = 4.5 jx jy / rho,
 //   C_0 = -(A + B),  C_x = 2A - B,  C_y = 2B - A,  C_(+-diag) = 2 (A + B) +- 2X,
-// evaluated in double-float and taken to the fixed point once each.  With
+// evaluated as fixed-point products and taken to 2^-59 once each.  With
 // every F_q and the C images integers, 36 (w_q T_q - F_q) is an integer, and
 //   rest      4 Y_0,  Y_0 = 4 (R + C_0) - 9 F_0
 //   axis      4 Y_q,  Y_q = T_q - 9 F_q
@@ -380,6 +396,67 @@ DF_HD int64_t to_fixed_nonneg(double d, bool& bad) {
   return r;
 }
 
+// The nine populations in the fixed point.  Unshifted: exact for
+// 2^-7 <= f below the limits of bgk_fma (a biased exponent in [1016, EMAX], one
+// shift of the significand); a cell with a smaller value goes through
+// to_fixed_nonneg out of line, one with a value past the limits is reported
+// before any further work (a 2048^2 lattice of density 3 in FMA arithmetic then
+// takes the 624 us per BGK step of the binary64 kernel; 702 when reported last).  SHIFTED: the significand at 2^62, negated in
+// one's complement, shifted right with half a unit added: rounded to nearest,
+// an error whose mean does not depend on the sign of h.  (Rounded toward zero,
+// h of the sign of c.u shrinks and |J| is damped by ~1e-16 per step, 2e-12 in u
+// over 10,000 plugin steps; rounded toward -infinity, one instruction pair
+// fewer, the error of one step is 1.4 times as large.)
+PLBM_NOINLINE void load_fixed_slow(const double* f, int64_t* F) {
+  bool b = false;  // stays false: the caller has checked the limits
+  F[0] = to_fixed_nonneg<1022>(f[0], b);
+  for (int q = 1; q < 5; q++) F[q] = to_fixed_nonneg<1020>(f[q], b);
+  for (int q = 5; q < 9; q++) F[q] = to_fixed_nonneg<1019>(f[q], b);
+}
+template <bool SHIFTED>
+DF_HD void load_fixed(const double (&f)[9], int64_t (&F)[9], bool& bad) {
+  bool odd = false;
+#pragma unroll
+  for (int q = 0; q < 9; q++) {
+    const uint64_t u = df::d2u(f[q]);
+    const uint32_t H = (uint32_t)(u >> 32), L = (uint32_t)u;
+    const uint32_t mh = (H & 0xFFFFFu) | 0x100000u;
+    if constexpr (SHIFTED) {
+      const uint32_t e = (H >> 20) & 0x7FFu;
+      odd |= e > (q == 0 ? 1021u : (q < 5 ? 1019u : 1018u));
+      const uint32_t rs = 1026u - e < 63u ? 1026u - e : 63u;
+      const uint64_t n = ((((uint64_t)mh << 32) | L) << 10) ^ (uint64_t)((int64_t)u >> 63);
+      // (rs > 32, |h| < 2^-28: rounded toward -infinity)
+      F[q] = (int64_t)(n + (1u << ((rs - 1u) & 31u))) >> rs;
+    } else {
+      const uint32_t sh = (H >> 20) - 1016u;  // a set sign bit makes this large
+      odd |= sh > (q == 0 ? 6u : (q < 5 ? 4u : 3u));
+      F[q] = (int64_t)(((uint64_t)funnel_l(L, mh, sh & 31u) << 32) | (uint64_t)(L << (sh & 31u)));
+    }
+  }
+  if constexpr (SHIFTED) {
+    bad |= odd;
+  } else if (odd) {
+    // past a limit, negative or not finite (a set sign bit included in H >> 20)
+#pragma unroll
+    for (int q = 0; q < 9; q++)
+      bad |= (uint32_t)(df::d2u(f[q]) >> 52) > (q == 0 ? 1022u : (q < 5 ? 1020u : 1019u));
+    if (bad) return;
+    double g[9];
+    int64_t G[9];
+#pragma unroll
+    for (int q = 0; q < 9; q++) g[q] = f[q];
+    load_fixed_slow(g, G);
+#pragma unroll
+    for (int q = 0; q < 9; q++) F[q] = G[q];
+  }
+}
+
+// rho outside [2^-2 + 2^-27, 4): the reciprocal's range.
+DF_HD bool rho_out_of_range(int64_t R) { return (uint32_t)((uint64_t)R >> 32) - 0x2000001u > 0x1dfffffeu; }
+constexpr int32_t kTurn02 = 26843545;    // 0.2 2^27
+constexpr uint32_t kTurn06 = 644245094;  // 0.6 2^30
+
 // SHIFTED: f holds h = f - w (the plugin's storage, sim/sim.F90:131).  The
 // linear brackets then take DH = sum h = rho - 1 in place of R (the w terms
 // cancel) and the nonlinear terms rho = 1 + DH.  Range for h: |h_0| < 1/2,
@@ -390,44 +467,22 @@ DF_HD int64_t to_fixed_nonneg(double d, bool& bad) {
 // a bias that leaves the odd moments alone (to_fixed_signed).
 template <bool SHIFTED = false>
 DF_HD void bgk_fma(double (&f)[9], const BgkParams& p, bool& bad) {
-  using namespace df;
   int64_t F[9];
-  if constexpr (SHIFTED) {
-    F[0] = to_fixed_signed<1021>(f[0], bad);
-    F[1] = to_fixed_signed<1019>(f[1], bad);
-    F[2] = to_fixed_signed<1019>(f[2], bad);
-    F[3] = to_fixed_signed<1019>(f[3], bad);
-    F[4] = to_fixed_signed<1019>(f[4], bad);
-    F[5] = to_fixed_signed<1018>(f[5], bad);
-    F[6] = to_fixed_signed<1018>(f[6], bad);
-    F[7] = to_fixed_signed<1018>(f[7], bad);
-    F[8] = to_fixed_signed<1018>(f[8], bad);
-  } else {
-    F[0] = to_fixed_nonneg<1022>(f[0], bad);
-    F[1] = to_fixed_nonneg<1020>(f[1], bad);
-    F[2] = to_fixed_nonneg<1020>(f[2], bad);
-    F[3] = to_fixed_nonneg<1020>(f[3], bad);
-    F[4] = to_fixed_nonneg<1020>(f[4], bad);
-    F[5] = to_fixed_nonneg<1019>(f[5], bad);
-    F[6] = to_fixed_nonneg<1019>(f[6], bad);
-    F[7] = to_fixed_nonneg<1019>(f[7], bad);
-    F[8] = to_fixed_nonneg<1019>(f[8], bad);
-  }
+  load_fixed<SHIFTED>(f, F, bad);
+  if (bad) return;
   // R: the zeroth moment of the stored values (rho, or DH when shifted)
   const int64_t R = (((F[5] + F[7]) + (F[6] + F[8])) + ((F[1] + F[3]) + (F[2] + F[4]))) + F[0];
   const int64_t d57 = F[5] - F[7], d86 = F[8] - F[6];
   const int64_t JX = (d57 + d86) + (F[1] - F[3]);
   const int64_t JY = (d57 - d86) + (F[2] - F[4]);
   const int64_t Rrho = SHIFTED ? R + kOne : R;
-  if constexpr (SHIFTED) bad |= Rrho < (kOne >> 2);
-  const df64 s15 = mul_f(recip(fixed_to_df_x(Rrho)), 1.5f);  // 1.5 / rho
-  const df64 jx = fixed_to_df_x(JX), jy = fixed_to_df_x(JY);
-  const df64 A = mul_lz(sqr_lz(jx), s15);
-  const df64 B = mul_lz(sqr_lz(jy), s15);
-  const df64 X = mul_f_lz(mul_lz(mul_lz(jx, jy), s15), 3.0f);
-  bad |= !(A.hi + B.hi < 0.2f);  // NaN (R = 0) fails too
-  const int64_t Ai = df_to_fixed_xu(A), Bi = df_to_fixed_xu(B), Xi = df_to_fixed_xu(X);
+  const int64_t I = recip_fixed(Rrho);                 // 2^61 / rho
+  const int64_t jx = shl(JX, 5), jy = shl(JY, 5);      // 2^64 j
+  const int64_t U = mulh64(jx, I), V = mulh64(jy, I);  // 2^61 u
+  const int64_t Ai = round_shr(3 * mulh64(jx, U), 3), Bi = round_shr(3 * mulh64(jy, V), 3);
+  const int64_t Xi = round_shr(9 * mulh64(jx, V), 3);
   const int64_t AB = Ai + Bi;
+  bad |= rho_out_of_range(Rrho) | ((int32_t)(AB >> 32) >= kTurn02);
   f[0] = fma_d(p.c4, fixed_to_double_tr(4 * (R - AB) - 9 * F[0] + scale_2m64(R, p.mass_k)), f[0]);
   const int64_t cx = R + (2 * Ai - Bi), cy = R + (2 * Bi - Ai);
   const int64_t jx3 = 3 * JX, jy3 = 3 * JY;
@@ -444,64 +499,50 @@ DF_HD void bgk_fma(double (&f)[9], const BgkParams& p, bool& bad) {
   f[8] = fma_d(p.c1, fixed_to_double_tr(dm - sm - 36 * F[8]), f[8]);
 }
 
-// Recursive-regularized constants (rr_fma).
+// Recursive-regularized constant (rr_fma): 1 - omega at scale 2^63.
 struct RrParams {
-  double w[3];   // 4/9, 1/9, 1/36 in binary64
-  df64 wdf[3];   // the same as double-float
-  df64 omb;      // 1 - omega
-  df64 third;    // 1/3
+  int64_t omb;
 };
-
+inline RrParams rr_fma_params(double omega) {
+  RrParams r;
+  const double b = ldexp(1.0 - omega, 63);
+  r.omb = b >= 0x1p63 ? INT64_MAX : (b <= -0x1p63 ? INT64_MIN + 1 : (int64_t)llrint(b));
+  return r;
+}
 
 // Recursive regularized collision with one binary64 FMA per population.
 // f'_q = w_q (T_q + N_q), T_q = R + 3 c_q.J, N_q the Hermite combination of
 // the six merged coefficients M = rho (u product) + (1 - omega) a of the
 // second-, third- and fourth-order Hermite terms (the equilibrium's and the
-// regularized non-equilibrium part's, src/collision_regularized.F90:99-194),
-// with a_xx = (3 Pxx - R)/3 - jx ux, a_yy alike, a_xy = Pxy - jx uy from exact
-// integer moments and the recursive third and fourth orders; so with the
-// fixed-point images of
-// M / 2 (exact halving in double-float), h.., every 36 (f'_q - f_q) / k_q is
-// an integer bracket:
-//   rest      4 Y_0,  Y_0 = 4 R - 9 F_0 - 12 (hxx + hyy) + 18 hxxyy
-//   axis      4 Y_q,  Y_q = T_q - 9 F_q + 6 hxx - 3 hyy - 9 hxxyy -+ 9 hyyx  (x; y alike)
-//   diagonal    Y_q,  Y_q = T_q - 36 F_q + 6 (hxx + hyy) + 18 hxxyy
-//                            +- 18 hxy +- 18 (hxxy +- hyyx)
+// regularized non-equilibrium part's, src/collision_regularized.F90:99-194).
+// With b = 1 - omega, B = b a and q = rho u u the recursion of the higher
+// orders closes over the merged coefficients:
+//   3 B_xx = b (3 P_xx - R - 3 q_xx), B_xy = b (P_xy - q_xy),  M = q + B,
+//   M_xxy  = u_y M_xx + 2 u_x B_xy,   M_yyx = u_x M_yy + 2 u_y B_xy,
+//   M_xxyy = u_y M_xxy + u_x (M_yyx - u_x q_yy)
+// (a_xxyy of the reference is u_x a_yyx + u_y a_xxy), fifteen fixed-point
+// products in all (mulh64) on exact integer moments.  Taken to integers of
+// 2^-59 once each as X3 = 1.5 M_xx, Y3 = 1.5 M_yy, K = 9 M_xy, GY = 4.5 M_xxy,
+// GX = 4.5 M_yyx and G = 4.5 M_xxyy, every 36 (f'_q - f_q) / k_q is an integer
+// bracket:
+//   rest      4 Y_0,  Y_0 = 4 R - 9 F_0 - 4 (X3 + Y3) + 2 G
+//   axis      4 Y_q,  Y_q = T_q - 9 F_q + 2 X3 - Y3 - G -+ GX  (x; y alike)
+//   diagonal    Y_q,  Y_q = T_q - 36 F_q + 2 (X3 + Y3) + 2 G +- K +- 2 (GY +- GX)
 // and f'_q = fma(k_q RN(1/36), Y_q 2^-59, f_q).  The Hermite parts of the
 // brackets sum to zero with the weights exactly, as T_q - 36 w_q F_q does; the
 // reference's binary64 weights (sums 1 - 2^-54) take 2^-54 of the mass and
 // momentum each step, restored by p.mass_k / p.mom_k (bgk_fma_params at
-// omega = 1).  Range as bgk_fma, and sum |M / 2| < 0.1 (checked on the
-// binary32 heads): then the Hermite parts add at most 3, 0.9 and 1.8 (units of
-// 2^59) to the rest, axis and diagonal brackets, which stay below 13 x 2^59.
+// omega = 1).  Range as bgk_fma, q_xx + q_yy < 0.2 and sum |M / 2| < 0.1: then the Hermite parts
+// add at most 3, 0.9 and 1.8 (units of 2^59) to the rest, axis and diagonal
+// brackets, which stay below 13 x 2^59, and no product's operand leaves int64.
 template <bool SHIFTED = false>
 DF_HD void rr_fma(double (&f)[9], const RrParams& r, const BgkParams& p, bool& bad) {
-  using namespace df;
   int64_t F[9];
-  if constexpr (SHIFTED) {
-    F[0] = to_fixed_signed<1021>(f[0], bad);
-    F[1] = to_fixed_signed<1019>(f[1], bad);
-    F[2] = to_fixed_signed<1019>(f[2], bad);
-    F[3] = to_fixed_signed<1019>(f[3], bad);
-    F[4] = to_fixed_signed<1019>(f[4], bad);
-    F[5] = to_fixed_signed<1018>(f[5], bad);
-    F[6] = to_fixed_signed<1018>(f[6], bad);
-    F[7] = to_fixed_signed<1018>(f[7], bad);
-    F[8] = to_fixed_signed<1018>(f[8], bad);
-  } else {
-    F[0] = to_fixed_nonneg<1022>(f[0], bad);
-    F[1] = to_fixed_nonneg<1020>(f[1], bad);
-    F[2] = to_fixed_nonneg<1020>(f[2], bad);
-    F[3] = to_fixed_nonneg<1020>(f[3], bad);
-    F[4] = to_fixed_nonneg<1020>(f[4], bad);
-    F[5] = to_fixed_nonneg<1019>(f[5], bad);
-    F[6] = to_fixed_nonneg<1019>(f[6], bad);
-    F[7] = to_fixed_nonneg<1019>(f[7], bad);
-    F[8] = to_fixed_nonneg<1019>(f[8], bad);
-  }
+  load_fixed<SHIFTED>(f, F, bad);
+  if (bad) return;
   const int64_t s57 = F[5] + F[7], s68 = F[6] + F[8];
   const int64_t sd = s57 + s68;
-  const int64_t R = ((s57 + s68) + ((F[1] + F[3]) + (F[2] + F[4]))) + F[0];
+  const int64_t R = (sd + ((F[1] + F[3]) + (F[2] + F[4]))) + F[0];
   const int64_t d57 = F[5] - F[7], d86 = F[8] - F[6];
   const int64_t JX = (d57 + d86) + (F[1] - F[3]);
   const int64_t JY = (d57 - d86) + (F[2] - F[4]);
@@ -509,53 +550,43 @@ DF_HD void rr_fma(double (&f)[9], const RrParams& r, const BgkParams& p, bool& b
   const int64_t PYY3 = 3 * ((F[2] + F[4]) + sd) - R;
   const int64_t PXY = s57 - s68;
   const int64_t Rrho = SHIFTED ? R + kOne : R;
-  if constexpr (SHIFTED) bad |= Rrho < (kOne >> 2);
-  const df64 rho = fixed_to_df_x(Rrho);
-  const df64 inv = recip(rho);
-  const df64 jx = fixed_to_df_x(JX), jy = fixed_to_df_x(JY);
-  const df64 ux = mul_lz(jx, inv), uy = mul_lz(jy, inv);
-  // rho times the velocity products: rho ux^2 = jx ux, rho ux uy = jx uy, ...
-  const df64 qxx = mul_lz(jx, ux), qyy = mul_lz(jy, uy), qxy = mul_lz(jx, uy);
-  const df64 uxx = sqr_lz(ux), uyy = sqr_lz(uy), uxy = mul_lz(ux, uy);
-  const df64 axx = sub_lz(mul_lz(fixed_to_df_x(PXX3), r.third), qxx);
-  const df64 ayy = sub_lz(mul_lz(fixed_to_df_x(PYY3), r.third), qyy);
-  const df64 axy = sub_lz(fixed_to_df_x(PXY), qxy);
-  const df64 axxy = add_lz(mul_pow2(mul_lz(ux, axy), 2.0f), mul_lz(uy, axx));
-  const df64 ayyx = add_lz(mul_pow2(mul_lz(uy, axy), 2.0f), mul_lz(ux, ayy));
-  const df64 axxyy =
-      sub_lz(sub_lz(sub_lz(mul_pow2(add_lz(mul_lz(ux, ayyx), mul_lz(uy, axxy)), 2.0f), mul_lz(uxx, ayy)),
-                    mul_lz(uyy, axx)),
-             mul_pow2(mul_lz(uxy, axy), 4.0f));
-  // M / 2 = (rho (u product) + (1 - omega) a) / 2
-  const df64 mxx = mul_pow2(add_lz(qxx, mul_lz(r.omb, axx)), 0.5f);
-  const df64 myy = mul_pow2(add_lz(qyy, mul_lz(r.omb, ayy)), 0.5f);
-  const df64 mxy = mul_pow2(add_lz(qxy, mul_lz(r.omb, axy)), 0.5f);
-  const df64 mxxy = mul_pow2(add_lz(mul_lz(qxx, uy), mul_lz(r.omb, axxy)), 0.5f);
-  const df64 myyx = mul_pow2(add_lz(mul_lz(qyy, ux), mul_lz(r.omb, ayyx)), 0.5f);
-  const df64 mxxyy = mul_pow2(add_lz(mul_lz(qxx, uyy), mul_lz(r.omb, axxyy)), 0.5f);
-  // sum |M / 2| < 0.1 (NaN fails too)
-  bad |= !(fabsf(mxx.hi) + fabsf(myy.hi) + fabsf(mxy.hi) + fabsf(mxxy.hi) + fabsf(myyx.hi) + fabsf(mxxyy.hi) < 0.1f);
-  const int64_t hxx = df_to_fixed_xu(mxx), hyy = df_to_fixed_xu(myy), hxy = df_to_fixed_xu(mxy);
-  const int64_t hxxy = df_to_fixed_xu(mxxy), hyyx = df_to_fixed_xu(myyx), hxxyy = df_to_fixed_xu(mxxyy);
-  f[0] = fma_d(p.c4, fixed_to_double_tr(4 * R - 9 * F[0] - 12 * (hxx + hyy) + 18 * hxxyy + scale_2m64(R, p.mass_k)),
-               f[0]);
-  const int64_t jx3 = 3 * JX + scale_2m64(JX, p.mom_k), jy3 = 3 * JY + scale_2m64(JY, p.mom_k);
-  const int64_t nx_ = R + 6 * hxx - 3 * hyy - 9 * hxxyy, nxo = 9 * hyyx;
-  const int64_t ny_ = R + 6 * hyy - 3 * hxx - 9 * hxxyy, nyo = 9 * hxxy;
-  f[1] = fma_d(p.c4, fixed_to_double_tr(nx_ + jx3 - nxo - 9 * F[1]), f[1]);
-  f[3] = fma_d(p.c4, fixed_to_double_tr(nx_ - jx3 + nxo - 9 * F[3]), f[3]);
-  f[2] = fma_d(p.c4, fixed_to_double_tr(ny_ + jy3 - nyo - 9 * F[2]), f[2]);
-  f[4] = fma_d(p.c4, fixed_to_double_tr(ny_ - jy3 + nyo - 9 * F[4]), f[4]);
-  // diagonal pairs without the momentum correction (the axis pairs carry it):
-  // q=5 (+x,+y): +18 hxy + 18 (hxxy + hyyx); q=7: +18 hxy - 18 (hxxy + hyyx)
-  // q=6 (-x,+y): -18 hxy + 18 (hxxy - hyyx); q=8: -18 hxy - 18 (hxxy - hyyx)
-  const int64_t dsum = R + 6 * (hxx + hyy) + 18 * hxxyy;
-  const int64_t sp = 3 * (JX + JY), sm = 3 * (JY - JX);
-  const int64_t a5 = 18 * (hxy + hxxy + hyyx), a6 = 18 * (hxy - hxxy + hyyx);
-  f[5] = fma_d(p.c1, fixed_to_double_tr(dsum + sp + a5 - 36 * F[5]), f[5]);
-  f[7] = fma_d(p.c1, fixed_to_double_tr(dsum - sp + 36 * hxy - a5 - 36 * F[7]), f[7]);
-  f[6] = fma_d(p.c1, fixed_to_double_tr(dsum + sm - a6 - 36 * F[6]), f[6]);
-  f[8] = fma_d(p.c1, fixed_to_double_tr(dsum - sm - 36 * hxy + a6 - 36 * F[8]), f[8]);
+  const int64_t I = recip_fixed(Rrho);                                                 // 2^61 / rho
+  const int64_t jx = shl(JX, 5), jy = shl(JY, 5);                                      // 2^64 j
+  const int64_t U = mulh64(jx, I), V = mulh64(jy, I);                                  // 2^61 u
+  const int64_t qxx = mulh64(jx, U), qyy = mulh64(jy, V), qxy = mulh64(jx, V);         // 2^61 rho u u
+  const int64_t u = shl(U, 2), v = shl(V, 2);                                          // 2^63 u
+  // 3 M_xx, 3 M_yy, M_xy and B_xy, scale 2^60
+  const int64_t mxx = round_shr(3 * qxx, 1) + mulh64(shl(PXX3, 2) - 3 * qxx, r.omb);
+  const int64_t myy = round_shr(3 * qyy, 1) + mulh64(shl(PYY3, 2) - 3 * qyy, r.omb);
+  const int64_t bxy = mulh64(shl(PXY, 2) - qxy, r.omb);
+  const int64_t mxy = round_shr(qxy, 1) + bxy;
+  // 3 M_xxy, 3 M_yyx, 3 M_xxyy, scale 2^62
+  const int64_t mx3 = shl(mxx, 3), my3 = shl(myy, 3), b3 = shl(bxy, 3);
+  const int64_t mxxy = mulh64(mx3, v) + 6 * mulh64(b3, u);
+  const int64_t myyx = mulh64(my3, u) + 6 * mulh64(b3, v);
+  const int64_t mxxyy = mulh64(shl(mxxy, 1), v) + mulh64(shl(myyx - 3 * mulh64(shl(qyy, 2), u), 1), u);
+  // sum |M / 2| < 0.1, on the leading words
+  const uint32_t sum2 = uabs_hi(mxx) + uabs_hi(myy) + 3 * uabs_hi(mxy);  // scale 6 2^28
+  const uint32_t sum3 = uabs_hi(mxxy) + uabs_hi(myyx) + uabs_hi(mxxyy);  // scale 6 2^30
+  bad |= rho_out_of_range(Rrho) | ((int32_t)((qxx + qyy) >> 34) >= kTurn02) | (sum2 >= kTurn06 / 4) |
+         (4 * sum2 + sum3 >= kTurn06);
+  const int64_t X3 = round_shr(mxx, 2), Y3 = round_shr(myy, 2), K = round_shr(9 * mxy, 1);
+  const int64_t GY = round_shr(3 * mxxy, 4), GX = round_shr(3 * myyx, 4), G = round_shr(3 * mxxyy, 4);
+  f[0] = fma_d(p.c4, fixed_to_double_tr(4 * (R - X3 - Y3) - 9 * F[0] + 2 * G + scale_2m64(R, p.mass_k)), f[0]);
+  const int64_t jx3 = 3 * JX, jy3 = 3 * JY;
+  const int64_t ax = jx3 + scale_2m64(JX, p.mom_k) - GX, ay = jy3 + scale_2m64(JY, p.mom_k) - GY;
+  const int64_t cx = R + 2 * X3 - Y3 - G, cy = R + 2 * Y3 - X3 - G;
+  f[1] = fma_d(p.c4, fixed_to_double_tr(cx + ax - 9 * F[1]), f[1]);
+  f[3] = fma_d(p.c4, fixed_to_double_tr(cx - ax - 9 * F[3]), f[3]);
+  f[2] = fma_d(p.c4, fixed_to_double_tr(cy + ay - 9 * F[2]), f[2]);
+  f[4] = fma_d(p.c4, fixed_to_double_tr(cy - ay - 9 * F[4]), f[4]);
+  // diagonal pairs without the momentum correction (the axis pairs carry it)
+  const int64_t c = R + 2 * (X3 + Y3 + G), dp = c + K, dm = c - K;
+  const int64_t sp = (jx3 + jy3) + 2 * (GY + GX), sm = (jy3 - jx3) + 2 * (GY - GX);
+  f[5] = fma_d(p.c1, fixed_to_double_tr(dp + sp - 36 * F[5]), f[5]);
+  f[7] = fma_d(p.c1, fixed_to_double_tr(dp - sp - 36 * F[7]), f[7]);
+  f[6] = fma_d(p.c1, fixed_to_double_tr(dm + sm - 36 * F[6]), f[6]);
+  f[8] = fma_d(p.c1, fixed_to_double_tr(dm - sm - 36 * F[8]), f[8]);
 }
 
 // (a b) / 2^sh, 0 < sh < 64, of the exact 128-bit product, rounded to nearest
@@ -629,32 +660,14 @@ DF_HD int64_t abs64(int64_t v) { return v < 0 ? -v : v; }
 template <bool SHIFTED = false>
 DF_HD void trt_fma(double (&f)[9], const TrtFmaParams& p, bool& bad) {
   int64_t F[9];
-  if constexpr (SHIFTED) {
-    F[0] = to_fixed_signed<1021>(f[0], bad);
-    F[1] = to_fixed_signed<1019>(f[1], bad);
-    F[2] = to_fixed_signed<1019>(f[2], bad);
-    F[3] = to_fixed_signed<1019>(f[3], bad);
-    F[4] = to_fixed_signed<1019>(f[4], bad);
-    F[5] = to_fixed_signed<1018>(f[5], bad);
-    F[6] = to_fixed_signed<1018>(f[6], bad);
-    F[7] = to_fixed_signed<1018>(f[7], bad);
-    F[8] = to_fixed_signed<1018>(f[8], bad);
-  } else {
-    F[0] = to_fixed_nonneg<1022>(f[0], bad);
-    F[1] = to_fixed_nonneg<1020>(f[1], bad);
-    F[2] = to_fixed_nonneg<1020>(f[2], bad);
-    F[3] = to_fixed_nonneg<1020>(f[3], bad);
-    F[4] = to_fixed_nonneg<1020>(f[4], bad);
-    F[5] = to_fixed_nonneg<1019>(f[5], bad);
-    F[6] = to_fixed_nonneg<1019>(f[6], bad);
-    F[7] = to_fixed_nonneg<1019>(f[7], bad);
-    F[8] = to_fixed_nonneg<1019>(f[8], bad);
-  }
+  load_fixed<SHIFTED>(f, F, bad);
+  if (bad) return;
   const int64_t R = (((F[5] + F[7]) + (F[6] + F[8])) + ((F[1] + F[3]) + (F[2] + F[4]))) + F[0];
   const int64_t d57 = F[5] - F[7], d86 = F[8] - F[6];
   const int64_t JX = (d57 + d86) + (F[1] - F[3]);
   const int64_t JY = (d57 - d86) + (F[2] - F[4]);
-  const int64_t X2 = mul_shr(JX, JX, kScale), Y2 = mul_shr(JY, JY, kScale), XY = mul_shr(JX, JY, kScale);
+  const int64_t jx = shl(JX, 5), jy = shl(JY, 5);  // 2^64 j
+  const int64_t X2 = round_shr(mulh64(jx, jx), 5), Y2 = round_shr(mulh64(jy, jy), 5), XY = round_shr(mulh64(jx, jy), 5);
   const int64_t J2 = X2 + Y2;
   const int64_t sx = 9 * (F[1] + F[3]) - 2 * R - 6 * X2 + 3 * Y2, dx = 3 * (F[1] - F[3]) - 2 * JX;
   const int64_t sy = 9 * (F[2] + F[4]) - 2 * R - 6 * Y2 + 3 * X2, dy = 3 * (F[2] - F[4]) - 2 * JY;

@@ -12,15 +12,14 @@ constexpr int kBatchMaxThreads = 512;
 // One grid of a batch, as the kernels see it.
 struct alignas(16) BatchGrid {
   CollParams p;       // relaxation parameters (grid's omega / TRT magic)
-  hy::BgkParams hp;   // the same for the hybrid binary64 BGK (bgk_fma)
+  hy::BgkParams hp;   // the same for the fixed-point binary64 BGK (bgk_fma)
   hy::TrtFmaParams ht;  // ... and TRT (trt_fma)
   long long off;      // element offset of lattice A; lattice B follows it
   int nx, ny, ld;
   int kind;           // K_BGK or K_TRT
   int ty;             // tile rows along y; tile columns = threads / ty
-  int hybrid;         // binary64 grid in hybrid arithmetic
   int lty;            // log2(ty)
-  int pad;
+  int pad[2];
 };
 
 hy::BgkParams hybrid_bgk_params(double omega);
@@ -32,7 +31,6 @@ struct BatchLaunch {
   const int* tile_grid;    // device, grid index of each tile
   int ngrids, ntiles;
   int nt_bgk;              // tiles [0, nt_bgk) belong to BGK grids, the rest to TRT grids
-  int hybrid;              // binary64 grids in hybrid arithmetic (batch-wide)
   int threads, ctas;       // ctas: persistent mode only (per-step: one CTA per tile)
   int persistent;          // 1: one cooperative launch for all steps
   int small_index;         // every grid's lattice pair has < 2^32 elements

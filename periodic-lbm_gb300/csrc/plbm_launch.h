@@ -53,15 +53,22 @@ PLBM_DECLARE_F64(fma)
 PLBM_DECLARE_F64(strict)
 #undef PLBM_DECLARE_F64
 
-// binary64 storage, hybrid arithmetic (hybrid.cuh), YFast pull, BGK, TRT and RR
-cudaError_t step_pull_df64(int kind, const Sweep& s, const CollParams& p);
-// The plugin step (shifted binary64, x-fastest, collide then push) in the
-// hybrid arithmetic (BGK, TRT, RR).
-cudaError_t step_push_hybrid(int kind, const Sweep& s, const CollParams& p);
+// binary64 storage, fixed-point arithmetic (hybrid.cuh), YFast pull, BGK, TRT
+// and RR: the step of PLBM_MATH_HYBRID (report: a cell out of range sets the
+// range flag) and of PLBM_MATH_FMA.
+cudaError_t step_pull_fixed(int kind, const Sweep& s, const CollParams& p, bool report);
+// The plugin step (shifted binary64, x-fastest, collide then push) in the same
+// arithmetic (BGK, TRT, RR).
+cudaError_t step_push_fixed(int kind, const Sweep& s, const CollParams& p, bool report);
 // A finite-volume / finite-difference streaming scheme (stencil form) fused
-// with the hybrid collision (BGK, TRT, RR).
-cudaError_t step_scheme_hybrid(int scheme, int kind, const Sweep& s, double dt, const CollParams& p);
+// with the fixed-point collision (BGK, TRT, RR).
+cudaError_t step_scheme_fixed(int scheme, int kind, const Sweep& s, double dt, const CollParams& p, bool report);
 cudaError_t hybrid_range_flag(int* flag, int reset);
+// The PLBM_MATH_FMA step: the fixed point for BGK, TRT and RR, the binary64
+// kernel for the improved BGK.
+inline cudaError_t step_pull_f64(int kind, const Sweep& s, const CollParams& p) {
+  return kind == K_BGKI ? fma::step_pull_f64(kind, s, p) : step_pull_fixed(kind, s, p, false);
+}
 
 // Deviation storage (storage = 1 float, 2 half), binary32 arithmetic.
 cudaError_t step_pull_dev(int storage, int kind, const Sweep& s, const CollParams& p);
@@ -70,7 +77,7 @@ cudaError_t collide_dev(int storage, int kind, const Sweep& s, const CollParams&
 cudaError_t step_push_dev(int storage, int kind, const Sweep& s, const CollParams& p);
 // Deviation storage with the collision in binary64 (math 1, BGK/TRT/RR),
 // compensated binary32 (math 2, BGK) or double-float (math 3, BGK)
-// arithmetic; compiled in step_df64.cu.
+// arithmetic; step_df64.cu.
 cudaError_t step_pull_dev_hi(int storage, int math, int kind, const Sweep& s, const CollParams& p);
 
 // Field kernels (fields.cu).  layout: 0 = YFast (src/), 1 = XFast (sim/).

@@ -74,7 +74,11 @@ cudaError_t push_step(const PluginSim* s, int from, const CollParams& p) {
   Sweep sw{s->nx, s->ny, s->ld, s->f[from], s->f[1 - from], s->stream};
   if (s->storage != PLBM_F64) return step_push_dev(s->storage, s->kind, sw, p);
   if (s->math == PLBM_MATH_STRICT) return strict::step_push_shift_f64(s->kind, sw, p);
-  if (s->math == PLBM_MATH_HYBRID) return step_push_hybrid(s->kind, sw, p);
+  if (s->math == PLBM_MATH_HYBRID) return step_push_fixed(s->kind, sw, p, true);
+  // BGK: the fixed point's error is below the binary64 operator's, which rounds
+  // rho = 1 + sum h to 2^-53; the binary64 TRT and RR work on sum h alone and keep
+  // more digits of small h than 2^-59.
+  if (s->kind == K_BGK) return step_push_fixed(s->kind, sw, p, false);
   return fma::step_push_shift_f64(s->kind, sw, p);
 }
 

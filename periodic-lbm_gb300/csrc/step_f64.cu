@@ -181,16 +181,31 @@ cudaError_t launch_step(int kind, const Sweep& s, const CollParams& p) {
   if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   const double* a = static_cast<const double*>(s.src);
   double* b = static_cast<double*>(s.dst);
+#define PLBM_STEP(K) k_step<L, K, SHIFT, PUSH><<<(unsigned)blocks, bs, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, p)
+#ifdef PLBM_STRICT
   switch (kind) {
-    case K_BGK: k_step<L, K_BGK, SHIFT, PUSH><<<(unsigned)blocks, bs, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, p); break;
-    case K_TRT: k_step<L, K_TRT, SHIFT, PUSH><<<(unsigned)blocks, bs, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, p); break;
-    case K_RR: k_step<L, K_RR, SHIFT, PUSH><<<(unsigned)blocks, bs, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, p); break;
+    case K_BGK: PLBM_STEP(K_BGK); break;
+    case K_TRT: PLBM_STEP(K_TRT); break;
+    case K_RR: PLBM_STEP(K_RR); break;
     case K_BGKI:
-      if (SHIFT) return cudaErrorNotSupported;
-      k_step<L, K_BGKI, false, PUSH><<<(unsigned)blocks, bs, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, p);
+      if constexpr (SHIFT) return cudaErrorNotSupported;
+      else PLBM_STEP(K_BGKI);
       break;
     default: return cudaErrorInvalidValue;
   }
+#else
+  // BGK (both layouts), TRT and RR (unshifted) in FMA arithmetic run in the fixed
+  // point (step_hybrid.cu)
+  if constexpr (SHIFT) {
+    if (kind == K_TRT) PLBM_STEP(K_TRT);
+    else if (kind == K_RR) PLBM_STEP(K_RR);
+    else return cudaErrorNotSupported;
+  } else {
+    if (kind != K_BGKI) return cudaErrorInvalidValue;
+    PLBM_STEP(K_BGKI);
+  }
+#endif
+#undef PLBM_STEP
   return cudaGetLastError();
 }
 
