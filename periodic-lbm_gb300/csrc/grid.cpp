@@ -454,11 +454,13 @@ cudaError_t stream_scheme(const plbm_grid_t* g, const Sweep& s) {
 cudaError_t fused_step(plbm_grid_t* g, const void* a, void* b, const CollParams& p) {
   Sweep s{g->nx, g->ny, g->ld, a, b, g->stream};
   if (g->streaming != PLBM_STREAM_LBM) {
-    // FMA arithmetic: one fused kernel, the scheme in stencil form then the
-    // collision; strict: the reference's two passes, expression by expression
-    if (g->math == PLBM_MATH_FMA && !(g->kind == PLBM_BGKI && g->ld != g->ny))
-      return fma::step_scheme_f64(g->streaming, g->kind, s, g->dt, p);
-    if (g->math == PLBM_MATH_HYBRID) return step_scheme_fixed(g->streaming, g->kind, s, g->dt, p, true);
+    // FMA and hybrid arithmetic: one fused kernel, in the fixed point (the
+    // improved BGK: the scheme in stencil form then the binary64 collision);
+    // strict: the reference's two passes, expression by expression
+    if (g->math != PLBM_MATH_STRICT && g->kind != PLBM_BGKI)
+      return step_scheme_fixed(g->streaming, g->kind, s, g->dt, p, g->math == PLBM_MATH_HYBRID);
+    if (g->math == PLBM_MATH_FMA && g->ld == g->ny)
+      return fma::step_scheme_f64(g->streaming, s, g->dt, p);
     cudaError_t e = stream_scheme(g, s);
     if (e != cudaSuccess) return e;
     return g->math == PLBM_MATH_STRICT ? strict::collide_f64(g->kind, s, p) : fma::collide_f64(g->kind, s, p);

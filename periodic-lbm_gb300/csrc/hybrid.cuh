@@ -242,6 +242,16 @@ DF_HD float i2f(int32_t v) {
 
 PLBM_NOINLINE double fixed_to_double_any_slow(int64_t T) { return fixed_to_double_any(T); }
 
+// int64 v > 0 (scale 2^SCALE) -> binary64 rounded to nearest, ties away from
+// zero (10 instructions; the carry of the rounding runs into the exponent).
+template <int SCALE>
+DF_HD double pos_fixed_to_double(int64_t v) {
+  const int lz = clz64((uint64_t)v);
+  const uint64_t n = ((uint64_t)v << lz) + 0x400u;  // bit 63 set, or 2^64 -> 0 on a carry
+  const uint64_t m = (n >> 11) | ((uint64_t)(n < 0x400u) << 53);
+  return df::u2d(((uint64_t)(uint32_t)(1085 - SCALE - lz) << 52) + m);
+}
+
 // int64 fixed point (scale 2^59) -> binary64 for |T| >= 2^32 (others out of
 // line, exactly): the magnitude taken in one's complement (a negative T comes
 // out 2^-59 smaller in magnitude) and truncated to 53 bits.  The error is below
@@ -465,11 +475,10 @@ constexpr uint32_t kTurn06 = 644245094;  // 0.6 2^30
 // |JX +- JY| < 3/4 and |Y_0| < 10.3, |Y_axis| < 4.9, |Y_diag| < 6.75 (units of
 // 2^59).  Small h are rounded to the fixed point with ties toward +infinity,
 // a bias that leaves the odd moments alone (to_fixed_signed).
-template <bool SHIFTED = false>
-DF_HD void bgk_fma(double (&f)[9], const BgkParams& p, bool& bad) {
-  int64_t F[9];
-  load_fixed<SHIFTED>(f, F, bad);
-  if (bad) return;
+//
+// bgk_brackets: Y of the fixed-point populations F.
+template <bool SHIFTED>
+DF_HD void bgk_brackets(const int64_t (&F)[9], const BgkParams& p, int64_t (&Y)[9], bool& bad) {
   // R: the zeroth moment of the stored values (rho, or DH when shifted)
   const int64_t R = (((F[5] + F[7]) + (F[6] + F[8])) + ((F[1] + F[3]) + (F[2] + F[4]))) + F[0];
   const int64_t d57 = F[5] - F[7], d86 = F[8] - F[6];
@@ -483,20 +492,30 @@ DF_HD void bgk_fma(double (&f)[9], const BgkParams& p, bool& bad) {
   const int64_t Xi = round_shr(9 * mulh64(jx, V), 3);
   const int64_t AB = Ai + Bi;
   bad |= rho_out_of_range(Rrho) | ((int32_t)(AB >> 32) >= kTurn02);
-  f[0] = fma_d(p.c4, fixed_to_double_tr(4 * (R - AB) - 9 * F[0] + scale_2m64(R, p.mass_k)), f[0]);
+  Y[0] = 4 * (R - AB) - 9 * F[0] + scale_2m64(R, p.mass_k);
   const int64_t cx = R + (2 * Ai - Bi), cy = R + (2 * Bi - Ai);
   const int64_t jx3 = 3 * JX, jy3 = 3 * JY;
   const int64_t ax = jx3 + scale_2m64(JX, p.mom_k), ay = jy3 + scale_2m64(JY, p.mom_k);
-  f[1] = fma_d(p.c4, fixed_to_double_tr(cx + ax - 9 * F[1]), f[1]);
-  f[3] = fma_d(p.c4, fixed_to_double_tr(cx - ax - 9 * F[3]), f[3]);
-  f[2] = fma_d(p.c4, fixed_to_double_tr(cy + ay - 9 * F[2]), f[2]);
-  f[4] = fma_d(p.c4, fixed_to_double_tr(cy - ay - 9 * F[4]), f[4]);
+  Y[1] = cx + ax - 9 * F[1];
+  Y[3] = cx - ax - 9 * F[3];
+  Y[2] = cy + ay - 9 * F[2];
+  Y[4] = cy - ay - 9 * F[4];
   const int64_t dp = R + 2 * (AB + Xi), dm = R + 2 * (AB - Xi);
   const int64_t sp = jx3 + jy3, sm = jy3 - jx3;
-  f[5] = fma_d(p.c1, fixed_to_double_tr(dp + sp - 36 * F[5]), f[5]);
-  f[7] = fma_d(p.c1, fixed_to_double_tr(dp - sp - 36 * F[7]), f[7]);
-  f[6] = fma_d(p.c1, fixed_to_double_tr(dm + sm - 36 * F[6]), f[6]);
-  f[8] = fma_d(p.c1, fixed_to_double_tr(dm - sm - 36 * F[8]), f[8]);
+  Y[5] = dp + sp - 36 * F[5];
+  Y[7] = dp - sp - 36 * F[7];
+  Y[6] = dm + sm - 36 * F[6];
+  Y[8] = dm - sm - 36 * F[8];
+}
+
+template <bool SHIFTED = false>
+DF_HD void bgk_fma(double (&f)[9], const BgkParams& p, bool& bad) {
+  int64_t F[9], Y[9];
+  load_fixed<SHIFTED>(f, F, bad);
+  if (bad) return;
+  bgk_brackets<SHIFTED>(F, p, Y, bad);
+#pragma unroll
+  for (int q = 0; q < 9; q++) f[q] = fma_d(q < 5 ? p.c4 : p.c1, fixed_to_double_tr(Y[q]), f[q]);
 }
 
 // Recursive-regularized constant (rr_fma): 1 - omega at scale 2^63.
@@ -535,11 +554,8 @@ inline RrParams rr_fma_params(double omega) {
 // omega = 1).  Range as bgk_fma, q_xx + q_yy < 0.2 and sum |M / 2| < 0.1: then the Hermite parts
 // add at most 3, 0.9 and 1.8 (units of 2^59) to the rest, axis and diagonal
 // brackets, which stay below 13 x 2^59, and no product's operand leaves int64.
-template <bool SHIFTED = false>
-DF_HD void rr_fma(double (&f)[9], const RrParams& r, const BgkParams& p, bool& bad) {
-  int64_t F[9];
-  load_fixed<SHIFTED>(f, F, bad);
-  if (bad) return;
+template <bool SHIFTED>
+DF_HD void rr_brackets(const int64_t (&F)[9], const RrParams& r, const BgkParams& p, int64_t (&Y)[9], bool& bad) {
   const int64_t s57 = F[5] + F[7], s68 = F[6] + F[8];
   const int64_t sd = s57 + s68;
   const int64_t R = (sd + ((F[1] + F[3]) + (F[2] + F[4]))) + F[0];
@@ -572,21 +588,31 @@ DF_HD void rr_fma(double (&f)[9], const RrParams& r, const BgkParams& p, bool& b
          (4 * sum2 + sum3 >= kTurn06);
   const int64_t X3 = round_shr(mxx, 2), Y3 = round_shr(myy, 2), K = round_shr(9 * mxy, 1);
   const int64_t GY = round_shr(3 * mxxy, 4), GX = round_shr(3 * myyx, 4), G = round_shr(3 * mxxyy, 4);
-  f[0] = fma_d(p.c4, fixed_to_double_tr(4 * (R - X3 - Y3) - 9 * F[0] + 2 * G + scale_2m64(R, p.mass_k)), f[0]);
+  Y[0] = 4 * (R - X3 - Y3) - 9 * F[0] + 2 * G + scale_2m64(R, p.mass_k);
   const int64_t jx3 = 3 * JX, jy3 = 3 * JY;
   const int64_t ax = jx3 + scale_2m64(JX, p.mom_k) - GX, ay = jy3 + scale_2m64(JY, p.mom_k) - GY;
   const int64_t cx = R + 2 * X3 - Y3 - G, cy = R + 2 * Y3 - X3 - G;
-  f[1] = fma_d(p.c4, fixed_to_double_tr(cx + ax - 9 * F[1]), f[1]);
-  f[3] = fma_d(p.c4, fixed_to_double_tr(cx - ax - 9 * F[3]), f[3]);
-  f[2] = fma_d(p.c4, fixed_to_double_tr(cy + ay - 9 * F[2]), f[2]);
-  f[4] = fma_d(p.c4, fixed_to_double_tr(cy - ay - 9 * F[4]), f[4]);
+  Y[1] = cx + ax - 9 * F[1];
+  Y[3] = cx - ax - 9 * F[3];
+  Y[2] = cy + ay - 9 * F[2];
+  Y[4] = cy - ay - 9 * F[4];
   // diagonal pairs without the momentum correction (the axis pairs carry it)
   const int64_t c = R + 2 * (X3 + Y3 + G), dp = c + K, dm = c - K;
   const int64_t sp = (jx3 + jy3) + 2 * (GY + GX), sm = (jy3 - jx3) + 2 * (GY - GX);
-  f[5] = fma_d(p.c1, fixed_to_double_tr(dp + sp - 36 * F[5]), f[5]);
-  f[7] = fma_d(p.c1, fixed_to_double_tr(dp - sp - 36 * F[7]), f[7]);
-  f[6] = fma_d(p.c1, fixed_to_double_tr(dm + sm - 36 * F[6]), f[6]);
-  f[8] = fma_d(p.c1, fixed_to_double_tr(dm - sm - 36 * F[8]), f[8]);
+  Y[5] = dp + sp - 36 * F[5];
+  Y[7] = dp - sp - 36 * F[7];
+  Y[6] = dm + sm - 36 * F[6];
+  Y[8] = dm - sm - 36 * F[8];
+}
+
+template <bool SHIFTED = false>
+DF_HD void rr_fma(double (&f)[9], const RrParams& r, const BgkParams& p, bool& bad) {
+  int64_t F[9], Y[9];
+  load_fixed<SHIFTED>(f, F, bad);
+  if (bad) return;
+  rr_brackets<SHIFTED>(F, r, p, Y, bad);
+#pragma unroll
+  for (int q = 0; q < 9; q++) f[q] = fma_d(q < 5 ? p.c4 : p.c1, fixed_to_double_tr(Y[q]), f[q]);
 }
 
 // (a b) / 2^sh, 0 < sh < 64, of the exact 128-bit product, rounded to nearest
@@ -657,11 +683,7 @@ inline TrtFmaParams trt_fma_params(double lambda_e, double lambda_d, const doubl
 
 DF_HD int64_t abs64(int64_t v) { return v < 0 ? -v : v; }
 
-template <bool SHIFTED = false>
-DF_HD void trt_fma(double (&f)[9], const TrtFmaParams& p, bool& bad) {
-  int64_t F[9];
-  load_fixed<SHIFTED>(f, F, bad);
-  if (bad) return;
+DF_HD void trt_brackets(const int64_t (&F)[9], const TrtFmaParams& p, int64_t (&Y)[9], bool& bad) {
   const int64_t R = (((F[5] + F[7]) + (F[6] + F[8])) + ((F[1] + F[3]) + (F[2] + F[4]))) + F[0];
   const int64_t d57 = F[5] - F[7], d86 = F[8] - F[6];
   const int64_t JX = (d57 + d86) + (F[1] - F[3]);
@@ -676,18 +698,28 @@ DF_HD void trt_fma(double (&f)[9], const TrtFmaParams& p, bool& bad) {
   const int64_t lim = (int64_t)1 << 61;
   bad |= (abs64(sx) | abs64(sy) | abs64(sp) | abs64(sm)) >= lim;
   bad |= (abs64(dx) | abs64(dy) | abs64(dp) | abs64(dm)) >= p.dmax;
-  f[0] = fma_d(p.c2, fixed_to_double_tr(4 * R - 6 * J2 - 9 * F[0] + scale_2m64(R, p.mass_k)), f[0]);
+  Y[0] = 4 * R - 6 * J2 - 9 * F[0] + scale_2m64(R, p.mass_k);
   const int64_t rx = mul_shr(dx, p.r_fx, p.r_sh) - scale_2m64(JX, p.mom_k);
   const int64_t ry = mul_shr(dy, p.r_fx, p.r_sh) - scale_2m64(JY, p.mom_k);
   const int64_t rp = mul_shr(dp, p.r_fx, p.r_sh), rm = mul_shr(dm, p.r_fx, p.r_sh);
-  f[1] = fma_d(p.c, fixed_to_double_tr(-(sx + rx)), f[1]);
-  f[3] = fma_d(p.c, fixed_to_double_tr(rx - sx), f[3]);
-  f[2] = fma_d(p.c, fixed_to_double_tr(-(sy + ry)), f[2]);
-  f[4] = fma_d(p.c, fixed_to_double_tr(ry - sy), f[4]);
-  f[5] = fma_d(p.ch, fixed_to_double_tr(-(sp + rp)), f[5]);
-  f[7] = fma_d(p.ch, fixed_to_double_tr(rp - sp), f[7]);
-  f[8] = fma_d(p.ch, fixed_to_double_tr(-(sm + rm)), f[8]);
-  f[6] = fma_d(p.ch, fixed_to_double_tr(rm - sm), f[6]);
+  Y[1] = -(sx + rx);
+  Y[3] = rx - sx;
+  Y[2] = -(sy + ry);
+  Y[4] = ry - sy;
+  Y[5] = -(sp + rp);
+  Y[7] = rp - sp;
+  Y[8] = -(sm + rm);
+  Y[6] = rm - sm;
+}
+
+template <bool SHIFTED = false>
+DF_HD void trt_fma(double (&f)[9], const TrtFmaParams& p, bool& bad) {
+  int64_t F[9], Y[9];
+  load_fixed<SHIFTED>(f, F, bad);
+  if (bad) return;
+  trt_brackets(F, p, Y, bad);
+#pragma unroll
+  for (int q = 0; q < 9; q++) f[q] = fma_d(q == 0 ? p.c2 : (q < 5 ? p.c : p.ch), fixed_to_double_tr(Y[q]), f[q]);
 }
 
 }  // namespace hy

@@ -46,12 +46,15 @@ int block_for(long long cells);
   /* grid%streaming => stream_fvm_bardow (1), stream_fdm_bardow (2, 3 iso,    */          \
   /* 4 least squares), stream_fdm_sofonea (5): src/fvm_bardow.F90:393-886     */          \
   cudaError_t stream_scheme_f64(int scheme, const Sweep& s, double dt);                   \
-  /* the same fused with collide_* in stencil form (9 FMAs per population) */             \
-  cudaError_t step_scheme_f64(int scheme, int kind, const Sweep& s, double dt, const CollParams& p); \
   }
 PLBM_DECLARE_F64(fma)
 PLBM_DECLARE_F64(strict)
 #undef PLBM_DECLARE_F64
+namespace fma {
+// a finite-volume / finite-difference scheme in stencil form fused with
+// collide_bgk_improved (ld == ny)
+cudaError_t step_scheme_f64(int scheme, const Sweep& s, double dt, const CollParams& p);
+}
 
 // binary64 storage, fixed-point arithmetic (hybrid.cuh), YFast pull, BGK, TRT
 // and RR: the step of PLBM_MATH_HYBRID (report: a cell out of range sets the
@@ -60,8 +63,8 @@ cudaError_t step_pull_fixed(int kind, const Sweep& s, const CollParams& p, bool 
 // The plugin step (shifted binary64, x-fastest, collide then push) in the same
 // arithmetic (BGK, TRT, RR).
 cudaError_t step_push_fixed(int kind, const Sweep& s, const CollParams& p, bool report);
-// A finite-volume / finite-difference streaming scheme (stencil form) fused
-// with the fixed-point collision (BGK, TRT, RR).
+// A finite-volume / finite-difference streaming scheme fused with the
+// fixed-point collision (BGK, TRT, RR).
 cudaError_t step_scheme_fixed(int scheme, int kind, const Sweep& s, double dt, const CollParams& p, bool report);
 cudaError_t hybrid_range_flag(int* flag, int reset);
 // The PLBM_MATH_FMA step: the fixed point for BGK, TRT and RR, the binary64

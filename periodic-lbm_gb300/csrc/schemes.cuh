@@ -10,7 +10,8 @@
 //
 // Every scheme is linear in v, so scheme_value(delta_k) is the coefficient of
 // v[k]; stencil_coefficients() tabulates them (9 per population) for the
-// stencil-form kernels of the FMA and hybrid builds, which then need 9 fused
+// stencil-form kernels (the Gaussian-weighted schemes, large time steps, the
+// improved BGK and the out-of-range cells), which then need 9 fused
 // multiply-adds per population.
 #pragma once
 #include <math.h>

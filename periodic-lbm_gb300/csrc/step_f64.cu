@@ -114,9 +114,11 @@ __global__ void __launch_bounds__(kBlock) k_stream_scheme(const double* __restri
   }
 }
 
-// Fused stencil-form streaming + collide_* (FMA build): one read pass of the
-// 3x3 neighbourhoods (L1/L2 reuse), one write of the 9 collided populations.
-template <int TAPS, int KIND>
+#ifndef PLBM_STRICT
+// Fused stencil-form streaming + collide_bgk_improved (the other collisions run
+// in the fixed point, step_hybrid.cu): one read pass of the 3x3 neighbourhoods
+// (L1/L2 reuse), one write of the 9 collided populations.
+template <int TAPS>
 __global__ void __launch_bounds__(kBlock) k_step_scheme(const double* __restrict__ src, double* __restrict__ dst,
                                                        int nx, int ny, int ld, int ftiles, sch::Stencil st,
                                                        CollParams p) {
@@ -124,10 +126,11 @@ __global__ void __launch_bounds__(kBlock) k_step_scheme(const double* __restrict
   if (!cell_of<YFast>(ftiles, nx, ny, x, y)) return;
   double f[9];
   sch::stencil_pull<YFast, TAPS>(src, x, y, nx, ny, ld, st, f);
-  collide_ref<KIND>(f, p);
+  collide_ref<K_BGKI>(f, p);
 #pragma unroll
   for (int q = 0; q < 9; q++) dst[YFast::off(x, y, q, nx, ny, ld)] = f[q];
 }
+#endif
 
 // lbm_stream: fdst(y,x,q) = fsrc(y - cy, x - cx, q) for rows 1:ny.
 __global__ void __launch_bounds__(kBlock) k_stream(const double* __restrict__ src, double* __restrict__ dst,
@@ -261,32 +264,25 @@ cudaError_t stream_scheme_f64(int scheme, const Sweep& s, double dt) {
   return cudaGetLastError();
 }
 
-cudaError_t step_scheme_f64(int scheme, int kind, const Sweep& s, double dt, const CollParams& p) {
+#ifndef PLBM_STRICT
+cudaError_t step_scheme_f64(int scheme, const Sweep& s, double dt, const CollParams& p) {
   const int ft = tiles(s.ny);
   const long long blocks = (long long)ft * s.nx;
   if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-  if (kind == K_BGKI && s.ld != s.ny) return cudaErrorNotSupported;
+  if (s.ld != s.ny) return cudaErrorNotSupported;
+  if (scheme < sch::FVM || scheme > sch::FDM_WLS_G2) return cudaErrorInvalidValue;
   const sch::Stencil st = sch::stencil_coefficients(scheme, dt);
   const double* a = static_cast<const double*>(s.src);
   double* b = static_cast<double*>(s.dst);
   const unsigned nb = (unsigned)blocks;
-#define PLBM_SCH_KIND(SC)                                                                                     \
-  switch (kind) {                                                                                             \
-    case K_BGK: k_step_scheme<SC, K_BGK><<<nb, kBlock, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, st, p); break; \
-    case K_TRT: k_step_scheme<SC, K_TRT><<<nb, kBlock, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, st, p); break; \
-    case K_RR: k_step_scheme<SC, K_RR><<<nb, kBlock, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, st, p); break;   \
-    case K_BGKI: k_step_scheme<SC, K_BGKI><<<nb, kBlock, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, st, p); break; \
-    default: return cudaErrorInvalidValue;                                                                    \
-  }
-  if (scheme < sch::FVM || scheme > sch::FDM_WLS_G2) return cudaErrorInvalidValue;
   switch (sch::taps_of(scheme)) {
-    case sch::TAPS_LINE: PLBM_SCH_KIND(sch::TAPS_LINE) break;
-    case sch::TAPS_AXIS3: PLBM_SCH_KIND(sch::TAPS_AXIS3) break;
-    default: PLBM_SCH_KIND(sch::TAPS_FULL) break;
+    case sch::TAPS_LINE: k_step_scheme<sch::TAPS_LINE><<<nb, kBlock, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, st, p); break;
+    case sch::TAPS_AXIS3: k_step_scheme<sch::TAPS_AXIS3><<<nb, kBlock, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, st, p); break;
+    default: k_step_scheme<sch::TAPS_FULL><<<nb, kBlock, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, st, p); break;
   }
-#undef PLBM_SCH_KIND
   return cudaGetLastError();
 }
+#endif
 
 cudaError_t stream_f64(const Sweep& s) {
   const int ft = tiles(s.ny);

@@ -124,6 +124,158 @@ __global__ void __launch_bounds__(kBlock) k_step_scheme_hybrid(const double* __r
   for (int q = 0; q < 9; q++) dst[YFast::off(x, y, q, nx, ny, ld)] = f[q];
 }
 
+// ---- finite-difference streaming in the fixed point --------------------------
+// Every scheme but the Gaussian-weighted ones is
+//   f*_q = f_q - a1 D1 + a2 D2,
+// D1 and D2 integer combinations of the 3x3 neighbourhood (first differences
+// along c_q, second differences), so on int64 populations the sums are exact
+// and two products per population remain where the stencil form takes 3 or 9
+// binary64 FMAs (48 per cell for FVM / central FDM: the binary64 pipe's 25
+// cycles per cell and SM).  A CTA converts the populations of a 32 x TX tile
+// and its halo to the fixed point once, in shared memory.  The streamed
+// population joins the collision as an integer, and the new one,
+//   f'_q = F_q + (a2 D2 - a1 D1) + k_q c Y_q  (at 2^-61),
+// is rounded to binary64 once: no binary64 instruction at all.
+// Rule: LINE (Sofonea), CENTRAL (FVM, which expands to the same sums, and central
+// FDM), ISO and WLS, while a1 and a2 are below 2^(shift - 4) (time steps up to
+// about 1, the scheme's own stability limit); other schemes and steps keep the
+// stencil form.  512^2, central FDM, BGK, dt = 0.3: 68 us per step in the stencil
+// form with the binary64 collision, 33 us with the fixed-point collision, 20.5 us
+// here (12.7 GLUPS; 2048^2 17.0 against 4.2 and 8.0); error against binary64
+// arithmetic of the reference's expressions 4.4e-16 (stencil form 2.1e-15).
+// Bound by issue: about 1,500 instructions per cell, the ALU pipe 67 % busy.
+enum { FORM_LINE = 0, FORM_CENTRAL = 1, FORM_ISO = 2, FORM_WLS = 3 };
+// Left shift of D1, D2 before the product: the largest for which |D| 2^shift stays
+// below 2^63 for axis populations below 1/4 and diagonal ones below 1/8.
+__host__ __device__ constexpr int form_shift(int form) { return form <= FORM_CENTRAL ? 3 : (form == FORM_ISO ? 1 : 2); }
+
+struct SchemeFx {
+  int64_t a1s, a2s, a1d, a2d;  // a1, a2 of axis and diagonal populations, 2^(66 - shift) a
+  int64_t c;                   // 2^66 of the collision's constant (1/36 of the rate)
+};
+
+template <int FORM>
+__device__ __forceinline__ void scheme_differences(const int64_t (&v)[9], int q, int64_t& d1, int64_t& d2) {
+  using namespace sch;
+  const int cx = cx_of(q), cy = cy_of(q);
+  if (FORM == FORM_LINE || (FORM == FORM_CENTRAL && q <= 4)) {
+    const int64_t u = v[nb(cx, cy)], d = v[nb(-cx, -cy)];
+    d1 = u - d;
+    d2 = u + d - 2 * v[C];
+    return;
+  }
+  if (FORM == FORM_CENTRAL) {
+    const int64_t dx = v[E] - v[W], dy = v[N] - v[S];
+    const int64_t xy = (v[NE] + v[SW]) - (v[NW] + v[SE]);
+    d1 = (cx > 0 ? dx : -dx) + (cy > 0 ? dy : -dy);
+    d2 = 2 * ((v[E] + v[W]) + (v[N] + v[S]) - 4 * v[C]) + (cx * cy > 0 ? xy : -xy);
+    return;
+  }
+  constexpr int wa = FORM == FORM_ISO ? 4 : 1, wb = FORM == FORM_ISO ? 10 : 1;
+  const int64_t dx = (v[NE] - v[NW]) + (v[SE] - v[SW]) + wa * (v[E] - v[W]);
+  const int64_t dy = (v[NE] - v[SE]) + (v[NW] - v[SW]) + wa * (v[N] - v[S]);
+  const int64_t xx = (v[NE] + v[NW] - 2 * v[N]) + (v[SE] + v[SW] - 2 * v[S]) + wb * (v[E] + v[W] - 2 * v[C]);
+  const int64_t yy = (v[NE] + v[SE] - 2 * v[E]) + (v[NW] + v[SW] - 2 * v[W]) + wb * (v[N] + v[S] - 2 * v[C]);
+  d1 = (cx > 0 ? dx : (cx < 0 ? -dx : 0)) + (cy > 0 ? dy : (cy < 0 ? -dy : 0));
+  if (q <= 4) {
+    d2 = cx ? xx : yy;
+  } else {
+    const int64_t xy = (v[NE] + v[SW]) - (v[NW] + v[SE]);
+    constexpr int kx = FORM == FORM_ISO ? 1 : 2, kd = FORM == FORM_ISO ? 6 : 3;
+    d2 = kx * (xx + yy) + (cx * cy > 0 ? kd * xy : -kd * xy);
+  }
+}
+
+__host__ __device__ constexpr int form_taps(int form) {
+  return form == FORM_LINE ? sch::TAPS_LINE : (form == FORM_CENTRAL ? sch::TAPS_AXIS3 : sch::TAPS_FULL);
+}
+
+// 256 threads: warp w loads population w + 1 of the tile, then takes the columns
+// w, w + 8, ... below TX (its lanes the 32 rows).
+template <int FORM, int KIND, int TX>
+__global__ void __launch_bounds__(256, KIND == K_RR ? 3 : 4)
+    k_step_scheme_fixed(const double* __restrict__ src, double* __restrict__ dst, int nx, int ny, int ld, int ytiles,
+                        SchemeFx sc, sch::Stencil st, HybridArgs a) {
+  constexpr int ROWS = 34;
+  __shared__ int64_t sm[8][TX + 2][ROWS];
+  __shared__ int tile_bad;
+  const int x0 = (blockIdx.x / ytiles) * TX, y0 = (blockIdx.x % ytiles) * 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) tile_bad = 0;
+  __syncthreads();
+  {
+    bool bad = false;
+    const double* f = src + (size_t)(warp + 1) * ld * nx;
+    // every load first, then the conversions (their rare out-of-line path would
+    // otherwise put one memory latency after the other)
+    auto load = [&](int c, int r) {
+      const int gx = x0 - 1 + c, gy = y0 - 1 + r;
+      if (gx > nx || gy > ny) return 0.0;  // past the last cell's neighbours
+      return __ldg(f + (size_t)(gx < 0 ? nx - 1 : (gx == nx ? 0 : gx)) * ld +
+                   (gy < 0 ? ny - 1 : (gy == ny ? 0 : gy)));
+    };
+    auto convert = [&](double d) {
+      return warp < 4 ? hy::to_fixed_nonneg<1020>(d, bad) : hy::to_fixed_nonneg<1019>(d, bad);
+    };
+    constexpr int EX = (2 * (TX + 2) + 31) / 32;  // rows 32 and 33, two per column
+    double d[TX + 2], e[EX];
+#pragma unroll
+    for (int c = 0; c < TX + 2; c++) d[c] = load(c, lane);
+#pragma unroll
+    for (int i = 0; i < EX; i++) e[i] = lane + 32 * i < 2 * (TX + 2) ? load((lane >> 1) + 16 * i, 32 + (lane & 1)) : 0.0;
+#pragma unroll
+    for (int c = 0; c < TX + 2; c++) sm[warp][c][lane] = convert(d[c]);
+#pragma unroll
+    for (int i = 0; i < EX; i++)
+      if (lane + 32 * i < 2 * (TX + 2)) sm[warp][(lane >> 1) + 16 * i][32 + (lane & 1)] = convert(e[i]);
+    if (bad) tile_bad = 1;
+  }
+  __syncthreads();
+  const int y = y0 + lane;
+  if (y >= ny) return;
+  const size_t P = (size_t)ld * nx;
+#pragma unroll 1
+  for (int c = warp; c < TX && x0 + c < nx; c += 8) {
+    const int x = x0 + c;
+    const size_t o = (size_t)x * ld + y;
+    bool bad = tile_bad;
+    int64_t F[9], Z[9];
+    if (!bad) {
+      F[0] = hy::to_fixed_nonneg<1022>(__ldg(src + o), bad);
+      Z[0] = hy::shl(F[0], 2);
+#pragma unroll
+      for (int q = 1; q < 9; q++) {
+        int64_t v[9], d1, d2;
+#pragma unroll
+        for (int k = 0; k < 9; k++) v[k] = sm[q - 1][c + 1 + sch::ex(k)][lane + 1 + sch::ey(k)];
+        scheme_differences<FORM>(v, q, d1, d2);
+        constexpr int S = form_shift(FORM);
+        const int64_t d = hy::mulh64(hy::shl(d2, S), q < 5 ? sc.a2s : sc.a2d) -
+                          hy::mulh64(hy::shl(d1, S), q < 5 ? sc.a1s : sc.a1d);
+        Z[q] = hy::shl(v[sch::C], 2) + d;
+        F[q] = hy::round_shr(Z[q], 2);
+        bad |= (uint32_t)((uint64_t)F[q] >> 32) >= (1u << (q < 5 ? 25 : 24));
+      }
+      int64_t Y[9];
+      if (KIND == K_TRT) hy::trt_brackets(F, a.trt, Y, bad);
+      else if (KIND == K_RR) hy::rr_brackets<false>(F, a.rr, a.rr1, Y, bad);
+      else hy::bgk_brackets<false>(F, a.bgk1, Y, bad);
+#pragma unroll
+      for (int q = 0; q < 9; q++) {
+        const int k = q == 0 ? 4 : (q > 4 ? 1 : (KIND == K_TRT ? 2 : 4));
+        Z[q] += k * hy::mulh64(Y[q], sc.c);
+        bad |= Z[q] <= 0;
+      }
+    }
+    if (bad) {
+      scheme_fallback_cell<form_taps(FORM), KIND>(src, dst, x, y, nx, ny, ld, st, a.ref, a.report);
+      continue;
+    }
+#pragma unroll
+    for (int q = 0; q < 9; q++) dst[q * P + o] = hy::pos_fixed_to_double<61>(Z[q]);
+  }
+}
+
 // The plugin step (sim/sim.F90:404-505 + :568-624) in the hybrid arithmetic:
 // shifted binary64 populations h = f - w in the x-fastest layout, collide at
 // the cell, push along c_q.  Out-of-range cells take the shifted binary64
@@ -251,6 +403,65 @@ cudaError_t step_push_fixed(int kind, const Sweep& s, const CollParams& cp, bool
   return cudaGetLastError();
 }
 
+namespace {
+// The fixed-point constants of a scheme, or false where it keeps the stencil
+// form (see k_step_scheme_fixed).
+bool scheme_fixed_constants(int scheme, int kind, double dt, double omega, int& form, SchemeFx& c) {
+  double a1s, a2s, a1d, a2d;
+  switch (scheme) {
+    case sch::SOFONEA:
+      form = FORM_LINE;
+      a1s = 0.5 * dt, a2s = 0.5 * dt * dt;
+      a1d = dt * 0.35355339059327373, a2d = 0.25 * dt * dt;
+      break;
+    case sch::FVM:
+    case sch::FDM:
+      form = FORM_CENTRAL;
+      a1s = a1d = 0.5 * dt, a2s = 0.5 * dt * dt, a2d = 0.25 * dt * dt;
+      break;
+    case sch::FDM_ISO:
+      form = FORM_ISO;
+      a1s = a1d = dt / 12.0, a2s = a2d = dt * dt / 24.0;
+      break;
+    case sch::FDM_WLS:
+      form = FORM_WLS;
+      a1s = a1d = dt / 6.0, a2s = dt * dt / 6.0, a2d = dt * dt / 12.0;
+      break;
+    default: return false;
+  }
+  const int s = form_shift(form);
+  const double lim = ldexp(1.0, s - 4);
+  if (!(a1s < lim && a2s < lim && a1d < lim && a2d < lim)) return false;
+  c.a1s = llrint(ldexp(a1s, 66 - s));
+  c.a2s = llrint(ldexp(a2s, 66 - s));
+  c.a1d = llrint(ldexp(a1d, 66 - s));
+  c.a2d = llrint(ldexp(a2d, 66 - s));
+  c.c = llrint(ldexp((kind == K_RR ? 1.0 : omega) / 36.0, 66));
+  return true;
+}
+
+// Tile columns of k_step_scheme_fixed: two for grids whose wider tiles would not
+// give every SM a CTA, 16 (two cells per thread, the smaller halo) where every SM
+// gets several.  BGK, central FDM, MLUPS with 2 / 8 / 16 columns: 64^2 1,205 / 885 / 525,
+// 128^2 3,849 / 3,538 / 2,084, 256^2 7,966 / 9,788 / 8,206, 512^2 8,510 / 12,742 /
+// 11,587, 1024^2 - / 10,019 / 10,011 (an earlier form), 2048^2 9,895 / 16,486 / 17,019.
+int scheme_tile(const Sweep& s) {
+  const long long cells = (long long)s.nx * s.ny;
+  return cells > (1 << 20) ? 16 : (cells > 40000 ? 8 : 2);
+}
+
+template <int FORM, int TX>
+void launch_scheme_fixed(int kind, const Sweep& s, const SchemeFx& c, const sch::Stencil& st, const HybridArgs& a) {
+  const double* src = static_cast<const double*>(s.src);
+  double* dst = static_cast<double*>(s.dst);
+  const int yt = (s.ny + 31) / 32;
+  const unsigned nb = (unsigned)((long long)yt * ((s.nx + TX - 1) / TX));
+  if (kind == K_TRT) k_step_scheme_fixed<FORM, K_TRT, TX><<<nb, 256, 0, s.stream>>>(src, dst, s.nx, s.ny, s.ld, yt, c, st, a);
+  else if (kind == K_RR) k_step_scheme_fixed<FORM, K_RR, TX><<<nb, 256, 0, s.stream>>>(src, dst, s.nx, s.ny, s.ld, yt, c, st, a);
+  else k_step_scheme_fixed<FORM, K_BGK, TX><<<nb, 256, 0, s.stream>>>(src, dst, s.nx, s.ny, s.ld, yt, c, st, a);
+}
+}  // namespace
+
 cudaError_t step_scheme_fixed(int scheme, int kind, const Sweep& s, double dt, const CollParams& cp, bool report) {
   if (kind != K_BGK && kind != K_TRT && kind != K_RR) return cudaErrorNotSupported;
   if (scheme < sch::FVM || scheme > sch::FDM_WLS_G2) return cudaErrorInvalidValue;
@@ -259,6 +470,23 @@ cudaError_t step_scheme_fixed(int scheme, int kind, const Sweep& s, double dt, c
   if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   const sch::Stencil st = sch::stencil_coefficients(scheme, dt);
   const HybridArgs a = hybrid_args(cp, report);
+  int form;
+  SchemeFx c;
+  if (scheme_fixed_constants(scheme, kind, dt, cp.omega, form, c)) {
+    const int tx = scheme_tile(s);
+#define PLBM_SCH_FX(F)                                             \
+  if (tx == 16) launch_scheme_fixed<F, 16>(kind, s, c, st, a);     \
+  else if (tx == 8) launch_scheme_fixed<F, 8>(kind, s, c, st, a);  \
+  else launch_scheme_fixed<F, 2>(kind, s, c, st, a)
+    switch (form) {
+      case FORM_LINE: PLBM_SCH_FX(FORM_LINE); break;
+      case FORM_CENTRAL: PLBM_SCH_FX(FORM_CENTRAL); break;
+      case FORM_ISO: PLBM_SCH_FX(FORM_ISO); break;
+      default: PLBM_SCH_FX(FORM_WLS); break;
+    }
+#undef PLBM_SCH_FX
+    return cudaGetLastError();
+  }
   const double* src = static_cast<const double*>(s.src);
   double* dst = static_cast<double*>(s.dst);
   const unsigned nb = (unsigned)blocks;
