@@ -206,13 +206,12 @@ extern "C" int plbm_adjoint_forward(plbm_adjoint_t* a, const double* u0, double 
   const void* cur = lat(a->ck, a, 0);
   int tog = 0;
   for (int n = 0; n < a->nsteps; n++) {
-    void* dst = lat(a->work, a, tog);
-    tog ^= 1;
+    // a checkpoint is written by the step that reaches it
+    const bool ck = (n + 1) % a->K == 0 && n + 1 < a->nsteps;
+    void* dst = ck ? lat(a->ck, a, (n + 1) / a->K) : lat(a->work, a, tog);
+    if (!ck) tog ^= 1;
     CUDA_TRY(fwd_step(a, cur, dst, p, a->stream), "forward step");
     cur = dst;
-    if ((n + 1) % a->K == 0 && (n + 1) < a->nsteps)
-      CUDA_TRY(cudaMemcpyAsync(lat(a->ck, a, (n + 1) / a->K), cur, a->lat_bytes, cudaMemcpyDeviceToDevice, a->stream),
-               "checkpoint copy");
   }
   a->fT = cur;
   if (uT) {

@@ -13,7 +13,8 @@
 //   S0 = sum w_q lambda_q, A = sum w_q lambda_q (1 - 4.5 (c_q.u)^2 + 1.5 u^2),
 //   B = sum w_q lambda_q (3 + 9 c_q.u) c_q.
 // The per-cell adjoint arithmetic runs in the storage's type (binary64 for
-// PLBM_F64, binary32 for PLBM_F32DEV): lambda, its weighted sums and mu; with
+// PLBM_F64, whose forward state u and feq - g come from the fixed point of
+// hybrid.cuh, binary32 for PLBM_F32DEV): lambda, its weighted sums and mu; with
 // plbm_adjoint_set_math(PLBM_MATH_HYBRID) the binary32 reverse step is the
 // compensated one of coll_df64.cuh (k_adj_step_comp).  The
 // gradients are accumulated in binary64: each cell's dL/domega term is taken
@@ -24,13 +25,12 @@
 
 #include "../../include/plbm_gpu.h"
 #include "coll_df64.cuh"
+#include "hybrid.cuh"
 #include "plbm_adjoint.h"
 #include "plbm_launch.h"
 
 namespace plbm {
 namespace {
-
-inline int tiles(int n) { return (n + kBlock - 1) / kBlock; }
 
 __device__ __forceinline__ bool yfast_cell(int ftiles, int ny, int& x, int& y) {
   x = blockIdx.x / ftiles;
@@ -78,6 +78,110 @@ __device__ __forceinline__ void cell_state(const R (&g)[9], R& rho, R& ux, R& uy
     const R hg = SHIFT ? g[q] : g[q] - w;
     neq[q] = heq - hg;  // feq_q - g_q
   }
+}
+
+// One cell of the reverse step, binary32: mu = J_C(g)^T lambda and the dL/domega
+// term sum_q l_q (feq_q - g_q).  (The binary64 form's pair sums would not run
+// faster here, where the loads bind, and round otherwise.)
+__device__ __forceinline__ float reverse_cell(const float (&g)[9], const float (&l)[9], float om, float (&mu)[9]) {
+  typedef float R;
+  R neq[9], rho, ux, uy;
+  cell_state<R, true>(g, rho, ux, uy, neq);
+  const R u2 = ux * ux + uy * uy;
+  R s0 = 0, A = 0, Bx = 0, By = 0, d = 0;
+#pragma unroll
+  for (int q = 0; q < 9; q++) {
+    d += l[q] * neq[q];
+    const R cu = (R)cx_of(q) * ux + (R)cy_of(q) * uy;
+    const R wl = (R)w_of(q) * l[q];
+    s0 += wl;
+    A += wl * (R(1) - R(4.5) * cu * cu + R(1.5) * u2);
+    const R b = wl * (R(3) + R(9) * cu);
+    Bx += b * (R)cx_of(q);
+    By += b * (R)cy_of(q);
+  }
+  const R omb = R(1) - om;
+  const R ex = Bx - R(3) * s0 * ux, ey = By - R(3) * s0 * uy;
+#pragma unroll
+  for (int p = 0; p < 9; p++) mu[p] = omb * l[p] + om * (A + (R)cx_of(p) * ex + (R)cy_of(p) * ey);
+  return d;
+}
+
+// u and the dL/domega term in binary64 for a cell outside the fixed point's
+// range, out of line.
+__device__ __noinline__ double forward_state_ref(const double* gp, const double* lp, double* u) {
+  double g[9], neq[9], rho, d = 0.0;
+  for (int q = 0; q < 9; q++) g[q] = gp[q];
+  cell_state<double, false>(g, rho, u[0], u[1], neq);
+  for (int q = 0; q < 9; q++) d += lp[q] * neq[q];
+  return d;
+}
+
+// Binary64: u and 36 (feq_q - g_q) / k_q = Y_q from the fixed point (hybrid.cuh),
+// whose error is below that of the binary64 expressions, so that the binary64
+// pipe is left with the sums over lambda.
+__device__ __forceinline__ double forward_state(const double (&g)[9], const double (&l)[9], double& ux, double& uy) {
+  int64_t F[9], Y[9], U, V;
+  bool bad = false;
+  const hy::BgkParams none = {0.0, 0.0, 0, 0};
+  hy::load_fixed<false>(g, F, bad);
+  if (!bad) hy::bgk_brackets<false>(F, none, Y, U, V, bad);
+  if (bad) {
+    double gc[9], lc[9], u[2];
+#pragma unroll
+    for (int q = 0; q < 9; q++) gc[q] = g[q], lc[q] = l[q];
+    const double d = forward_state_ref(gc, lc, u);
+    ux = u[0];
+    uy = u[1];
+    return d;
+  }
+  ux = hy::fixed_to_double_tr<61>(U);
+  uy = hy::fixed_to_double_tr<61>(V);
+  double ds = l[0] * hy::fixed_to_double_tr(Y[0]), dd = l[5] * hy::fixed_to_double_tr(Y[5]);
+#pragma unroll
+  for (int q = 1; q < 5; q++) ds += l[q] * hy::fixed_to_double_tr(Y[q]);
+#pragma unroll
+  for (int q = 6; q < 9; q++) dd += l[q] * hy::fixed_to_double_tr(Y[q]);
+  return (4.0 * ds + dd) * (1.0 / 36.0);
+}
+
+// The same cell in binary64, where the pipe's two operations per cycle and SM
+// bind.  mu from the weighted moments of lambda, taken from the pair sums and
+// differences:
+//   Kxx, Kyy, Kxy = sum w l c c,  M1 = sum w l c,  S0 = sum w l,
+//   Q = K u,  N = 4.5 u.Q - 1.5 u^2 S0,  A = S0 - N,  E = 3 M1 + 9 Q - 3 S0 u,
+//   mu_p = (1 - omega) l_p + omega (A + c_p.E):
+// about 60 operations and 11 for dL/domega, where the sums over all nine
+// populations, with products by zero velocity components that floating point may
+// not drop, two divisions and the equilibria took more than three times as many.
+// 256^2: 46.8 us per reverse step (with its share of the recomputation) before,
+// 19.0 now; 1024^2 618 and 187.
+__device__ __forceinline__ double reverse_cell(const double (&g)[9], const double (&l)[9], double om,
+                                               double (&mu)[9]) {
+  double ux, uy;
+  const double d = forward_state(g, l, ux, uy);
+  const double l57 = l[5] + l[7], l86 = l[8] + l[6], m57 = l[5] - l[7], m86 = l[8] - l[6];
+  const double kd = WD * (l57 + l86), kxy = WD * (l57 - l86);
+  const double l24 = l[2] + l[4];
+  const double kxx = kd + WS * (l[1] + l[3]), kyy = kd + WS * l24;
+  const double s0 = (kxx + WS * l24) + W0 * l[0];
+  const double mx = WD * (m57 + m86) + WS * (l[1] - l[3]), my = WD * (m57 - m86) + WS * (l[2] - l[4]);
+  const double qx = ux * kxx + uy * kxy, qy = uy * kyy + ux * kxy;
+  const double n = 4.5 * (ux * qx + uy * qy) - (1.5 * s0) * (ux * ux + uy * uy);
+  const double omb = 1.0 - om, om3 = 3.0 * om;
+  const double a = om * (s0 - n);
+  const double ex = om3 * ((mx + 3.0 * qx) - s0 * ux), ey = om3 * ((my + 3.0 * qy) - s0 * uy);
+  const double ep = ex + ey, em = ex - ey;
+  mu[0] = omb * l[0] + a;
+  mu[1] = omb * l[1] + (a + ex);
+  mu[3] = omb * l[3] + (a - ex);
+  mu[2] = omb * l[2] + (a + ey);
+  mu[4] = omb * l[4] + (a - ey);
+  mu[5] = omb * l[5] + (a + ep);
+  mu[7] = omb * l[7] + (a - ep);
+  mu[8] = omb * l[8] + (a + em);
+  mu[6] = omb * l[6] + (a - em);
+  return d;
 }
 
 // Warp sum in binary64 of the cells' dL/domega terms.  Each warp adds its sum
@@ -161,34 +265,15 @@ __global__ void __launch_bounds__(kBlock) k_adj_step(const void* __restrict__ f,
     const I y0 = (I)y, ym = (I)wrap_m(y, ny), yp = (I)wrap_p(y, ny);
     const I off[9] = {c0 + y0,         P + cm + y0,     2 * P + c0 + ym, 3 * P + cp + y0, 4 * P + c0 + yp,
                       5 * P + cm + ym, 6 * P + cp + ym, 7 * P + cp + yp, 8 * P + cm + yp};
-    R g[9], l[9], neq[9], rho, ux, uy;
+    R g[9], l[9], mu[9];
 #pragma unroll
     for (int q = 0; q < 9; q++) {
       g[q] = (R)__ldg(fe + off[q]);
       l[q] = (R)__ldg(li + ((I)q * P + c0 + y0));
     }
-    cell_state<R, AdjTraits<ST>::shift>(g, rho, ux, uy, neq);
-    const R u2 = ux * ux + uy * uy;
-    R s0 = 0, A = 0, Bx = 0, By = 0, d = 0;
+    part = reverse_cell(g, l, om, mu);
 #pragma unroll
-    for (int q = 0; q < 9; q++) {
-      d += l[q] * neq[q];
-      const R cu = (R)cx_of(q) * ux + (R)cy_of(q) * uy;
-      const R wl = (R)w_of(q) * l[q];
-      s0 += wl;
-      A += wl * (R(1) - R(4.5) * cu * cu + R(1.5) * u2);
-      const R b = wl * (R(3) + R(9) * cu);
-      Bx += b * (R)cx_of(q);
-      By += b * (R)cy_of(q);
-    }
-    part = d;
-    const R omb = R(1) - om;
-    const R ex = Bx - R(3) * s0 * ux, ey = By - R(3) * s0 * uy;
-#pragma unroll
-    for (int p = 0; p < 9; p++) {
-      const R mu = omb * l[p] + om * (A + (R)cx_of(p) * ex + (R)cy_of(p) * ey);
-      lo[off[p]] = (E)mu;
-    }
+    for (int p = 0; p < 9; p++) lo[off[p]] = (E)mu[p];
   }
   const double t = warp_sum((double)part);
   if ((threadIdx.x & 31) == 0) dom[(size_t)blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5)] += t;
@@ -247,6 +332,8 @@ __global__ void __launch_bounds__(kBlock) k_adj_u0(const void* __restrict__ lam,
   grad[o] = ax;
   grad[n + o] = ay;
 }
+
+inline int tiles(int n) { return (n + kBlock - 1) / kBlock; }
 
 template <int ST>
 cudaError_t dispatch(int what, const AdjLaunch& a) {

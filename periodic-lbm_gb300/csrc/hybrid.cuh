@@ -240,6 +240,7 @@ DF_HD float i2f(int32_t v) {
 #endif
 }
 
+DF_HD constexpr double pow2_const(int e) { return e == 0 ? 1.0 : (e > 0 ? 2.0 * pow2_const(e - 1) : 0.5 * pow2_const(e + 1)); }
 PLBM_NOINLINE double fixed_to_double_any_slow(int64_t T) { return fixed_to_double_any(T); }
 
 // int64 v > 0 (scale 2^SCALE) -> binary64 rounded to nearest, ties away from
@@ -252,22 +253,23 @@ DF_HD double pos_fixed_to_double(int64_t v) {
   return df::u2d(((uint64_t)(uint32_t)(1085 - SCALE - lz) << 52) + m);
 }
 
-// int64 fixed point (scale 2^59) -> binary64 for |T| >= 2^32 (others out of
+// int64 fixed point (scale 2^SCALE) -> binary64 for |T| >= 2^32 (others out of
 // line, exactly): the magnitude taken in one's complement (a negative T comes
 // out 2^-59 smaller in magnitude) and truncated to 53 bits.  The error is below
 // 2^-52 relative plus 2^-59 absolute -- for the non-equilibrium brackets it
 // converts, negligible against the binary64 rounding of the populations.
+template <int SCALE = kScale>
 DF_HD double fixed_to_double_tr(int64_t T) {
   const uint32_t hi = (uint32_t)((uint64_t)T >> 32), lo = (uint32_t)(uint64_t)T;
   const uint32_t s = (uint32_t)((int32_t)hi >> 31);  // 0 or ~0
   const uint32_t ah = hi ^ s, al = lo ^ s;
-  if (ah == 0u) return fixed_to_double_any_slow(T);
+  if (ah == 0u) return fixed_to_double_any_slow(T) * pow2_const(kScale - SCALE);
   const uint32_t lz = clz32(ah);  // 0..31
   const uint32_t nh = funnel_l(al, ah, lz), nl = al << lz;  // bit 63 of (nh:nl) set
   const uint32_t mh = nh >> 11, ml = funnel_r(nl, nh, 11);  // 53 bits, leading one at bit 52
-  // value = (nh:nl) 2^(-lz - 59): biased exponent 1027 - lz; the leading one of
-  // mh (bit 20) adds the final 1 to the exponent field
-  const uint32_t eh = (1026u - lz) * 0x100000u + mh;
+  // value = (nh:nl) 2^(-lz - SCALE): biased exponent 1086 - SCALE - lz; the leading
+  // one of mh (bit 20) adds the final 1 to the exponent field
+  const uint32_t eh = (1085u - (uint32_t)SCALE - lz) * 0x100000u + mh;
   return df::u2d(((uint64_t)(eh | (s & 0x80000000u)) << 32) | (uint64_t)ml);
 }
 
@@ -476,9 +478,9 @@ constexpr uint32_t kTurn06 = 644245094;  // 0.6 2^30
 // 2^59).  Small h are rounded to the fixed point with ties toward +infinity,
 // a bias that leaves the odd moments alone (to_fixed_signed).
 //
-// bgk_brackets: Y of the fixed-point populations F.
+// bgk_brackets: Y of the fixed-point populations F, and u at 2^61.
 template <bool SHIFTED>
-DF_HD void bgk_brackets(const int64_t (&F)[9], const BgkParams& p, int64_t (&Y)[9], bool& bad) {
+DF_HD void bgk_brackets(const int64_t (&F)[9], const BgkParams& p, int64_t (&Y)[9], int64_t& U, int64_t& V, bool& bad) {
   // R: the zeroth moment of the stored values (rho, or DH when shifted)
   const int64_t R = (((F[5] + F[7]) + (F[6] + F[8])) + ((F[1] + F[3]) + (F[2] + F[4]))) + F[0];
   const int64_t d57 = F[5] - F[7], d86 = F[8] - F[6];
@@ -487,7 +489,7 @@ DF_HD void bgk_brackets(const int64_t (&F)[9], const BgkParams& p, int64_t (&Y)[
   const int64_t Rrho = SHIFTED ? R + kOne : R;
   const int64_t I = recip_fixed(Rrho);                 // 2^61 / rho
   const int64_t jx = shl(JX, 5), jy = shl(JY, 5);      // 2^64 j
-  const int64_t U = mulh64(jx, I), V = mulh64(jy, I);  // 2^61 u
+  U = mulh64(jx, I), V = mulh64(jy, I);                // 2^61 u
   const int64_t Ai = round_shr(3 * mulh64(jx, U), 3), Bi = round_shr(3 * mulh64(jy, V), 3);
   const int64_t Xi = round_shr(9 * mulh64(jx, V), 3);
   const int64_t AB = Ai + Bi;
@@ -506,6 +508,12 @@ DF_HD void bgk_brackets(const int64_t (&F)[9], const BgkParams& p, int64_t (&Y)[
   Y[7] = dp - sp - 36 * F[7];
   Y[6] = dm + sm - 36 * F[6];
   Y[8] = dm - sm - 36 * F[8];
+}
+
+template <bool SHIFTED>
+DF_HD void bgk_brackets(const int64_t (&F)[9], const BgkParams& p, int64_t (&Y)[9], bool& bad) {
+  int64_t U, V;
+  bgk_brackets<SHIFTED>(F, p, Y, U, V, bad);
 }
 
 template <bool SHIFTED = false>
