@@ -251,6 +251,7 @@ __global__ void __launch_bounds__(kBlock) k_adj_step(const void* __restrict__ f,
                                                     void* __restrict__ lam_out, double* __restrict__ dom,
                                                     typename AdjTraits<ST>::real om, int nx, int ny, int ld,
                                                     int ftiles) {
+  chain_begin();
   typedef typename AdjTraits<ST>::real R;
   typedef typename AdjTraits<ST>::elem E;
   int x, y;
@@ -268,8 +269,8 @@ __global__ void __launch_bounds__(kBlock) k_adj_step(const void* __restrict__ f,
     R g[9], l[9], mu[9];
 #pragma unroll
     for (int q = 0; q < 9; q++) {
-      g[q] = (R)__ldg(fe + off[q]);
-      l[q] = (R)__ldg(li + ((I)q * P + c0 + y0));
+      g[q] = (R)ld_chain(fe + off[q]);
+      l[q] = (R)ld_chain(li + ((I)q * P + c0 + y0));
     }
     part = reverse_cell(g, l, om, mu);
 #pragma unroll
@@ -288,6 +289,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_adj_step_comp(const float* __rest
                                                          float* __restrict__ lo, double* __restrict__ dom,
                                                          df::AdjDevParams cpar, int nx, int ny, int ld,
                                                          int ftiles) {
+  chain_begin();
   int x, y;
   const bool in = yfast_cell(ftiles, ny, x, y);
   float part = 0.0f;
@@ -300,8 +302,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_adj_step_comp(const float* __rest
     float g[9], l[9], mu[9];
 #pragma unroll
     for (int q = 0; q < 9; q++) {
-      g[q] = __ldg(fe + off[q]);
-      l[q] = __ldg(li + ((I)q * P + c0 + y0));
+      g[q] = ld_chain(fe + off[q]);
+      l[q] = ld_chain(li + ((I)q * P + c0 + y0));
     }
     part = df::adj_step_comp(g, l, mu, cpar);
 #pragma unroll
@@ -359,17 +361,17 @@ cudaError_t dispatch(int what, const AdjLaunch& a) {
         const float* la = static_cast<const float*>(a.lam_in);
         float* lb = static_cast<float*>(a.lam_out);
         if ((unsigned long long)a.ld * (unsigned long long)a.nx * 9ull < (1ull << 32))
-          k_adj_step_comp<uint32_t><<<nb, kBlock, 0, a.stream>>>(fa, la, lb, a.dom, cpar, a.nx, a.ny, a.ld, ft);
+          chained(k_adj_step_comp<uint32_t>, nb, kBlock, a.stream)(fa, la, lb, a.dom, cpar, a.nx, a.ny, a.ld, ft);
         else
-          k_adj_step_comp<size_t><<<nb, kBlock, 0, a.stream>>>(fa, la, lb, a.dom, cpar, a.nx, a.ny, a.ld, ft);
+          chained(k_adj_step_comp<size_t>, nb, kBlock, a.stream)(fa, la, lb, a.dom, cpar, a.nx, a.ny, a.ld, ft);
         break;
       }
       if ((unsigned long long)a.ld * (unsigned long long)a.nx * 9ull < (1ull << 32))
-        k_adj_step<ST, uint32_t><<<nb, kBlock, 0, a.stream>>>(a.f, a.lam_in, a.lam_out, a.dom,
+        chained(k_adj_step<ST, uint32_t>, nb, kBlock, a.stream)(a.f, a.lam_in, a.lam_out, a.dom,
                                                               (typename AdjTraits<ST>::real)a.omega, a.nx, a.ny,
                                                               a.ld, ft);
       else
-        k_adj_step<ST, size_t><<<nb, kBlock, 0, a.stream>>>(a.f, a.lam_in, a.lam_out, a.dom,
+        chained(k_adj_step<ST, size_t>, nb, kBlock, a.stream)(a.f, a.lam_in, a.lam_out, a.dom,
                                                             (typename AdjTraits<ST>::real)a.omega, a.nx, a.ny, a.ld,
                                                             ft);
       break;

@@ -40,12 +40,12 @@ struct alignas(16) Ctrl {
   int where;          // step at which the timeout happened
 };
 
-// Population load: ld.global.cg (L2 only) inside the persistent kernel, the
-// read-only path in the per-step kernel.
+// Population load: ld.global.cg (L2 only) inside the persistent kernel, an
+// ordinary load in the per-step kernels.
 template <bool CG, typename E>
 __device__ __forceinline__ E load_pop(const E* p) {
   if constexpr (CG) return __ldcg(p);
-  else return __ldg(p);
+  else return ld_chain(p);
 }
 
 // One binary64 cell outside the hybrid range: pull, the binary64 operator,
@@ -209,6 +209,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch_kind(const BatchGrid* __re
                                                           const int2* __restrict__ tile_xy,
                                                           const int* __restrict__ tile_grid, int t0, int parity,
                                                           typename S::elem* base) {
+  chain_begin();
   const int t = t0 + (int)blockIdx.x;
   do_tile<S, false, I, KIND>(grids + __ldg(tile_grid + t), __ldg(tile_xy + t), parity, base);
 }
@@ -221,6 +222,7 @@ __global__ void __launch_bounds__(kBatchMaxThreads) k_batch_step(const BatchGrid
                                                                 const int2* __restrict__ tile_xy,
                                                                 const int* __restrict__ tile_grid, int parity,
                                                                 typename S::elem* base) {
+  chain_begin();
   const int t = (int)blockIdx.x;
   do_tile<S, false, I, -1>(grids + __ldg(tile_grid + t), __ldg(tile_xy + t), parity, base);
 }
@@ -230,13 +232,12 @@ cudaError_t launch_kinds(const BatchLaunch& L, int parity) {
   typedef typename S::elem E;
   E* base = static_cast<E*>(L.base);
   const int ntrt = L.ntiles - L.nt_bgk;
+  constexpr int bgk_blocks = MAXT == 128 ? 8 : batch_min_blocks<S>(MAXT);
   constexpr int trt_blocks = MAXT == 128 ? 7 : batch_min_blocks<S>(MAXT);
   if (L.nt_bgk > 0)
-    k_batch_kind<S, I, K_BGK, MAXT, MAXT == 128 ? 8 : batch_min_blocks<S>(MAXT)>
-        <<<L.nt_bgk, L.threads, 0, L.stream>>>(L.grids, L.tile_xy, L.tile_grid, 0, parity, base);
+    chained(k_batch_kind<S, I, K_BGK, MAXT, bgk_blocks>, L.nt_bgk, L.threads, L.stream)(L.grids, L.tile_xy, L.tile_grid, 0, parity, base);
   if (ntrt > 0)
-    k_batch_kind<S, I, K_TRT, MAXT, trt_blocks>
-        <<<ntrt, L.threads, 0, L.stream>>>(L.grids, L.tile_xy, L.tile_grid, L.nt_bgk, parity, base);
+    chained(k_batch_kind<S, I, K_TRT, MAXT, trt_blocks>, ntrt, L.threads, L.stream)(L.grids, L.tile_xy, L.tile_grid, L.nt_bgk, parity, base);
   return cudaGetLastError();
 }
 
@@ -266,7 +267,7 @@ cudaError_t launch_batch(const BatchLaunch& L, int nsteps, int parity0) {
     if (L.threads <= 128 && (!S::ddf || L.threads == 128)) {
       e = launch_kinds<S, I, 128>(L, parity);
     } else if constexpr (S::ddf) {
-      k_batch_step<S, I><<<L.ntiles, L.threads, 0, L.stream>>>(L.grids, L.tile_xy, L.tile_grid, parity, base);
+      chained(k_batch_step<S, I>, L.ntiles, L.threads, L.stream)(L.grids, L.tile_xy, L.tile_grid, parity, base);
       e = cudaGetLastError();
     } else {
       e = L.threads <= 256 ? launch_kinds<S, I, 256>(L, parity) : launch_kinds<S, I, kBatchMaxThreads>(L, parity);

@@ -24,17 +24,19 @@
 
 using namespace plbm;
 
-int plbm::block_for(long long cells) {
+int plbm::block_for(long long cells, bool binary64) {
   static std::atomic<int> sms[64];  // SM count per device, 0 until first asked
+  const int most = binary64 ? (cells <= (1 << 18) ? 64 : 128)
+                            : (cells <= (1 << 17) ? 64 : (cells < (1 << 18) ? 128 : kBlock));
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return kBlock;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return most;
   int n = sms[dev].load(std::memory_order_relaxed);
   if (n < 1) {
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) return kBlock;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) return most;
     sms[dev].store(n, std::memory_order_relaxed);
   }
   const long long per_sm = (cells + n - 1) / n;
-  if (per_sm >= kBlock) return kBlock;
+  if (per_sm >= most) return most;
   return (int)(per_sm < 32 ? 32 : (per_sm + 31) / 32 * 32);
 }
 

@@ -69,12 +69,37 @@ __device__ __forceinline__ int wrap_add(int v, int d, int n) {
 }
 
 // ---------------------------------------------------------------------------
+// Lattice load of the kernels that are launched in chains (plbm_launch.h): an
+// ordinary load that stays behind the kernel's wait for its predecessors (a load
+// through the read-only path could be moved before it).
+__device__ __forceinline__ double ld_chain(const double* p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float ld_chain(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ __half ld_chain(const __half* p) {
+  unsigned short v;
+  asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
+  return __ushort_as_half(v);
+}
+__device__ __forceinline__ __half2 ld_chain(const __half2* p) {
+  unsigned v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return *reinterpret_cast<const __half2*>(&v);
+}
+
+// ---------------------------------------------------------------------------
 // Storage traits: how one population is held in HBM.
 struct StoreF64 {
   typedef double elem;
   typedef double real;
   static constexpr bool ddf = false;
-  __device__ __forceinline__ static double load(const double* p, size_t i) { return __ldg(p + i); }
+  __device__ __forceinline__ static double load(const double* p, size_t i) { return ld_chain(p + i); }
   __device__ __forceinline__ static void store(double* p, size_t i, double v) { p[i] = v; }
 };
 // binary64 populations stored shifted (h = f - w), sim/sim.F90:131
@@ -82,14 +107,14 @@ struct StoreF64Shift {
   typedef double elem;
   typedef double real;
   static constexpr bool ddf = true;
-  __device__ __forceinline__ static double load(const double* p, size_t i) { return __ldg(p + i); }
+  __device__ __forceinline__ static double load(const double* p, size_t i) { return ld_chain(p + i); }
   __device__ __forceinline__ static void store(double* p, size_t i, double v) { p[i] = v; }
 };
 struct StoreF32Dev {
   typedef float elem;
   typedef float real;
   static constexpr bool ddf = true;
-  __device__ __forceinline__ static float load(const float* p, size_t i) { return __ldg(p + i); }
+  __device__ __forceinline__ static float load(const float* p, size_t i) { return ld_chain(p + i); }
   __device__ __forceinline__ static void store(float* p, size_t i, float v) { p[i] = v; }
 };
 constexpr float F16_SCALE = 32768.0f;          // 2^15, PLBM_F16_SCALE_LOG2
@@ -99,7 +124,7 @@ struct StoreF16Dev {
   typedef float real;
   static constexpr bool ddf = true;
   __device__ __forceinline__ static float load(const __half* p, size_t i) {
-    return __half2float(__ldg(p + i)) * F16_INV_SCALE;
+    return __half2float(ld_chain(p + i)) * F16_INV_SCALE;
   }
   __device__ __forceinline__ static void store(__half* p, size_t i, float v) {
     p[i] = __float2half_rn(v * F16_SCALE);

@@ -21,13 +21,60 @@ constexpr int kBlock = 256;
 // partial triple (the staging of plbm_velocity_l2_error_noalloc holds them).
 constexpr int kReduceBlocks = 1216;
 
-// Threads per block for a fused step over `cells` cells: kBlock, or, for a
-// grid with fewer than kBlock cells per SM, the smallest multiple of 32 that
-// covers the grid with one CTA per SM.  A small grid then spreads over every
-// SM instead of a few: each SM's binary64 pipe retires about 2 FMAs per
-// cycle, so a 64^2 grid in 16 CTAs of 256 threads spent ~4.5 us per step in
-// its collision arithmetic.
-int block_for(long long cells);
+// Threads per block for a fused step of `cells` threads (cells, or pairs of
+// cells).  Small CTAs spread a small grid evenly: with kernels chained, the CTAs
+// of the next step take the slots this one leaves, and 256-thread CTAs then end up
+// 3 on some SMs and 1 on others (256^2 RR, 256 / 128 / 64 threads: 5.5 / 5.4 / 5.45 us
+// per step; 320^2 BGK 6.1 / 5.2 / 5.3, 2048^2 RR 149 / 143 / 143; binary32 deviation
+// storage 320^2 2.9 / 2.6 / 2.1, 512^2 3.7 / 3.8 / 5.0).  A grid with less than that per
+// SM takes the smallest multiple of 32 that covers it with one CTA per SM: each
+// SM's binary64 pipe retires about 2 FMAs per cycle, so the strict kernel of a 64^2
+// grid in 16 CTAs of 256 threads spent ~4.5 us per step in its collision.
+int block_for(long long cells, bool binary64);
+
+// Launches of a time loop's kernels, chained by programmatic dependent launch:
+// the next kernel's CTAs are placed while this kernel still runs, and each waits
+// (chain_begin, the first statement of every such kernel) until the kernels
+// before it have completed and their writes are visible.  A dependent launch on
+// one stream otherwise leaves the GPU idle for about 4 us (2 us inside a CUDA
+// graph): 64^2 BGK steps issued one call at a time 5.2 -> 2.7 us each, in a captured
+// loop 2.8 -> 2.45; 2048^2 binary32 47.3 -> 44.8, binary16 30.9 -> 28.3.
+// A kernel lets its successor be placed only after its own wait, so at most two
+// kernels of a chain are on the GPU, the second one waiting; no kernel's reads
+// can be left in an SM's L1 by the time its buffer is overwritten and read again.
+// The lattices are read with ld_chain, not through the read-only path, whose data
+// may not change during a kernel's residence.
+#ifdef __CUDACC__
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+}
+template <typename... P>
+struct Chained {
+  void (*kernel)(P...);
+  unsigned blocks;
+  int threads;
+  cudaStream_t stream;
+  // The launch error is returned, and kept for cudaGetLastError.
+  template <typename... A>
+  cudaError_t operator()(const A&... args) const {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+  }
+};
+template <typename... P>
+Chained<P...> chained(void (*kernel)(P...), unsigned blocks, int threads, cudaStream_t stream) {
+  return {kernel, blocks, threads, stream};
+}
+#endif
 
 // The binary64 reference kernels exist twice, once compiled with FMA
 // contraction (namespace fma) and once without (namespace strict).

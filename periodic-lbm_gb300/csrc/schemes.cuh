@@ -142,15 +142,15 @@ inline Stencil stencil_coefficients(int scheme, double dt) {
 template <class L>
 __device__ __forceinline__ void gather(const double* __restrict__ a, int q, int x, int y, int xp, int xm, int yp,
                                        int ym, int nx, int ny, int ld, double (&v)[9]) {
-  v[C] = __ldg(a + L::off(x, y, q, nx, ny, ld));
-  v[E] = __ldg(a + L::off(xp, y, q, nx, ny, ld));
-  v[N] = __ldg(a + L::off(x, yp, q, nx, ny, ld));
-  v[W] = __ldg(a + L::off(xm, y, q, nx, ny, ld));
-  v[S] = __ldg(a + L::off(x, ym, q, nx, ny, ld));
-  v[NE] = __ldg(a + L::off(xp, yp, q, nx, ny, ld));
-  v[NW] = __ldg(a + L::off(xm, yp, q, nx, ny, ld));
-  v[SW] = __ldg(a + L::off(xm, ym, q, nx, ny, ld));
-  v[SE] = __ldg(a + L::off(xp, ym, q, nx, ny, ld));
+  v[C] = ld_chain(a + L::off(x, y, q, nx, ny, ld));
+  v[E] = ld_chain(a + L::off(xp, y, q, nx, ny, ld));
+  v[N] = ld_chain(a + L::off(x, yp, q, nx, ny, ld));
+  v[W] = ld_chain(a + L::off(xm, y, q, nx, ny, ld));
+  v[S] = ld_chain(a + L::off(x, ym, q, nx, ny, ld));
+  v[NE] = ld_chain(a + L::off(xp, yp, q, nx, ny, ld));
+  v[NW] = ld_chain(a + L::off(xm, yp, q, nx, ny, ld));
+  v[SW] = ld_chain(a + L::off(xm, ym, q, nx, ny, ld));
+  v[SE] = ld_chain(a + L::off(xp, ym, q, nx, ny, ld));
 }
 
 // Tap patterns of the stencil form:
@@ -173,7 +173,7 @@ __device__ __forceinline__ void stencil_pull(const double* __restrict__ src, int
                                              const Stencil& st, double (&f)[9]) {
   const int xp = x + 1 == nx ? 0 : x + 1, xm = x == 0 ? nx - 1 : x - 1;
   const int yp = y + 1 == ny ? 0 : y + 1, ym = y == 0 ? ny - 1 : y - 1;
-  f[0] = __ldg(src + L::off(x, y, 0, nx, ny, ld));
+  f[0] = ld_chain(src + L::off(x, y, 0, nx, ny, ld));
 #pragma unroll
   for (int q = 1; q < 9; q++) {
     double v[9];

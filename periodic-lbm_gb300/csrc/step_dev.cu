@@ -29,6 +29,7 @@ template <class L, class S, int KIND, bool PUSH>
 __global__ void __launch_bounds__(kBlock) k_step_dev(const typename S::elem* __restrict__ src,
                                                     typename S::elem* __restrict__ dst, int nx, int ny,
                                                     int ld, int ftiles, CollParams p) {
+  chain_begin();
   int x, y;
   if (!dev_cell<L>(ftiles, nx, ny, x, y)) return;
   float h[9];
@@ -98,6 +99,7 @@ template <class S, int KIND, typename I>
 __global__ void __launch_bounds__(kBlock) k_step_dev_pull(const typename S::elem* __restrict__ src,
                                                          typename S::elem* __restrict__ dst, int nx, int ny,
                                                          int ld, int ftiles, ShiftParamsF p) {
+  chain_begin();
   const int x = blockIdx.x / ftiles;
   const int y = (blockIdx.x - x * ftiles) * blockDim.x + threadIdx.x;
   if (y >= ny) return;
@@ -110,7 +112,7 @@ __global__ void __launch_bounds__(kBlock) k_step_dev_pull(const typename S::elem
   if constexpr (std::is_same<S, StoreF16Dev>::value) {
     float H[9];
 #pragma unroll
-    for (int q = 0; q < 9; q++) H[q] = __half2float(__ldg(src + offs[q]));
+    for (int q = 0; q < 9; q++) H[q] = __half2float(ld_chain(src + offs[q]));
     if constexpr (KIND == K_TRT) coll_trt_shift<float, true>(H, p.a, p.b, p.c);
     else if constexpr (KIND == K_RR) coll_rr_shift<float, true>(H, p.a, p.b, p.c);
     else coll_bgk_shift_f16scaled(H, p.a);
@@ -136,6 +138,7 @@ __global__ void __launch_bounds__(kBlock) k_step_dev_pull(const typename S::elem
 template <int KIND, typename I>
 __global__ void __launch_bounds__(kBlock) k_step_f16_pull2(const __half* __restrict__ src, __half* __restrict__ dst,
                                                           int nx, int ny, int ld, int ftiles, ShiftParamsF p) {
+  chain_begin();
   const int x = blockIdx.x / ftiles;
   const int y = 2 * ((blockIdx.x - x * ftiles) * blockDim.x + threadIdx.x);
   if (y >= ny) return;
@@ -144,16 +147,16 @@ __global__ void __launch_bounds__(kBlock) k_step_f16_pull2(const __half* __restr
   const I y0 = (I)y, y1 = (I)(y + 1), ym = (I)wrap_m(y, ny), yp = (I)wrap_p(y + 1, ny);
   const __half2* s2 = reinterpret_cast<const __half2*>(src);
   float A[9], B[9];
-  const float2 v0 = __half22float2(__ldg(s2 + (c0 + y0) / 2));
-  const float2 v1 = __half22float2(__ldg(s2 + (P + cm + y0) / 2));
-  const float2 v3 = __half22float2(__ldg(s2 + (3 * P + cp + y0) / 2));
+  const float2 v0 = __half22float2(ld_chain(s2 + (c0 + y0) / 2));
+  const float2 v1 = __half22float2(ld_chain(s2 + (P + cm + y0) / 2));
+  const float2 v3 = __half22float2(ld_chain(s2 + (3 * P + cp + y0) / 2));
   A[0] = v0.x, B[0] = v0.y, A[1] = v1.x, B[1] = v1.y, A[3] = v3.x, B[3] = v3.y;
-  A[2] = __half2float(__ldg(src + 2 * P + c0 + ym)), B[2] = __half2float(__ldg(src + 2 * P + c0 + y0));
-  A[4] = __half2float(__ldg(src + 4 * P + c0 + y1)), B[4] = __half2float(__ldg(src + 4 * P + c0 + yp));
-  A[5] = __half2float(__ldg(src + 5 * P + cm + ym)), B[5] = __half2float(__ldg(src + 5 * P + cm + y0));
-  A[6] = __half2float(__ldg(src + 6 * P + cp + ym)), B[6] = __half2float(__ldg(src + 6 * P + cp + y0));
-  A[7] = __half2float(__ldg(src + 7 * P + cp + y1)), B[7] = __half2float(__ldg(src + 7 * P + cp + yp));
-  A[8] = __half2float(__ldg(src + 8 * P + cm + y1)), B[8] = __half2float(__ldg(src + 8 * P + cm + yp));
+  A[2] = __half2float(ld_chain(src + 2 * P + c0 + ym)), B[2] = __half2float(ld_chain(src + 2 * P + c0 + y0));
+  A[4] = __half2float(ld_chain(src + 4 * P + c0 + y1)), B[4] = __half2float(ld_chain(src + 4 * P + c0 + yp));
+  A[5] = __half2float(ld_chain(src + 5 * P + cm + ym)), B[5] = __half2float(ld_chain(src + 5 * P + cm + y0));
+  A[6] = __half2float(ld_chain(src + 6 * P + cp + ym)), B[6] = __half2float(ld_chain(src + 6 * P + cp + y0));
+  A[7] = __half2float(ld_chain(src + 7 * P + cp + y1)), B[7] = __half2float(ld_chain(src + 7 * P + cp + yp));
+  A[8] = __half2float(ld_chain(src + 8 * P + cm + y1)), B[8] = __half2float(ld_chain(src + 8 * P + cm + yp));
   if constexpr (KIND == K_TRT) {
     coll_trt_shift<float, true>(A, p.a, p.b, p.c);
     coll_trt_shift<float, true>(B, p.a, p.b, p.c);
@@ -202,7 +205,7 @@ inline int tiles(int n) { return (n + kBlock - 1) / kBlock; }
 
 template <class L, class S, bool PUSH>
 cudaError_t launch_dev(int kind, const Sweep& s, const CollParams& p) {
-  const int bs = block_for((long long)s.nx * s.ny);
+  const int bs = block_for((long long)s.nx * s.ny, false);
   const int ft = ((L::x_fast ? s.nx : s.ny) + bs - 1) / bs;
   const long long blocks = (long long)ft * (L::x_fast ? s.ny : s.nx);
   if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
@@ -210,9 +213,9 @@ cudaError_t launch_dev(int kind, const Sweep& s, const CollParams& p) {
   const E* a = static_cast<const E*>(s.src);
   E* b = static_cast<E*>(s.dst);
   switch (kind) {
-    case K_BGK: k_step_dev<L, S, K_BGK, PUSH><<<(unsigned)blocks, bs, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, p); break;
-    case K_TRT: k_step_dev<L, S, K_TRT, PUSH><<<(unsigned)blocks, bs, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, p); break;
-    case K_RR: k_step_dev<L, S, K_RR, PUSH><<<(unsigned)blocks, bs, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, p); break;
+    case K_BGK: chained(k_step_dev<L, S, K_BGK, PUSH>, (unsigned)blocks, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p); break;
+    case K_TRT: chained(k_step_dev<L, S, K_TRT, PUSH>, (unsigned)blocks, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p); break;
+    case K_RR: chained(k_step_dev<L, S, K_RR, PUSH>, (unsigned)blocks, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p); break;
     default: return cudaErrorNotSupported;
   }
   return cudaGetLastError();
@@ -236,7 +239,7 @@ cudaError_t launch_collide_dev(int kind, const Sweep& s, const CollParams& p) {
 
 template <class S, typename I>
 cudaError_t launch_pull_dev(int kind, const Sweep& s, const CollParams& cp) {
-  const int bs = block_for((long long)s.nx * s.ny);
+  const int bs = block_for((long long)s.nx * s.ny, false);
   const int ft = (s.ny + bs - 1) / bs;
   const long long blocks = (long long)ft * s.nx;
   if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
@@ -246,9 +249,9 @@ cudaError_t launch_pull_dev(int kind, const Sweep& s, const CollParams& cp) {
   const ShiftParamsF p = shift_params(kind, cp);
   const unsigned nb = (unsigned)blocks;
   switch (kind) {
-    case K_BGK: k_step_dev_pull<S, K_BGK, I><<<nb, bs, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, p); break;
-    case K_TRT: k_step_dev_pull<S, K_TRT, I><<<nb, bs, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, p); break;
-    case K_RR: k_step_dev_pull<S, K_RR, I><<<nb, bs, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, p); break;
+    case K_BGK: chained(k_step_dev_pull<S, K_BGK, I>, nb, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p); break;
+    case K_TRT: chained(k_step_dev_pull<S, K_TRT, I>, nb, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p); break;
+    case K_RR: chained(k_step_dev_pull<S, K_RR, I>, nb, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p); break;
     default: return cudaErrorNotSupported;
   }
   return cudaGetLastError();
@@ -256,7 +259,7 @@ cudaError_t launch_pull_dev(int kind, const Sweep& s, const CollParams& cp) {
 
 template <typename I>
 cudaError_t launch_f16_pull2(int kind, const Sweep& s, const CollParams& cp) {
-  const int bs = block_for((long long)s.nx * (s.ny / 2));
+  const int bs = block_for((long long)s.nx * (s.ny / 2), false);
   const int ft = (s.ny / 2 + bs - 1) / bs;
   const long long blocks = (long long)ft * s.nx;
   if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
@@ -265,9 +268,9 @@ cudaError_t launch_f16_pull2(int kind, const Sweep& s, const CollParams& cp) {
   const ShiftParamsF p = shift_params(kind, cp);
   const unsigned nb = (unsigned)blocks;
   switch (kind) {
-    case K_BGK: k_step_f16_pull2<K_BGK, I><<<nb, bs, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, p); break;
-    case K_TRT: k_step_f16_pull2<K_TRT, I><<<nb, bs, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, p); break;
-    case K_RR: k_step_f16_pull2<K_RR, I><<<nb, bs, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, p); break;
+    case K_BGK: chained(k_step_f16_pull2<K_BGK, I>, nb, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p); break;
+    case K_TRT: chained(k_step_f16_pull2<K_TRT, I>, nb, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p); break;
+    case K_RR: chained(k_step_f16_pull2<K_RR, I>, nb, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p); break;
     default: return cudaErrorNotSupported;
   }
   return cudaGetLastError();

@@ -16,6 +16,7 @@ template <class S>
 __global__ void __launch_bounds__(kBlock) k_step_dev_df(const typename S::elem* __restrict__ src,
                                                        typename S::elem* __restrict__ dst, int nx, int ny, int ld,
                                                        int ftiles, df::DfParams p) {
+  chain_begin();
   const int x = blockIdx.x / ftiles;
   const int y = (blockIdx.x - x * ftiles) * blockDim.x + threadIdx.x;
   if (y >= ny) return;
@@ -36,6 +37,7 @@ template <class S, typename I>
 __global__ void __launch_bounds__(kBlock) k_step_dev_comp(const typename S::elem* __restrict__ src,
                                                          typename S::elem* __restrict__ dst, int nx, int ny, int ld,
                                                          int ftiles, df::DevParams p) {
+  chain_begin();
   const int x = blockIdx.x / ftiles;
   const int y = (blockIdx.x - x * ftiles) * blockDim.x + threadIdx.x;
   if (y >= ny) return;
@@ -63,6 +65,7 @@ template <class S, int KIND>
 __global__ void __launch_bounds__(kBlock) k_step_dev_d(const typename S::elem* __restrict__ src,
                                                       typename S::elem* __restrict__ dst, int nx, int ny, int ld,
                                                       int ftiles, CollParams p) {
+  chain_begin();
   const int x = blockIdx.x / ftiles;
   const int y = (blockIdx.x - x * ftiles) * blockDim.x + threadIdx.x;
   if (y >= ny) return;
@@ -103,13 +106,13 @@ cudaError_t step_pull_dev_hi(int storage, int math, int kind, const Sweep& s, co
     if (storage == ST_F32DEV) {
       const float* a = static_cast<const float*>(s.src);
       float* b = static_cast<float*>(s.dst);
-      if (small) k_step_dev_comp<StoreF32Dev, uint32_t><<<nb, kBlock, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, p);
-      else k_step_dev_comp<StoreF32Dev, size_t><<<nb, kBlock, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, p);
+      if (small) chained(k_step_dev_comp<StoreF32Dev, uint32_t>, nb, kBlock, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p);
+      else chained(k_step_dev_comp<StoreF32Dev, size_t>, nb, kBlock, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p);
     } else if (storage == ST_F16DEV) {
       const __half* a = static_cast<const __half*>(s.src);
       __half* b = static_cast<__half*>(s.dst);
-      if (small) k_step_dev_comp<StoreF16Dev, uint32_t><<<nb, kBlock, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, p);
-      else k_step_dev_comp<StoreF16Dev, size_t><<<nb, kBlock, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, p);
+      if (small) chained(k_step_dev_comp<StoreF16Dev, uint32_t>, nb, kBlock, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p);
+      else chained(k_step_dev_comp<StoreF16Dev, size_t>, nb, kBlock, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p);
     } else {
       return cudaErrorInvalidValue;
     }
@@ -126,10 +129,10 @@ cudaError_t step_pull_dev_hi(int storage, int math, int kind, const Sweep& s, co
     p.ws3 = split_const(3.0 * WS);
     p.wd3 = split_const(3.0 * WD);
     if (storage == ST_F32DEV)
-      k_step_dev_df<StoreF32Dev><<<nb, kBlock, 0, s.stream>>>(static_cast<const float*>(s.src),
+      chained(k_step_dev_df<StoreF32Dev>, nb, kBlock, s.stream)(static_cast<const float*>(s.src),
                                                               static_cast<float*>(s.dst), s.nx, s.ny, s.ld, ft, p);
     else if (storage == ST_F16DEV)
-      k_step_dev_df<StoreF16Dev><<<nb, kBlock, 0, s.stream>>>(static_cast<const __half*>(s.src),
+      chained(k_step_dev_df<StoreF16Dev>, nb, kBlock, s.stream)(static_cast<const __half*>(s.src),
                                                               static_cast<__half*>(s.dst), s.nx, s.ny, s.ld, ft, p);
     else
       return cudaErrorInvalidValue;
@@ -137,13 +140,13 @@ cudaError_t step_pull_dev_hi(int storage, int math, int kind, const Sweep& s, co
   }
 #define PLBM_DEVD(S, E)                                                                                      \
   switch (kind) {                                                                                            \
-    case K_BGK: k_step_dev_d<S, K_BGK><<<nb, kBlock, 0, s.stream>>>(static_cast<const E*>(s.src),            \
+    case K_BGK: chained(k_step_dev_d<S, K_BGK>, nb, kBlock, s.stream)(static_cast<const E*>(s.src),            \
                                                                     static_cast<E*>(s.dst), s.nx, s.ny, s.ld, \
                                                                     ft, cp); break;                           \
-    case K_TRT: k_step_dev_d<S, K_TRT><<<nb, kBlock, 0, s.stream>>>(static_cast<const E*>(s.src),            \
+    case K_TRT: chained(k_step_dev_d<S, K_TRT>, nb, kBlock, s.stream)(static_cast<const E*>(s.src),            \
                                                                     static_cast<E*>(s.dst), s.nx, s.ny, s.ld, \
                                                                     ft, cp); break;                           \
-    case K_RR: k_step_dev_d<S, K_RR><<<nb, kBlock, 0, s.stream>>>(static_cast<const E*>(s.src),              \
+    case K_RR: chained(k_step_dev_d<S, K_RR>, nb, kBlock, s.stream)(static_cast<const E*>(s.src),              \
                                                                   static_cast<E*>(s.dst), s.nx, s.ny, s.ld,   \
                                                                   ft, cp); break;                             \
     default: return cudaErrorNotSupported;                                                                   \

@@ -52,6 +52,7 @@ __device__ __forceinline__ bool cell_of<XFast>(int ftiles, int nx, int ny, int& 
 template <class L, int KIND, bool SHIFT, bool PUSH>
 __global__ void __launch_bounds__(kBlock) k_step(const double* __restrict__ src, double* __restrict__ dst,
                                                 int nx, int ny, int ld, int ftiles, CollParams p) {
+  chain_begin();
   int x, y;
   if (!cell_of<L>(ftiles, nx, ny, x, y)) return;
   double f[9];
@@ -59,7 +60,7 @@ __global__ void __launch_bounds__(kBlock) k_step(const double* __restrict__ src,
   for (int q = 0; q < 9; q++) {
     const int sx = PUSH ? x : wrap_add(x, -cx_of(q), nx);
     const int sy = PUSH ? y : wrap_add(y, -cy_of(q), ny);
-    f[q] = __ldg(src + L::off(sx, sy, q, nx, ny, ld));
+    f[q] = ld_chain(src + L::off(sx, sy, q, nx, ny, ld));
   }
   if (SHIFT) collide_shift<KIND, double>(f, p);
   else collide_ref<KIND>(f, p);
@@ -122,6 +123,7 @@ template <int TAPS>
 __global__ void __launch_bounds__(kBlock) k_step_scheme(const double* __restrict__ src, double* __restrict__ dst,
                                                        int nx, int ny, int ld, int ftiles, sch::Stencil st,
                                                        CollParams p) {
+  chain_begin();
   int x, y;
   if (!cell_of<YFast>(ftiles, nx, ny, x, y)) return;
   double f[9];
@@ -176,7 +178,7 @@ inline int tiles(int n) { return (n + kBlock - 1) / kBlock; }
 
 template <class L, bool SHIFT, bool PUSH>
 cudaError_t launch_step(int kind, const Sweep& s, const CollParams& p) {
-  const int bs = block_for((long long)s.nx * s.ny);
+  const int bs = block_for((long long)s.nx * s.ny, true);
   const int nfast = L::x_fast ? s.nx : s.ny;
   const int ft = (nfast + bs - 1) / bs;
   const int nslow = L::x_fast ? s.ny : s.nx;
@@ -184,7 +186,7 @@ cudaError_t launch_step(int kind, const Sweep& s, const CollParams& p) {
   if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   const double* a = static_cast<const double*>(s.src);
   double* b = static_cast<double*>(s.dst);
-#define PLBM_STEP(K) k_step<L, K, SHIFT, PUSH><<<(unsigned)blocks, bs, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, p)
+#define PLBM_STEP(K) chained(k_step<L, K, SHIFT, PUSH>, (unsigned)blocks, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p)
 #ifdef PLBM_STRICT
   switch (kind) {
     case K_BGK: PLBM_STEP(K_BGK); break;
@@ -276,9 +278,9 @@ cudaError_t step_scheme_f64(int scheme, const Sweep& s, double dt, const CollPar
   double* b = static_cast<double*>(s.dst);
   const unsigned nb = (unsigned)blocks;
   switch (sch::taps_of(scheme)) {
-    case sch::TAPS_LINE: k_step_scheme<sch::TAPS_LINE><<<nb, kBlock, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, st, p); break;
-    case sch::TAPS_AXIS3: k_step_scheme<sch::TAPS_AXIS3><<<nb, kBlock, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, st, p); break;
-    default: k_step_scheme<sch::TAPS_FULL><<<nb, kBlock, 0, s.stream>>>(a, b, s.nx, s.ny, s.ld, ft, st, p); break;
+    case sch::TAPS_LINE: chained(k_step_scheme<sch::TAPS_LINE>, nb, kBlock, s.stream)(a, b, s.nx, s.ny, s.ld, ft, st, p); break;
+    case sch::TAPS_AXIS3: chained(k_step_scheme<sch::TAPS_AXIS3>, nb, kBlock, s.stream)(a, b, s.nx, s.ny, s.ld, ft, st, p); break;
+    default: chained(k_step_scheme<sch::TAPS_FULL>, nb, kBlock, s.stream)(a, b, s.nx, s.ny, s.ld, ft, st, p); break;
   }
   return cudaGetLastError();
 }

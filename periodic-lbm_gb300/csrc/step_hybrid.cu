@@ -39,7 +39,7 @@ __device__ __noinline__ void hybrid_fallback_cell(const double* __restrict__ src
 #pragma unroll
   for (int q = 0; q < 9; q++) {
     const int sx = wrap_add(x, -cx_of(q), nx), sy = wrap_add(y, -cy_of(q), ny);
-    f[q] = src[YFast::off(sx, sy, q, nx, ny, ld)];
+    f[q] = ld_chain(src + YFast::off(sx, sy, q, nx, ny, ld));
   }
   collide_ref<KIND>(f, p);
 #pragma unroll
@@ -58,6 +58,7 @@ constexpr int hybrid_min_blocks(int kind) { return kind == K_RR ? 3 : 4; }
 template <typename I, int KIND>
 __global__ void __launch_bounds__(kBlock, hybrid_min_blocks(KIND)) k_step_hybrid(const double* __restrict__ src, double* __restrict__ dst,
                                                        int nx, int ny, int ld, int ftiles, HybridArgs a) {
+  chain_begin();
   const int x = blockIdx.x / ftiles;
   const int y = (blockIdx.x - x * ftiles) * blockDim.x + threadIdx.x;
   if (y >= ny) return;
@@ -66,15 +67,15 @@ __global__ void __launch_bounds__(kBlock, hybrid_min_blocks(KIND)) k_step_hybrid
   const I y0 = (I)y, ym = (I)wrap_m(y, ny), yp = (I)wrap_p(y, ny);
   double f[9];
   // pull: f_q(x, y) = f_q(x - cx_q, y - cy_q) of the source lattice
-  f[0] = __ldg(src + (c0 + y0));
-  f[1] = __ldg(src + (P + cm + y0));
-  f[2] = __ldg(src + (2 * P + c0 + ym));
-  f[3] = __ldg(src + (3 * P + cp + y0));
-  f[4] = __ldg(src + (4 * P + c0 + yp));
-  f[5] = __ldg(src + (5 * P + cm + ym));
-  f[6] = __ldg(src + (6 * P + cp + ym));
-  f[7] = __ldg(src + (7 * P + cp + yp));
-  f[8] = __ldg(src + (8 * P + cm + yp));
+  f[0] = ld_chain(src + (c0 + y0));
+  f[1] = ld_chain(src + (P + cm + y0));
+  f[2] = ld_chain(src + (2 * P + c0 + ym));
+  f[3] = ld_chain(src + (3 * P + cp + y0));
+  f[4] = ld_chain(src + (4 * P + c0 + yp));
+  f[5] = ld_chain(src + (5 * P + cm + ym));
+  f[6] = ld_chain(src + (6 * P + cp + ym));
+  f[7] = ld_chain(src + (7 * P + cp + yp));
+  f[8] = ld_chain(src + (8 * P + cm + yp));
   bool bad = false;
   if (KIND == K_TRT) hy::trt_fma(f, a.trt, bad);
   else if (KIND == K_RR) hy::rr_fma(f, a.rr, a.rr1, bad);
@@ -107,6 +108,7 @@ template <int TAPS, int KIND>
 __global__ void __launch_bounds__(kBlock) k_step_scheme_hybrid(const double* __restrict__ src,
                                                               double* __restrict__ dst, int nx, int ny, int ld,
                                                               int ftiles, sch::Stencil st, HybridArgs a) {
+  chain_begin();
   const int x = blockIdx.x / ftiles;
   const int y = (blockIdx.x - x * ftiles) * blockDim.x + threadIdx.x;
   if (y >= ny) return;
@@ -196,6 +198,7 @@ template <int FORM, int KIND, int TX>
 __global__ void __launch_bounds__(256, KIND == K_RR ? 3 : 4)
     k_step_scheme_fixed(const double* __restrict__ src, double* __restrict__ dst, int nx, int ny, int ld, int ytiles,
                         SchemeFx sc, sch::Stencil st, HybridArgs a) {
+  chain_begin();
   constexpr int ROWS = 34;
   __shared__ int64_t sm[8][TX + 2][ROWS];
   __shared__ int tile_bad;
@@ -211,7 +214,7 @@ __global__ void __launch_bounds__(256, KIND == K_RR ? 3 : 4)
     auto load = [&](int c, int r) {
       const int gx = x0 - 1 + c, gy = y0 - 1 + r;
       if (gx > nx || gy > ny) return 0.0;  // past the last cell's neighbours
-      return __ldg(f + (size_t)(gx < 0 ? nx - 1 : (gx == nx ? 0 : gx)) * ld +
+      return ld_chain(f + (size_t)(gx < 0 ? nx - 1 : (gx == nx ? 0 : gx)) * ld +
                    (gy < 0 ? ny - 1 : (gy == ny ? 0 : gy)));
     };
     auto convert = [&](double d) {
@@ -241,7 +244,7 @@ __global__ void __launch_bounds__(256, KIND == K_RR ? 3 : 4)
     bool bad = tile_bad;
     int64_t F[9], Z[9];
     if (!bad) {
-      F[0] = hy::to_fixed_nonneg<1022>(__ldg(src + o), bad);
+      F[0] = hy::to_fixed_nonneg<1022>(ld_chain(src + o), bad);
       Z[0] = hy::shl(F[0], 2);
 #pragma unroll
       for (int q = 1; q < 9; q++) {
@@ -285,7 +288,7 @@ __device__ __noinline__ void push_fallback_cell(const double* __restrict__ src, 
                                                 int y, int nx, int ny, int ld, const CollParams& p, int report) {
   double f[9];
 #pragma unroll
-  for (int q = 0; q < 9; q++) f[q] = src[XFast::off(x, y, q, nx, ny, ld)];
+  for (int q = 0; q < 9; q++) f[q] = ld_chain(src + XFast::off(x, y, q, nx, ny, ld));
   collide_shift<KIND, double>(f, p);
 #pragma unroll
   for (int q = 0; q < 9; q++) dst[XFast::off(wrap_add(x, cx_of(q), nx), wrap_add(y, cy_of(q), ny), q, nx, ny, ld)] = f[q];
@@ -297,6 +300,7 @@ __global__ void __launch_bounds__(kBlock, hybrid_min_blocks(KIND)) k_push_hybrid
                                                                                 double* __restrict__ dst, int nx,
                                                                                 int ny, int ld, int ftiles,
                                                                                 HybridArgs a) {
+  chain_begin();
   const int y = blockIdx.x / ftiles;
   const int x = (blockIdx.x - y * ftiles) * blockDim.x + threadIdx.x;
   if (x >= nx) return;
@@ -304,7 +308,7 @@ __global__ void __launch_bounds__(kBlock, hybrid_min_blocks(KIND)) k_push_hybrid
   const I o = (I)y * L + (I)x;
   double f[9];
 #pragma unroll
-  for (int q = 0; q < 9; q++) f[q] = __ldg(src + ((I)q * P + o));
+  for (int q = 0; q < 9; q++) f[q] = ld_chain(src + ((I)q * P + o));
   bool bad = false;
   if (KIND == K_TRT) hy::trt_fma<true>(f, a.trt, bad);
   else if (KIND == K_RR) hy::rr_fma<true>(f, a.rr, a.rr1, bad);
@@ -332,9 +336,9 @@ cudaError_t launch_hybrid(const Sweep& s, unsigned blocks, int bs, int ft, const
   const double* src = static_cast<const double*>(s.src);
   double* dst = static_cast<double*>(s.dst);
   if ((unsigned long long)s.ld * (unsigned long long)s.nx * 9ull < (1ull << 32))
-    k_step_hybrid<uint32_t, KIND><<<blocks, bs, 0, s.stream>>>(src, dst, s.nx, s.ny, s.ld, ft, a);
+    chained(k_step_hybrid<uint32_t, KIND>, blocks, bs, s.stream)(src, dst, s.nx, s.ny, s.ld, ft, a);
   else
-    k_step_hybrid<size_t, KIND><<<blocks, bs, 0, s.stream>>>(src, dst, s.nx, s.ny, s.ld, ft, a);
+    chained(k_step_hybrid<size_t, KIND>, blocks, bs, s.stream)(src, dst, s.nx, s.ny, s.ld, ft, a);
   return cudaGetLastError();
 }
 
@@ -367,7 +371,7 @@ HybridArgs hybrid_args(const CollParams& cp, bool report) {
 
 cudaError_t step_pull_fixed(int kind, const Sweep& s, const CollParams& cp, bool report) {
   if (kind != K_BGK && kind != K_TRT && kind != K_RR) return cudaErrorNotSupported;
-  const int bs = block_for((long long)s.nx * s.ny);
+  const int bs = block_for((long long)s.nx * s.ny, true);
   const int ft = (s.ny + bs - 1) / bs;
   const long long blocks = (long long)ft * s.nx;
   if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
@@ -379,7 +383,7 @@ cudaError_t step_pull_fixed(int kind, const Sweep& s, const CollParams& cp, bool
 
 cudaError_t step_push_fixed(int kind, const Sweep& s, const CollParams& cp, bool report) {
   if (kind != K_BGK && kind != K_TRT && kind != K_RR) return cudaErrorNotSupported;
-  const int bs = block_for((long long)s.nx * s.ny);
+  const int bs = block_for((long long)s.nx * s.ny, true);
   const int ft = (s.nx + bs - 1) / bs;
   const long long blocks = (long long)ft * s.ny;
   if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
@@ -390,9 +394,9 @@ cudaError_t step_push_fixed(int kind, const Sweep& s, const CollParams& cp, bool
   const bool small = (unsigned long long)s.ld * (unsigned long long)s.ny * 9ull < (1ull << 32);
 #define PLBM_PUSH_HY(I)                                                                                      \
   switch (kind) {                                                                                            \
-    case K_BGK: k_push_hybrid<I, K_BGK><<<nb, bs, 0, s.stream>>>(src, dst, s.nx, s.ny, s.ld, ft, a); break; \
-    case K_TRT: k_push_hybrid<I, K_TRT><<<nb, bs, 0, s.stream>>>(src, dst, s.nx, s.ny, s.ld, ft, a); break; \
-    default: k_push_hybrid<I, K_RR><<<nb, bs, 0, s.stream>>>(src, dst, s.nx, s.ny, s.ld, ft, a); break;     \
+    case K_BGK: chained(k_push_hybrid<I, K_BGK>, nb, bs, s.stream)(src, dst, s.nx, s.ny, s.ld, ft, a); break; \
+    case K_TRT: chained(k_push_hybrid<I, K_TRT>, nb, bs, s.stream)(src, dst, s.nx, s.ny, s.ld, ft, a); break; \
+    default: chained(k_push_hybrid<I, K_RR>, nb, bs, s.stream)(src, dst, s.nx, s.ny, s.ld, ft, a); break;     \
   }
   if (small) {
     PLBM_PUSH_HY(uint32_t)
@@ -456,9 +460,9 @@ void launch_scheme_fixed(int kind, const Sweep& s, const SchemeFx& c, const sch:
   double* dst = static_cast<double*>(s.dst);
   const int yt = (s.ny + 31) / 32;
   const unsigned nb = (unsigned)((long long)yt * ((s.nx + TX - 1) / TX));
-  if (kind == K_TRT) k_step_scheme_fixed<FORM, K_TRT, TX><<<nb, 256, 0, s.stream>>>(src, dst, s.nx, s.ny, s.ld, yt, c, st, a);
-  else if (kind == K_RR) k_step_scheme_fixed<FORM, K_RR, TX><<<nb, 256, 0, s.stream>>>(src, dst, s.nx, s.ny, s.ld, yt, c, st, a);
-  else k_step_scheme_fixed<FORM, K_BGK, TX><<<nb, 256, 0, s.stream>>>(src, dst, s.nx, s.ny, s.ld, yt, c, st, a);
+  if (kind == K_TRT) chained(k_step_scheme_fixed<FORM, K_TRT, TX>, nb, 256, s.stream)(src, dst, s.nx, s.ny, s.ld, yt, c, st, a);
+  else if (kind == K_RR) chained(k_step_scheme_fixed<FORM, K_RR, TX>, nb, 256, s.stream)(src, dst, s.nx, s.ny, s.ld, yt, c, st, a);
+  else chained(k_step_scheme_fixed<FORM, K_BGK, TX>, nb, 256, s.stream)(src, dst, s.nx, s.ny, s.ld, yt, c, st, a);
 }
 }  // namespace
 
@@ -492,9 +496,9 @@ cudaError_t step_scheme_fixed(int scheme, int kind, const Sweep& s, double dt, c
   const unsigned nb = (unsigned)blocks;
 #define PLBM_SCH_HY(T)                                                                                        \
   switch (kind) {                                                                                             \
-    case K_BGK: k_step_scheme_hybrid<T, K_BGK><<<nb, kBlock, 0, s.stream>>>(src, dst, s.nx, s.ny, s.ld, ft, st, a); break; \
-    case K_TRT: k_step_scheme_hybrid<T, K_TRT><<<nb, kBlock, 0, s.stream>>>(src, dst, s.nx, s.ny, s.ld, ft, st, a); break; \
-    default: k_step_scheme_hybrid<T, K_RR><<<nb, kBlock, 0, s.stream>>>(src, dst, s.nx, s.ny, s.ld, ft, st, a); break;     \
+    case K_BGK: chained(k_step_scheme_hybrid<T, K_BGK>, nb, kBlock, s.stream)(src, dst, s.nx, s.ny, s.ld, ft, st, a); break; \
+    case K_TRT: chained(k_step_scheme_hybrid<T, K_TRT>, nb, kBlock, s.stream)(src, dst, s.nx, s.ny, s.ld, ft, st, a); break; \
+    default: chained(k_step_scheme_hybrid<T, K_RR>, nb, kBlock, s.stream)(src, dst, s.nx, s.ny, s.ld, ft, st, a); break;     \
   }
   switch (sch::taps_of(scheme)) {
     case sch::TAPS_LINE: PLBM_SCH_HY(sch::TAPS_LINE) break;
