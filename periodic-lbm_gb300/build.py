@@ -28,6 +28,7 @@ UNITS = [
     ("step_f64.cu", "step_f64_fma.o", ["--fmad=true"]),
     ("step_f64.cu", "step_f64_strict.o", ["--fmad=false", "-DPLBM_STRICT"]),
     ("step_dev.cu", "step_dev.o", ["--fmad=true"]),
+    ("step_march.cu", "step_march.o", ["--fmad=false"]),
     ("step_df64.cu", "step_df64.o", ["--fmad=false"]),
     ("step_hybrid.cu", "step_hybrid.o", ["--fmad=true"]),
     ("fields.cu", "fields.o", ["--fmad=false"]),

@@ -81,6 +81,19 @@ struct DevParams {
   float om_lo;
 };
 
+inline DevParams dev_params(double omega) {
+  const double w[3] = {4.0 / 9.0, 1.0 / 9.0, 1.0 / 36.0};
+  DevParams p;
+  for (int i = 0; i < 3; i++) {
+    const float hi = (float)w[i], hi3 = (float)(3.0 * w[i]);
+    p.w[i] = make(hi, (float)(w[i] - (double)hi));
+    p.w3[i] = make(hi3, (float)(3.0 * w[i] - (double)hi3));
+  }
+  p.om_hi = (float)omega;
+  p.om_lo = (float)(omega - (double)p.om_hi);
+  return p;
+}
+
 DF_HD df64 add_lazy(df64 a, df64 b) {
   df64 s = two_sum(a.hi, b.hi);
   s.lo += a.lo + b.lo;
@@ -109,56 +122,104 @@ DF_HD float relax(float h, float d, float om_hi, float om_lo) {
   return t + c;
 }
 
-// The update of a pair (q, qbar = -q): heq = a +- b with a = w (drho + rho nl_q)
-// (nl_q = 4.5 (c_q.u)^2 - 1.5 u^2) and b = 3 w c_q.j.  With the pair's exact
+// The same operations on values of type V (one cell or a pair of cells).
+template <typename V>
+struct dfv {
+  V hi, lo;
+};
+template <typename V>
+DF_HD dfv<V> two_sum_v(V a, V b) {
+  const V s = vadd(a, b), bb = vsub(s, a);
+  return {s, vadd(vsub(a, vsub(s, bb)), vsub(b, bb))};
+}
+template <typename V>
+DF_HD dfv<V> two_diff_v(V a, V b) {  // a - b
+  const V s = vsub(a, b), bb = vsub(s, a);
+  return {s, vsub(vsub(a, vsub(s, bb)), vadd(b, bb))};
+}
+template <typename V>
+DF_HD dfv<V> add_v(dfv<V> a, dfv<V> b) {
+  dfv<V> s = two_sum_v(a.hi, b.hi);
+  s.lo = vadd(s.lo, vadd(a.lo, b.lo));
+  return s;
+}
+template <typename V>
+DF_HD dfv<V> sub_v(dfv<V> a, dfv<V> b) {
+  dfv<V> s = two_diff_v(a.hi, b.hi);
+  s.lo = vadd(s.lo, vsub(a.lo, b.lo));
+  return s;
+}
+template <typename V>
+DF_HD dfv<V> add_one_v(dfv<V> a, V b) {
+  dfv<V> s = two_sum_v(a.hi, b);
+  s.lo = vadd(s.lo, a.lo);
+  return s;
+}
+// w a for a constant w: hi holds the NEGATED leading product (what the caller
+// subtracts from), lo the rest.  The product is formed as w a + 0, which no
+// compiler may contract into the sum that follows.
+template <typename V>
+DF_HD dfv<V> neg_scaled_v(df64 w, dfv<V> a) {
+  const V n = vfma(vset<V>(-w.hi), a.hi, vset<V>(0.0f));
+  const V e = vfma(vset<V>(w.hi), a.hi, n);
+  return {n, vfma(vset<V>(w.lo), a.hi, vfma(vset<V>(w.hi), a.lo, e))};
+}
+template <typename V>
+DF_HD V relax_v(V h, V d, V om_hi, V om_lo) {
+  const V t = vfma(om_hi, d, h);
+  return vadd(t, vfma(om_lo, d, vfma(om_hi, d, vsub(h, t))));
+}
+
+// The update of a pair (q, qbar = -q): heq = a +- b with a = w (drho + nl_q)
+// (nl_q = 4.5 (c_q.j)(c_q.u) - 1.5 j.u) and b = 3 w c_q.j.  With the pair's exact
 // sum S = h_q + h_qbar and difference D = h_q - h_qbar (the error-free sums
 // the moments are built from),
 //   heq_q - h_q = (a - S/2) + (b - D/2),  heq_qbar - h_qbar = (a - S/2) - (b - D/2):
 // a - S/2 and b - D/2 are the symmetric and antisymmetric non-equilibrium
 // parts, small against a and b, so their high parts subtract exactly (the
-// operands are within a factor two; the FMA with -1/2 forms S/2 exactly) and
+// operands are within a factor two; the FMA with 1/2 forms S/2 exactly) and
 // their low parts add in binary32.  This replaces the double-float sums
 // a + b, a - b of the two equilibria and 12 binary32 operations per pair.
-DF_HD void bgk_dev_comp(float (&h)[9], const DevParams& p) {
+// Everything is written in separately rounded operations, so that one cell per
+// thread and two in packed registers give the same bits.
+template <typename V>
+DF_HD void bgk_dev_comp(V (&h)[9], const DevParams& p) {
   // exact pairwise sums and differences of the stored values
-  const df64 s13 = two_sum(h[1], h[3]), s24 = two_sum(h[2], h[4]);
-  const df64 s57 = two_sum(h[5], h[7]), s68 = two_sum(h[6], h[8]);
-  const df64 d13 = two_sum(h[1], -h[3]), d24 = two_sum(h[2], -h[4]);
-  const df64 d57 = two_sum(h[5], -h[7]), d86 = two_sum(h[8], -h[6]);
-  const df64 drho = add_lazy(add_lazy(add_lazy(s57, s68), add_lazy(s13, s24)), make(h[0], 0.0f));
-  const df64 jx = add_lazy(add_lazy(d57, d86), d13);
-  const df64 jy = add_lazy(add_lazy(d57, neg(d86)), d24);
-  // nonlinear part in binary32: u = j / (1 + drho)
-  const float dr = drho.hi + drho.lo;
-  const float inv = 1.0f / (1.0f + dr);
-  const float jxf = jx.hi + jx.lo, jyf = jy.hi + jy.lo;
-  const float ux = jxf * inv, uy = jyf * inv;
-  const float rho = 1.0f + dr;
-  const float u2 = 1.5f * (ux * ux + uy * uy);
-  // h' = h + omega (heq - h), heq = w (drho + rho (4.5 (c.u)^2 - 1.5 u^2)) + 3 w c.j.
-  // The equilibrium's O(h) part is formed in double-float, the nonlinear term
-  // (binary32) joining the exact drho before the product with w (binary32
-  // weights in that product biased the relaxation rate by ~1e-8); heq - h is a
-  // small difference of nearby values and takes binary32; relax() adds
-  // omega (heq - h) with one rounding, to the storage format.
+  const dfv<V> s13 = two_sum_v(h[1], h[3]), s24 = two_sum_v(h[2], h[4]);
+  const dfv<V> s57 = two_sum_v(h[5], h[7]), s68 = two_sum_v(h[6], h[8]);
+  const dfv<V> d13 = two_diff_v(h[1], h[3]), d24 = two_diff_v(h[2], h[4]);
+  const dfv<V> d57 = two_diff_v(h[5], h[7]), d86 = two_diff_v(h[8], h[6]);
+  const dfv<V> drho = add_one_v(add_v(add_v(s57, s68), add_v(s13, s24)), h[0]);
+  const dfv<V> jx = add_v(add_v(d57, d86), d13);
+  const dfv<V> jy = add_v(sub_v(d57, d86), d24);
+  // nonlinear part in binary32: u = j / (1 + drho), nl = 4.5 (c.j)(c.u) - 1.5 j.u
+  const V jxf = vadd(jx.hi, jx.lo), jyf = vadd(jy.hi, jy.lo);
+  const V inv = vrcp(vadd(vset<V>(1.0f), vadd(drho.hi, drho.lo)));
+  const V ux = vmul(jxf, inv), uy = vmul(jyf, inv);
+  const V m = vfma(vset<V>(-1.5f), vfma(jyf, uy, vmul(jxf, ux)), vset<V>(0.0f));  // -1.5 j.u
+  // h' = h + omega (heq - h).  The equilibrium's O(h) part is formed in
+  // double-float, the nonlinear term (binary32) joining the exact drho before the
+  // product with w (binary32 weights in that product biased the relaxation rate by
+  // ~1e-8); heq - h is a small difference of nearby values and takes binary32;
+  // relax_v() adds omega (heq - h) with one rounding, to the storage format.
+  const V om_hi = vset<V>(p.om_hi), om_lo = vset<V>(p.om_lo), half = vset<V>(0.5f), mhalf = vset<V>(-0.5f);
   {
-    const df64 e = mul_lazy(p.w[0], add_lazy(drho, make(rho * -u2, 0.0f)));
-    h[0] = relax(h[0], (e.hi - h[0]) + e.lo, p.om_hi, p.om_lo);
+    const dfv<V> e = neg_scaled_v(p.w[0], add_one_v(drho, m));
+    h[0] = relax_v(h[0], vsub(e.lo, vadd(e.hi, h[0])), om_hi, om_lo);
   }
-#define PLBM_COMP_PAIR(QP, QM, CUF, CJ, S, D, WI)                                                       \
+#define PLBM_COMP_PAIR(QP, QM, CU, CJF, CJ, S, D, WI)                                                   \
   {                                                                                                    \
-    const float cu = (CUF);                                                                            \
-    const df64 a = mul_lazy(p.w[WI], add_lazy(drho, make(rho * fmaf_(4.5f * cu, cu, -u2), 0.0f)));    \
-    const df64 b = mul_lazy(p.w3[WI], CJ);                                                             \
-    const float sym = fmaf_(-0.5f, S.hi, a.hi) + fmaf_(-0.5f, S.lo, a.lo);                             \
-    const float asym = fmaf_(-0.5f, D.hi, b.hi) + fmaf_(-0.5f, D.lo, b.lo);                            \
-    h[QP] = relax(h[QP], sym + asym, p.om_hi, p.om_lo);                                                \
-    h[QM] = relax(h[QM], sym - asym, p.om_hi, p.om_lo);                                                \
+    const dfv<V> a = neg_scaled_v(p.w[WI], add_one_v(drho, vfma(vmul(vset<V>(4.5f), CJF), CU, m)));    \
+    const dfv<V> b = neg_scaled_v(p.w3[WI], CJ);                                                       \
+    const V sym = vsub(vfma(mhalf, S.lo, a.lo), vfma(half, S.hi, a.hi));                               \
+    const V asym = vsub(vfma(mhalf, D.lo, b.lo), vfma(half, D.hi, b.hi));                              \
+    h[QP] = relax_v(h[QP], vadd(sym, asym), om_hi, om_lo);                                             \
+    h[QM] = relax_v(h[QM], vsub(sym, asym), om_hi, om_lo);                                             \
   }
-  PLBM_COMP_PAIR(1, 3, ux, jx, s13, d13, 1)
-  PLBM_COMP_PAIR(2, 4, uy, jy, s24, d24, 1)
-  PLBM_COMP_PAIR(5, 7, ux + uy, add_lazy(jx, jy), s57, d57, 2)
-  PLBM_COMP_PAIR(8, 6, ux - uy, add_lazy(jx, neg(jy)), s68, d86, 2)
+  PLBM_COMP_PAIR(1, 3, ux, jxf, jx, s13, d13, 1)
+  PLBM_COMP_PAIR(2, 4, uy, jyf, jy, s24, d24, 1)
+  PLBM_COMP_PAIR(5, 7, vadd(ux, uy), vadd(jxf, jyf), add_v(jx, jy), s57, d57, 2)
+  PLBM_COMP_PAIR(8, 6, vsub(ux, uy), vsub(jxf, jyf), sub_v(jx, jy), s68, d86, 2)
 #undef PLBM_COMP_PAIR
 }
 

@@ -31,6 +31,61 @@
 #endif
 
 namespace plbm {
+
+// Binary32 operations by name, each rounded on its own in every build.  f32x2.cuh
+// overloads them for a pair of values, so that one template serves one cell per
+// thread and two.
+DF_HD float vadd(float a, float b) {
+#ifdef __CUDA_ARCH__
+  return __fadd_rn(a, b);
+#else
+  return a + b;
+#endif
+}
+DF_HD float vsub(float a, float b) {
+#ifdef __CUDA_ARCH__
+  return __fsub_rn(a, b);
+#else
+  return a - b;
+#endif
+}
+DF_HD float vmul(float a, float b) {
+#ifdef __CUDA_ARCH__
+  return __fmul_rn(a, b);
+#else
+  return a * b;
+#endif
+}
+DF_HD float vfma(float a, float b, float c) {
+#ifdef __CUDA_ARCH__
+  return __fmaf_rn(a, b, c);
+#else
+  return fmaf(a, b, c);
+#endif
+}
+DF_HD float rcp_seed(float x) {
+#ifdef __CUDA_ARCH__
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+#else
+  return 1.0f / x;
+#endif
+}
+// The constant c in a value of type V.
+template <typename V>
+DF_HD V vset(float c);
+template <>
+DF_HD float vset<float>(float c) { return c; }
+
+// 1 / x within 1 ulp: the hardware seed and one Newton step.
+template <typename V>
+DF_HD V vrcp(V x) {
+  const V r = rcp_seed(x);
+  const V e = vfma(vsub(vset<V>(0.0f), x), r, vset<V>(1.0f));
+  return vfma(e, r, r);
+}
+
 namespace df {
 
 struct df64 {

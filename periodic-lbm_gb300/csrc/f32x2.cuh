@@ -1,0 +1,107 @@
+// f32x2.cuh -- a pair of binary32 values in one 64-bit register, with the packed
+// operations of sm_100 and later (one instruction for both, each value rounded
+// as by the scalar operation), and the same operations on a single float, so that
+// one template serves a kernel with one cell per thread and one with two and gives
+// the same bits in both.  GB300 retires the packed operations at half the issue
+// slots of the scalar ones and the same 128 values per clock and SM (measured).
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+#include "df64.cuh"
+
+namespace plbm {
+
+struct f32x2 {
+  unsigned long long v;
+};
+DF_HD f32x2 pack2(float lo, float hi) {
+  return {((unsigned long long)df::f2u(hi) << 32) | (unsigned long long)df::f2u(lo)};
+}
+__device__ __forceinline__ float lo2(f32x2 a) {
+  return __uint_as_float((unsigned)a.v);
+}
+__device__ __forceinline__ float hi2(f32x2 a) {
+  return __uint_as_float((unsigned)(a.v >> 32));
+}
+
+__device__ __forceinline__ f32x2 vadd(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ f32x2 vsub(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ f32x2 vmul(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ f32x2 vfma(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+template <>
+DF_HD f32x2 vset<f32x2>(float c) { return pack2(c, c); }
+__device__ __forceinline__ f32x2 rcp_seed(f32x2 x) { return pack2(rcp_seed(lo2(x)), rcp_seed(hi2(x))); }
+
+// a / x with r = vrcp(x): the product and its exact residual added back
+// (Markstein 1990), within half an ulp and a hair.
+template <typename V>
+__device__ __forceinline__ V vquot(V a, V x, V r) {
+  const V q = vmul(a, r);
+  const V e = vfma(vsub(vset<V>(0.0f), x), q, a);
+  return vfma(e, r, q);
+}
+
+// BGK of the shifted populations h = f - w in binary32 (sim/sim.F90:445-499
+// with collide_bgk's equilibrium), h' = h + omega (heq - h).  With j = rho u,
+//   heq_q = w_q (dr + 4.5 (c.j)(c.u) - 1.5 j.u + 3 c.j),  dr = sum h:
+// the even part of a pair (q, -q) once, the odd part added and subtracted; 66
+// operations.  The O(h) terms come from dr and j themselves, not from rho - 1 and
+// rho u, which lose dr's low bits to the rounding of rho = 1 + dr.
+// SC: populations held scaled by S = 2^15 (binary16 storage): dr, j and heq scale
+// with them, rho = 1 + dr / S and u = (j / S) / rho.
+template <typename V, bool SC>
+__device__ __forceinline__ void bgk_dev(V (&h)[9], float omega) {
+  // the three binary32 weights share one relative error, 7e-9, with which mass and
+  // momentum drift; 3 w c.j with a rounded 3 w would drift four times as fast
+  const float w0 = 4.0f / 9.0f, ws = 1.0f / 9.0f, wd = 1.0f / 36.0f;
+  const V s13 = vadd(h[1], h[3]), s24 = vadd(h[2], h[4]), s57 = vadd(h[5], h[7]), s68 = vadd(h[6], h[8]);
+  const V d13 = vsub(h[1], h[3]), d24 = vsub(h[2], h[4]), d57 = vsub(h[5], h[7]), d86 = vsub(h[8], h[6]);
+  const V dr = vadd(vadd(vadd(s57, s68), vadd(s13, s24)), h[0]);
+  const V jx = vadd(vadd(d57, d86), d13), jy = vadd(vsub(d57, d86), d24);
+  V rho, ux, uy;
+  if constexpr (SC) {
+    const V is = vset<V>(1.0f / 32768.0f);
+    rho = vfma(dr, is, vset<V>(1.0f));
+    const V r = vrcp(rho);
+    ux = vquot(vmul(jx, is), rho, r);
+    uy = vquot(vmul(jy, is), rho, r);
+  } else {
+    rho = vadd(dr, vset<V>(1.0f));
+    const V r = vrcp(rho);
+    ux = vquot(jx, rho, r);
+    uy = vquot(jy, rho, r);
+  }
+  const V base = vfma(vset<V>(-1.5f), vfma(jy, uy, vmul(jx, ux)), dr);
+  // h' = h - omega (h - w heq'), all fused: no plain product feeds a sum or a
+  // difference (ptxas contracts a packed product and difference, .rn or not).
+  const V mom = vset<V>(-omega);
+  h[0] = vfma(mom, vfma(vset<V>(-w0), base, h[0]), h[0]);
+  auto pair = [&](int a, int b, V u, V j, float w) {
+    const V even = vfma(vmul(vset<V>(4.5f), j), u, base);
+    const V ha = vfma(vset<V>(3.0f), j, even), hb = vfma(vset<V>(-3.0f), j, even);
+    h[a] = vfma(mom, vfma(vset<V>(-w), ha, h[a]), h[a]);
+    h[b] = vfma(mom, vfma(vset<V>(-w), hb, h[b]), h[b]);
+  };
+  pair(1, 3, ux, jx, ws);
+  pair(2, 4, uy, jy, ws);
+  pair(5, 7, vadd(ux, uy), vadd(jx, jy), wd);
+  pair(8, 6, vsub(ux, uy), vsub(jx, jy), wd);
+}
+
+}  // namespace plbm

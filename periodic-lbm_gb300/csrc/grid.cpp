@@ -616,12 +616,24 @@ extern "C" int plbm_perform_lbm_step(plbm_grid_t* g, int nsteps) {
       return cuda_fail(e, "stream-collide graph");
     }
   }
-  for (int i = 0; i < nsteps; i++) {
-    cudaError_t e = fused_step(g, lattice(g, g->iold), lattice(g, g->inew), p);
+  // Large deviation-storage grids take several steps per pass over memory; the
+  // last step is always a single one, so that inew holds the state before it.
+  const bool comp = g->math == PLBM_MATH_HYBRID;
+  const bool march = g->streaming == PLBM_STREAM_LBM && g->storage != PLBM_F64 && (g->math == PLBM_MATH_FMA || comp) &&
+                     march_applies(g->storage, comp, g->kind, g->nx, g->ny);
+  MarchPlan plan = march ? march_plan(comp, nsteps) : MarchPlan{0, 0};
+  while (nsteps > 0) {
+    const int now = plan.threes-- > 0 ? 3 : (plan.twos-- > 0 ? 2 : 1);
+    cudaError_t e;
+    if (now > 1)
+      e = march_dev(g->storage, comp, now, Sweep{g->nx, g->ny, g->ld, lattice(g, g->iold), lattice(g, g->inew), g->stream}, p.omega);
+    else
+      e = fused_step(g, lattice(g, g->iold), lattice(g, g->inew), p);
     if (e != cudaSuccess) return cuda_fail(e, "stream-collide kernel");
     const int t = g->iold;  // src/periodic_lbm.f90:22-27
     g->iold = g->inew;
     g->inew = t;
+    nsteps -= now;
   }
   return ok();
 }

@@ -122,6 +122,16 @@ inline cudaError_t step_pull_f64(int kind, const Sweep& s, const CollParams& p) 
 
 // Deviation storage (storage = 1 float, 2 half), binary32 arithmetic.
 cudaError_t step_pull_dev(int storage, int kind, const Sweep& s, const CollParams& p);
+// Two or three steps of collide_bgk in one pass over memory (step_march.cu), bit for
+// bit those of step_pull_dev or (comp, binary32) of step_pull_dev_hi in compensated
+// arithmetic.  march_applies says for which grids, march_plan how many passes of
+// three and of two steps to take of nsteps; the rest are single steps, at least one.
+bool march_applies(int storage, bool comp, int kind, int nx, int ny);
+struct MarchPlan {
+  int threes, twos;
+};
+MarchPlan march_plan(bool comp, int nsteps);
+cudaError_t march_dev(int storage, bool comp, int steps, const Sweep& s, double omega);
 cudaError_t stream_dev(int storage, const Sweep& s);
 cudaError_t collide_dev(int storage, int kind, const Sweep& s, const CollParams& p);
 cudaError_t step_push_dev(int storage, int kind, const Sweep& s, const CollParams& p);
