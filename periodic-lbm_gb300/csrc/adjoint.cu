@@ -122,9 +122,9 @@ __device__ __noinline__ double forward_state_ref(const double* gp, const double*
 // pipe is left with the sums over lambda.
 __device__ __forceinline__ double forward_state(const double (&g)[9], const double (&l)[9], double& ux, double& uy) {
   int64_t F[9], Y[9], U, V;
-  bool bad = false;
-  const hy::BgkParams none = {0.0, 0.0, 0, 0};
-  hy::load_fixed<false>(g, F, bad);
+  bool bad = false, small;
+  const hy::BgkParams none = {0.0, 0.0, 0, 0, 0};
+  hy::load_fixed<false>(g, F, bad, small);
   if (!bad) hy::bgk_brackets<false>(F, none, Y, U, V, bad);
   if (bad) {
     double gc[9], lc[9], u[2];

@@ -23,8 +23,8 @@
 //     src/fvm_bardow.F90:99-126): the nonlinear terms of all nine populations
 //     are integer combinations of three products j_a u_b.
 //   TRT (trt_fma, incompressible, src/collision_trt.F90:98-152): symmetric
-//     and antisymmetric brackets of each pair, joined by one exact 128-bit
-//     product r D (r = lambda_d / lambda_e scaled).
+//     and antisymmetric brackets of each pair, joined by one product r D
+//     (r = lambda_d / lambda_e scaled) rounded to nearest.
 //   RR (rr_fma, src/collision_regularized.F90:72-194): the six merged Hermite
 //     coefficients of the equilibrium and the regularized part.
 // The products are fixed-point (mulh64, recip_fixed of fixed.cuh), each within
@@ -33,10 +33,12 @@
 // arithmetic, norm-wise: BGK 1.3e-16 against 1.4e-16, TRT 1.3e-16 / 1.4e-16, RR
 // 1.2e-16 / 1.2e-16; largest error of a population over its weight 3e-16 against
 // 1e-15).  Products in double-float, with conversions to and from the fixed
-// point, erred by 1e-15 of the weight at |u| = 0.05 and took 720 (BGK) and 1173
-// (RR) instructions per cell instead of 644 and 894; at 8192^2 a BGK step took
-// 1.762 ms instead of 1.700, RR 2.60 instead of 2.34, the plugin's BGK step 2.08
-// instead of 1.85.
+// point, erred by 1e-15 of the weight at |u| = 0.05 and took more instructions;
+// 8192^2, ms per step, with them / as fixed-point products / with every product
+// written as 32 x 32 -> 64 multiply-adds (mulh64 17 instructions, then 9; trt_rate
+// in place of an exact 128-bit product): BGK 1.76 / 1.70 / 1.58 (1.43 with the
+// columns copied ahead), TRT - / 1.89 / 1.79 (1.67), RR 2.60 / 2.24 / 2.05.  Bound by
+// the integer pipes; BGK at 97 % of the copy bandwidth.
 // Each states its range; a cell outside it reports `bad`, and the kernels then
 // evaluate that cell with the binary64 operator of the reference instead.
 // Populations stored shifted (h = f - w, the plugin's storage) take the same
@@ -95,27 +97,6 @@ DF_HD int64_t to_fixed_lim(double d, int emax, bool& bad) {
   return (u >> 63) ? -F : F;
 }
 
-
-// int64 fixed point -> double-float (leading 48 bits: hi truncated, lo exact).
-DF_HD df64 fixed_to_df(int64_t T) {
-  if (T == 0) return df::make(0.0f, 0.0f);
-  const uint32_t s = T < 0 ? 0x80000000u : 0u;
-  const uint64_t a = s ? (uint64_t)(-T) : (uint64_t)T;
-  const int lz = clz64(a);
-  const uint64_t n = a << lz;
-  const uint32_t mh = (uint32_t)(n >> 40);             // 24 bits, top bit set
-  const uint32_t ml = (uint32_t)(n >> 16) & 0xFFFFFFu;  // next 24 bits
-  // value = n * 2^(-lz - kScale); hi = mh * 2^(40 - lz - kScale)
-  const int eh = 40 - lz - kScale + 23;  // exponent of hi's leading bit
-  const float hi = df::u2f_bits(s | ((uint32_t)(eh + 127) << 23) | (mh & 0x7FFFFFu));
-  float lo = 0.0f;
-  if (ml) {
-    const float l = df::uint_to_float_rn(ml);  // exact, < 2^24
-    const float sc = df::u2f_bits((uint32_t)(16 - lz - kScale + 127) << 23);
-    lo = df::u2f_bits(df::f2u(l * sc) | s);
-  }
-  return df::make(hi, lo);
-}
 
 // ---- fast paths for the ranges lattice states live in --------------------
 // The general conversions are called out of line from the fast paths, so that
@@ -197,7 +178,7 @@ DF_HD uint32_t uabs_hi(int64_t a) {
 // a k / 2^64 rounded to nearest, for the constant corrections below
 // (|a| < 2^63, |k| < 2^31; a's low 32 bits do not take part).
 DF_HD int64_t scale_2m64(int64_t a, int32_t k) {
-  return ((int64_t)(int32_t)(a >> 32) * (int64_t)k + (int64_t(1) << 31)) >> 32;
+  return mad_wide((int32_t)(a >> 32), k, (int64_t)1 << 31) >> 32;
 }
 
 
@@ -240,6 +221,7 @@ DF_HD float i2f(int32_t v) {
 #endif
 }
 
+
 DF_HD constexpr double pow2_const(int e) { return e == 0 ? 1.0 : (e > 0 ? 2.0 * pow2_const(e - 1) : 0.5 * pow2_const(e + 1)); }
 PLBM_NOINLINE double fixed_to_double_any_slow(int64_t T) { return fixed_to_double_any(T); }
 
@@ -257,7 +239,9 @@ DF_HD double pos_fixed_to_double(int64_t v) {
 // line, exactly): the magnitude taken in one's complement (a negative T comes
 // out 2^-59 smaller in magnitude) and truncated to 53 bits.  The error is below
 // 2^-52 relative plus 2^-59 absolute -- for the non-equilibrium brackets it
-// converts, negligible against the binary64 rounding of the populations.
+// converts, negligible against the binary64 rounding of the populations.  (Selecting the
+// words without a branch put more on the ALU pipe, which binds: 8192^2 TRT 33.3
+// GLUPS against 36.)
 template <int SCALE = kScale>
 DF_HD double fixed_to_double_tr(int64_t T) {
   const uint32_t hi = (uint32_t)((uint64_t)T >> 32), lo = (uint32_t)(uint64_t)T;
@@ -273,40 +257,62 @@ DF_HD double fixed_to_double_tr(int64_t T) {
   return df::u2d(((uint64_t)(eh | (s & 0x80000000u)) << 32) | (uint64_t)ml);
 }
 
-// binary32 v, |v| < 16 -> int64 fixed point (scale 2^59), truncated toward
-// zero below 2^-58: the integer part of v 2^27 (F2I) is the high word and its
-// fraction 2^31 (F2I, signed) the low word shifted by one.  The fraction
-// t - trunc(t) is exact for either sign.  Exact for |v| >= 2^-35.
-DF_HD int64_t float_to_fixed_xu(float v) {
-  const float t = v * 0x1p27f;  // exact
-  const int32_t h = f2i_trunc(t);
-  const int32_t l = f2i_trunc((t - i2f(h)) * 0x1p31f);  // |l| < 2^31
-  return (int64_t)((uint64_t)(uint32_t)h << 32) + 2 * (int64_t)l;
+// ---- the new populations -------------------------------------------------------
+// f'_q = f_q + k_q c Y_q 2^-59 rounded to nearest, in the last places of f_q: with
+// the biased exponent E of f_q one place is 2^(E - 1075), so the change is
+// k_q c Y_q 2^(1016 - E) places, one fixed-point product (c at 2^66) and a right
+// shift, added to f_q's bits.  That is f'_q while its exponent is E; a cell with a
+// population that changes binade converts them all from 2^-61 (about one cell in
+// twenty of a flow of |u| = 0.05), one with a population below 2^-7 or a sign change
+// takes the binary64 FMAs out of line.  Against an integer-to-binary64 conversion
+// (sign, leading zeros, two shifts, a branch for small Y) and an FMA: no binary64
+// instruction, no branch per population.  The product is within 2 units of 2^-61
+// (diagonal) or 2^-59 (axis, rest; places of 2^-56 and 2^-54).  Norm-wise error
+// against 113-bit arithmetic as with the FMAs: BGK 1.31e-16 / 1.33e-16, TRT
+// 1.31e-16 / 1.32e-16, RR 1.16e-16 / 1.17e-16.
+PLBM_NOINLINE void finish_slow(double* f, const int64_t* Y, double c0, double cs, double cd) {
+  for (int q = 0; q < 9; q++) f[q] = fma_d(q == 0 ? c0 : (q < 5 ? cs : cd), fixed_to_double_tr(Y[q]), f[q]);
 }
-// A double-float (|value| < 16) in the fixed point: the sum of its halves' images.
-DF_HD int64_t df_to_fixed_xu(df64 c) { return float_to_fixed_xu(c.hi) + float_to_fixed_xu(c.lo); }
-
-PLBM_NOINLINE df64 fixed_to_df_slow(int64_t T) { return fixed_to_df(T); }
-
-// int64 fixed point -> double-float (leading 48 bits: hi and lo truncated)
-// for |T| >= 2^32 (others out of line).
-DF_HD df64 fixed_to_df_x(int64_t T) {
-  const uint32_t hi = (uint32_t)((uint64_t)T >> 32), lo = (uint32_t)(uint64_t)T;
-  const uint32_t s = (uint32_t)((int32_t)hi >> 31);
-  const uint64_t a = ((((uint64_t)hi << 32) | lo) ^ (((uint64_t)s << 32) | s)) + (uint64_t)(s & 1u);
-  const uint32_t ah = (uint32_t)(a >> 32), al = (uint32_t)a;
-  if (ah == 0u) return fixed_to_df_slow(T);
-  const uint32_t lz = clz32(ah);
-  const uint32_t nh = funnel_l(al, ah, lz), nl = al << lz;  // bit 31 of nh set
-  // value = (nh:nl) 2^(-lz - 59) = nh 2^(-lz - 27) + ...: hi = top 24 bits of
-  // nh, leading one at bit 23 (it adds the final 1 to the exponent field)
-  const uint32_t sgn = s & 0x80000000u;
-  const float fhi = df::u2f_bits(((130u - lz) * 0x800000u + (nh >> 8)) | sgn);
-  const uint32_t ml = funnel_r(nl, nh, 16) & 0xFFFFFFu;  // next 24 bits
-  // lo = ml 2^(16 - lz - 59): a signed scale (biased exponent 84 - lz) times
-  // the exact I2F of the 24-bit integer
-  const float sc = df::u2f_bits(((84u - lz) * 0x800000u) | sgn);
-  return df::make(fhi, i2f((int32_t)ml) * sc);
+// KS: log2 of k_q of the axis populations (2 BGK and RR, 1 TRT; k_0 = 4, k_diag =
+// 1).  c0, cs, cd: k_q c; small: a population below 2^-7 (load_fixed).
+template <int KS>
+DF_HD void finish(double (&f)[9], const int64_t (&Y)[9], int64_t c, double c0, double cs, double cd, bool small) {
+  uint64_t b[9];
+  int64_t m[9];
+  uint32_t moved = small ? 0x100000u : 0u;
+#pragma unroll
+  for (int q = 0; q < 9; q++) {
+    const uint64_t u = df::d2u(f[q]);
+    const uint32_t sh = ((uint32_t)(u >> 52) - 1014u - (q == 0 ? 2u : (q < 5 ? (uint32_t)KS : 0u))) & 31u;
+    m[q] = mulh64(Y[q], c);  // 4 c Y
+    b[q] = u + (uint64_t)((m[q] + (int64_t)((1u << sh) >> 1)) >> sh);
+    moved |= (uint32_t)((b[q] ^ u) >> 32);
+  }
+  if (moved >> 20) {
+    int64_t low = small ? 0 : 1;
+#pragma unroll
+    for (int q = 0; q < 9; q++) {  // the populations at 2^-61
+      const uint64_t u = df::d2u(f[q]);
+      const int64_t F = shl((int64_t)((u & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull), (int)((u >> 52) - 1014u) & 31);
+      m[q] = F + shl(m[q], q == 0 ? 2 : (q < 5 ? KS : 0));
+      low = m[q] < low ? m[q] : low;
+    }
+    if (low <= 0) {
+      double g[9];
+      int64_t Z[9];
+#pragma unroll
+      for (int q = 0; q < 9; q++) g[q] = f[q], Z[q] = Y[q];
+      finish_slow(g, Z, c0, cs, cd);
+#pragma unroll
+      for (int q = 0; q < 9; q++) f[q] = g[q];
+    } else {
+#pragma unroll
+      for (int q = 0; q < 9; q++) f[q] = pos_fixed_to_double<61>(m[q]);
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < 9; q++) f[q] = df::u2d(b[q]);
+  }
 }
 
 // ---- BGK with one binary64 FMA per population --------------------------------
@@ -349,6 +355,7 @@ struct BgkParams {
   double c4;       // 4 RN(omega / 36), exact
   int32_t mass_k;  // omega eps_m / c4 2^64, rounded (bgk_fma_params)
   int32_t mom_k;   // omega eps_j / (2 c4) 2^64, rounded
+  int64_t c_fx;    // c1 2^66
 };
 
 // a + b = s + e exactly (Knuth's two-sum).
@@ -382,6 +389,7 @@ inline BgkParams bgk_fma_params(double omega, const double (&w)[3]) {
   const double km = ldexp(omega * eps_m / p.c4, 64), kj = ldexp(0.5 * omega * eps_j / p.c4, 64);
   p.mass_k = fabs(km) < 0x1p30 ? (int32_t)llrint(km) : 0;
   p.mom_k = fabs(kj) < 0x1p30 ? (int32_t)llrint(kj) : 0;
+  p.c_fx = llrint(ldexp(p.c1, 66));
   return p;
 }
 
@@ -426,7 +434,7 @@ PLBM_NOINLINE void load_fixed_slow(const double* f, int64_t* F) {
   for (int q = 5; q < 9; q++) F[q] = to_fixed_nonneg<1019>(f[q], b);
 }
 template <bool SHIFTED>
-DF_HD void load_fixed(const double (&f)[9], int64_t (&F)[9], bool& bad) {
+DF_HD void load_fixed(const double (&f)[9], int64_t (&F)[9], bool& bad, bool& small) {
   bool odd = false;
 #pragma unroll
   for (int q = 0; q < 9; q++) {
@@ -443,9 +451,10 @@ DF_HD void load_fixed(const double (&f)[9], int64_t (&F)[9], bool& bad) {
     } else {
       const uint32_t sh = (H >> 20) - 1016u;  // a set sign bit makes this large
       odd |= sh > (q == 0 ? 6u : (q < 5 ? 4u : 3u));
-      F[q] = (int64_t)(((uint64_t)funnel_l(L, mh, sh & 31u) << 32) | (uint64_t)(L << (sh & 31u)));
+      F[q] = (int64_t)(((uint64_t)funnel_l(L, mh, sh & 31u) << 32) | (uint64_t)funnel_l(0u, L, sh & 31u));
     }
   }
+  small = odd;
   if constexpr (SHIFTED) {
     bad |= odd;
   } else if (odd) {
@@ -516,14 +525,19 @@ DF_HD void bgk_brackets(const int64_t (&F)[9], const BgkParams& p, int64_t (&Y)[
   bgk_brackets<SHIFTED>(F, p, Y, U, V, bad);
 }
 
-template <bool SHIFTED = false>
+template <bool SHIFTED = false, bool QUICK = false>
 DF_HD void bgk_fma(double (&f)[9], const BgkParams& p, bool& bad) {
   int64_t F[9], Y[9];
-  load_fixed<SHIFTED>(f, F, bad);
+  bool small;
+  load_fixed<SHIFTED>(f, F, bad, small);
   if (bad) return;
   bgk_brackets<SHIFTED>(F, p, Y, bad);
+  if constexpr (SHIFTED || !QUICK) {
 #pragma unroll
-  for (int q = 0; q < 9; q++) f[q] = fma_d(q < 5 ? p.c4 : p.c1, fixed_to_double_tr(Y[q]), f[q]);
+    for (int q = 0; q < 9; q++) f[q] = fma_d(q < 5 ? p.c4 : p.c1, fixed_to_double_tr(Y[q]), f[q]);
+  } else {
+    finish<2>(f, Y, p.c_fx, p.c4, p.c4, p.c1, small);
+  }
 }
 
 // Recursive-regularized constant (rr_fma): 1 - omega at scale 2^63.
@@ -613,14 +627,19 @@ DF_HD void rr_brackets(const int64_t (&F)[9], const RrParams& r, const BgkParams
   Y[8] = dm - sm - 36 * F[8];
 }
 
-template <bool SHIFTED = false>
+template <bool SHIFTED = false, bool QUICK = false>
 DF_HD void rr_fma(double (&f)[9], const RrParams& r, const BgkParams& p, bool& bad) {
   int64_t F[9], Y[9];
-  load_fixed<SHIFTED>(f, F, bad);
+  bool small;
+  load_fixed<SHIFTED>(f, F, bad, small);
   if (bad) return;
   rr_brackets<SHIFTED>(F, r, p, Y, bad);
+  if constexpr (SHIFTED || !QUICK) {
 #pragma unroll
-  for (int q = 0; q < 9; q++) f[q] = fma_d(q < 5 ? p.c4 : p.c1, fixed_to_double_tr(Y[q]), f[q]);
+    for (int q = 0; q < 9; q++) f[q] = fma_d(q < 5 ? p.c4 : p.c1, fixed_to_double_tr(Y[q]), f[q]);
+  } else {
+    finish<2>(f, Y, p.c_fx, p.c4, p.c4, p.c1, small);
+  }
 }
 
 // (a b) / 2^sh, 0 < sh < 64, of the exact 128-bit product, rounded to nearest
@@ -644,12 +663,12 @@ DF_HD int64_t mul_shr(int64_t a, int64_t b, int sh) {
 // Incompressible TRT with one binary64 FMA per population
 // (src/collision_trt.F90:98-152).  With c = RN(lambda_e / 18) and the exact
 // integer brackets of the pairs (axis: weights 1/9, diagonal: 1/36; J2 = |J|^2,
-// XY = JX JY as exact 128-bit products taken to the fixed point)
+// XY = JX JY as products taken to the fixed point)
 //   axis x    Sb = 9 (F_1 + F_3) - 2 R - 6 JX^2 + 3 JY^2,   D = 3 (F_1 - F_3) - 2 JX
 //   diagonal  Sb = 18 (F_5 + F_7) - R - 3 J2 -+ 9 XY,       D = 6 (F_5 - F_7) - (JX +- JY)
 // the reference's sym = les (...) is c Sb (axis) and c/2 Sb (diagonal), its
-// asym the same constants times r D with r = lambda_d / (6 c) (one exact
-// 64 x 64-bit product per pair), so
+// asym the same constants times r D with r = lambda_d / (6 c) (trt_rate, one
+// product per pair), so
 //   f'_p = fma(c_k, -(Sb + r D), f_p),  f'_m = fma(c_k, -(Sb - r D), f_m),
 //   f'_0 = fma(2c, 4 R - 6 J2 - 9 F_0, f_0)
 // (c_k = c on the axis pairs, c/2 on the diagonal ones).  The integer brackets
@@ -658,12 +677,14 @@ DF_HD int64_t mul_shr(int64_t a, int64_t b, int sh) {
 // the rest bracket (mass_k).  Range: the loads of bgk_fma, and |Sb| < 2^61,
 // |D| < dmax = 2^61 / r (checked), so every bracket stays below 2^62.
 struct TrtFmaParams {
-  double c, c2, ch;  // RN(lambda_e / 18), 2c, c/2
-  int64_t r_fx;      // r = lambda_d / (6c) = r_fx 2^-r_sh
-  int64_t dmax;      // largest |D| with |r D| < 2^61 (0: every cell falls back)
-  int32_t r_sh;
-  int32_t mass_k;    // lambda_e eps_m / (2c) 2^64
-  int32_t mom_k;     // lambda_d eps_j / (2c) 2^64
+  double c, c2, ch;    // RN(lambda_e / 18), 2c, c/2
+  int64_t dmax;        // smallest |D| out of range: |r D| < 2^61, |D| < 2^60 (0: every cell falls back)
+  int64_t r_round;     // half a unit of the product's discarded bits
+  int32_t r_hi, r_lo;  // r = lambda_d / (6c) = (r_hi 2^31 + r_lo) 2^-(r_s + 31)
+  int32_t r_s;
+  int32_t mass_k;      // lambda_e eps_m / (2c) 2^64
+  int32_t mom_k;       // lambda_d eps_j / (2c) 2^64
+  int64_t c_fx;        // (c / 2) 2^66
 };
 
 inline TrtFmaParams trt_fma_params(double lambda_e, double lambda_d, const double (&w)[3]) {
@@ -674,22 +695,36 @@ inline TrtFmaParams trt_fma_params(double lambda_e, double lambda_d, const doubl
   const double r = lambda_d / (6.0 * p.c);
   int e = 0;
   frexp(r, &e);  // r in [2^(e-1), 2^e)
-  int sh = 61 - e;
+  int sh = 61 - e;  // r 2^sh in [2^60, 2^61)
   if (sh > 63) sh = 63;
-  if (sh < 1) sh = 1;
-  const double rf = ldexp(r, sh);
-  p.r_sh = sh;
-  p.r_fx = rf < 0x1p62 ? (int64_t)llrint(rf) : 0;
-  p.dmax = r > 0 ? (int64_t)fmin(0x1p61 / r, 0x1p62) : ((int64_t)1 << 62);
-  if (!(rf < 0x1p62) || !(r >= 0)) p.dmax = 0;
+  const bool fits = r >= 0 && sh >= 33;
+  const int64_t rf = fits ? (int64_t)llrint(ldexp(r, sh)) : 0;
+  p.r_hi = (int32_t)(rf >> 31);
+  p.r_lo = (int32_t)(rf & 0x7fffffff);
+  p.r_s = fits ? sh - 31 : 2;
+  p.r_round = (int64_t)1 << (p.r_s - 2);
+  p.dmax = !fits ? 0 : (r > 0 ? (int64_t)fmin(0x1p61 / r, 0x1p60) : (int64_t)1 << 60);
   const double km = ldexp(lambda_e * weight_sum_error(w) / p.c2, 64);
   const double kj = ldexp(lambda_d * first_moment_error(w) / p.c2, 64);
   p.mass_k = fabs(km) < 0x1p30 ? (int32_t)llrint(km) : 0;
   p.mom_k = fabs(kj) < 0x1p30 ? (int32_t)llrint(kj) : 0;
+  p.c_fx = llrint(ldexp(p.ch, 66));
   return p;
 }
 
 DF_HD int64_t abs64(int64_t v) { return v < 0 ? -v : v; }
+
+// r D rounded to nearest (the error's mean is below 2^-25 unit: a bias in the
+// antisymmetric brackets is a uniform force, see mul_shr), |D| < 2^60: four 32 x 32
+// products.
+DF_HD int64_t trt_rate(int64_t D, const TrtFmaParams& p) {
+  const int32_t dh = (int32_t)(D >> 32);
+  const uint32_t dl = (uint32_t)D;
+  const uint64_t low = mad_wide_u(dl, (uint32_t)p.r_hi, mad_wide_u(dl, (uint32_t)p.r_lo, 0) >> 31);
+  const int64_t mid = mad_wide(dh, p.r_lo, p.r_round);  // + half a unit / 2
+  const int64_t a = (int64_t)(low + ((uint64_t)mid << 1));
+  return (a >> p.r_s) + (int64_t)((uint64_t)mad_wide(dh, p.r_hi, 0) << (32 - p.r_s));
+}
 
 DF_HD void trt_brackets(const int64_t (&F)[9], const TrtFmaParams& p, int64_t (&Y)[9], bool& bad) {
   const int64_t R = (((F[5] + F[7]) + (F[6] + F[8])) + ((F[1] + F[3]) + (F[2] + F[4]))) + F[0];
@@ -707,9 +742,9 @@ DF_HD void trt_brackets(const int64_t (&F)[9], const TrtFmaParams& p, int64_t (&
   bad |= (abs64(sx) | abs64(sy) | abs64(sp) | abs64(sm)) >= lim;
   bad |= (abs64(dx) | abs64(dy) | abs64(dp) | abs64(dm)) >= p.dmax;
   Y[0] = 4 * R - 6 * J2 - 9 * F[0] + scale_2m64(R, p.mass_k);
-  const int64_t rx = mul_shr(dx, p.r_fx, p.r_sh) - scale_2m64(JX, p.mom_k);
-  const int64_t ry = mul_shr(dy, p.r_fx, p.r_sh) - scale_2m64(JY, p.mom_k);
-  const int64_t rp = mul_shr(dp, p.r_fx, p.r_sh), rm = mul_shr(dm, p.r_fx, p.r_sh);
+  const int64_t rx = trt_rate(dx, p) - scale_2m64(JX, p.mom_k);
+  const int64_t ry = trt_rate(dy, p) - scale_2m64(JY, p.mom_k);
+  const int64_t rp = trt_rate(dp, p), rm = trt_rate(dm, p);
   Y[1] = -(sx + rx);
   Y[3] = rx - sx;
   Y[2] = -(sy + ry);
@@ -720,14 +755,19 @@ DF_HD void trt_brackets(const int64_t (&F)[9], const TrtFmaParams& p, int64_t (&
   Y[6] = rm - sm;
 }
 
-template <bool SHIFTED = false>
+template <bool SHIFTED = false, bool QUICK = false>
 DF_HD void trt_fma(double (&f)[9], const TrtFmaParams& p, bool& bad) {
   int64_t F[9], Y[9];
-  load_fixed<SHIFTED>(f, F, bad);
+  bool small;
+  load_fixed<SHIFTED>(f, F, bad, small);
   if (bad) return;
   trt_brackets(F, p, Y, bad);
+  if constexpr (SHIFTED || !QUICK) {
 #pragma unroll
-  for (int q = 0; q < 9; q++) f[q] = fma_d(q == 0 ? p.c2 : (q < 5 ? p.c : p.ch), fixed_to_double_tr(Y[q]), f[q]);
+    for (int q = 0; q < 9; q++) f[q] = fma_d(q == 0 ? p.c2 : (q < 5 ? p.c : p.ch), fixed_to_double_tr(Y[q]), f[q]);
+  } else {
+    finish<1>(f, Y, p.c_fx, p.c2, p.c, p.ch, small);
+  }
 }
 
 }  // namespace hy

@@ -47,17 +47,19 @@ __device__ __noinline__ void hybrid_fallback_cell(const double* __restrict__ src
   if (report) g_hybrid_range_flag = 1;
 }
 
-// Resident CTAs per SM the hybrid kernels are compiled for: BGK (bgk_fma) and
+// Resident CTAs per SM the one-cell kernels are compiled for: BGK (bgk_fma) and
 // TRT (trt_fma) at 4, RR (rr_fma) at 3 (register caps 64 and 80).  Capped at
 // 48 registers for 5 CTAs the BGK kernel spills and runs 2 % slower at 8192^2.
 constexpr int hybrid_min_blocks(int kind) { return kind == K_RR ? 3 : 4; }
 
 // I: index type of the lattice offsets; 32-bit when the whole lattice has
 // fewer than 2^32 elements (one multiply-add per address instead of 64-bit
-// arithmetic).
-template <typename I, int KIND>
-__global__ void __launch_bounds__(kBlock, hybrid_min_blocks(KIND)) k_step_hybrid(const double* __restrict__ src, double* __restrict__ dst,
-                                                       int nx, int ny, int ld, int ftiles, HybridArgs a) {
+// arithmetic).  QUICK: see kQuickCells.
+template <typename I, int KIND, bool QUICK>
+__global__ void __launch_bounds__(kBlock, hybrid_min_blocks(KIND)) k_step_hybrid(const double* __restrict__ src,
+                                                                                double* __restrict__ dst, int nx,
+                                                                                int ny, int ld, int ftiles,
+                                                                                HybridArgs a) {
   chain_begin();
   const int x = blockIdx.x / ftiles;
   const int y = (blockIdx.x - x * ftiles) * blockDim.x + threadIdx.x;
@@ -77,9 +79,9 @@ __global__ void __launch_bounds__(kBlock, hybrid_min_blocks(KIND)) k_step_hybrid
   f[7] = ld_chain(src + (7 * P + cp + yp));
   f[8] = ld_chain(src + (8 * P + cm + yp));
   bool bad = false;
-  if (KIND == K_TRT) hy::trt_fma(f, a.trt, bad);
-  else if (KIND == K_RR) hy::rr_fma(f, a.rr, a.rr1, bad);
-  else hy::bgk_fma(f, a.bgk1, bad);
+  if (KIND == K_TRT) hy::trt_fma<false, QUICK>(f, a.trt, bad);
+  else if (KIND == K_RR) hy::rr_fma<false, QUICK>(f, a.rr, a.rr1, bad);
+  else hy::bgk_fma<false, QUICK>(f, a.bgk1, bad);
   if (bad) {  // outside the hybrid range: the binary64 operator on the same inputs
     hybrid_fallback_cell<KIND>(src, dst, x, y, nx, ny, ld, a.ref, a.report);
     return;
@@ -87,6 +89,92 @@ __global__ void __launch_bounds__(kBlock, hybrid_min_blocks(KIND)) k_step_hybrid
   const I o = c0 + y0;
 #pragma unroll
   for (int q = 0; q < 9; q++) dst[(I)q * P + o] = f[q];
+}
+
+// The same step for large grids (BGK and TRT): a CTA keeps its 128 rows and walks
+// along x over seg columns, each thread copying its own nine populations of the
+// next column into shared memory (cp.async: no register held, no barrier, no
+// latency waited for) while it collides the present ones.  One cell per thread
+// leaves the loads' latency to the other CTAs of the SM, of which the registers
+// allow four; here the memory stays busy.  8192^2, GLUPS: BGK 42.4 one cell per
+// thread, 46.8 here (144 bytes per cell at the copy bandwidth: 48), TRT 37.5 and
+// 40.0; 2048^2 BGK 40.8 and 43.8, TRT 36.3 and 37.5.  RR (32.6 and 32.9, 31.8 and
+// 31.3) is bound by its instructions and keeps one cell per thread.  Three columns
+// in flight take shared memory from the L1 cache that the neighbours' rows live
+// in: slower.
+constexpr int kAheadThreads = 128;
+template <int KIND>
+__global__ void __launch_bounds__(kAheadThreads, 8)
+    k_step_ahead(const double* __restrict__ src, double* __restrict__ dst, int nx, int ny, int ld, int ytiles, int seg,
+                 HybridArgs a) {
+  __shared__ double sm[2][9][kAheadThreads];  // a thread reads what it copied itself
+  chain_begin();
+  const int bx = blockIdx.x / ytiles;
+  const int y = (blockIdx.x - bx * ytiles) * kAheadThreads + threadIdx.x;
+  if (y >= ny) return;
+  const unsigned ym = wrap_m(y, ny), yp = wrap_p(y, ny);
+  const size_t P = (size_t)ld * nx;
+  const int x0 = bx * seg, x1 = min(x0 + seg, nx);
+  auto copy_column = [&](int x, int stage) {
+    const double *c0 = src + (size_t)x * ld, *cm = src + (size_t)wrap_m(x, nx) * ld, *cp = src + (size_t)wrap_p(x, nx) * ld;
+    const unsigned s0 = (unsigned)__cvta_generic_to_shared(&sm[stage][0][threadIdx.x]);
+    auto copy = [&](int q, const double* p) {
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(s0 + q * (unsigned)(8 * kAheadThreads)), "l"(p)
+                   : "memory");
+    };
+    copy(0, c0 + y);
+    copy(1, cm + P + y);
+    copy(2, c0 + 2 * P + ym);
+    copy(3, cp + 3 * P + y);
+    copy(4, c0 + 4 * P + yp);
+    copy(5, cm + 5 * P + ym);
+    copy(6, cp + 6 * P + ym);
+    copy(7, cp + 7 * P + yp);
+    copy(8, cm + 8 * P + yp);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  copy_column(x0, 0);
+  int stage = 0;
+#pragma unroll 1
+  for (int x = x0; x < x1; x++) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    double f[9];
+#pragma unroll
+    for (int q = 0; q < 9; q++) f[q] = sm[stage][q][threadIdx.x];
+    stage ^= 1;
+    if (x + 1 < x1) copy_column(x + 1, stage);
+    bool bad = false;
+    if (KIND == K_TRT) hy::trt_fma(f, a.trt, bad);
+    else hy::bgk_fma(f, a.bgk1, bad);
+    if (bad) {
+      hybrid_fallback_cell<KIND>(src, dst, x, y, nx, ny, ld, a.ref, a.report);
+      continue;
+    }
+    double* o = dst + (size_t)x * ld;
+#pragma unroll
+    for (int q = 0; q < 9; q++) (o + q * P)[(unsigned)y] = f[q];
+  }
+}
+
+// Whether a grid takes k_step_ahead: BGK from 2^20 cells (1024^2 37.3 GLUPS against
+// 36.2 one cell per thread; 512^2 slower), TRT from 2^22 (2048^2 37.5 and 36.3;
+// 1024^2 31.7 and 32.7), rows enough to fill half a CTA.
+bool takes_ahead(int kind, const Sweep& s) {
+  const long long cells = (long long)s.nx * s.ny;
+  return s.ny >= kAheadThreads / 2 && ((kind == K_BGK && cells >= 1 << 20) || (kind == K_TRT && cells >= 1 << 22));
+}
+
+template <int KIND>
+cudaError_t launch_ahead(const Sweep& s, const HybridArgs& a) {
+  const int yt = (s.ny + kAheadThreads - 1) / kAheadThreads;
+  // Columns per CTA: 4 keep the last wave short (2048^2 BGK 43.8 GLUPS against 43.2 with
+  // 8), 8 where there are tens of waves (8192^2 46.8 against 46.5).
+  const int seg = (long long)s.nx * s.ny >= 1 << 25 ? 8 : 4;
+  const long long blocks = (long long)yt * ((s.nx + seg - 1) / seg);
+  if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+  chained(k_step_ahead<KIND>, (unsigned)blocks, kAheadThreads, s.stream)(
+      static_cast<const double*>(s.src), static_cast<double*>(s.dst), s.nx, s.ny, s.ld, yt, seg, a);
+  return cudaGetLastError();
 }
 
 // A finite-volume / finite-difference streaming scheme in stencil form fused
@@ -331,14 +419,30 @@ __global__ void __launch_bounds__(kBlock, hybrid_min_blocks(KIND)) k_push_hybrid
   dst[8 * P + rm + xp] = f[8];
 }
 
+// Cells up to which the last operations take the branch-free form (hy::finish): a
+// grid of so few warps waits for one warp's chain of instructions, which that form
+// shortens; with more warps its 130 further instructions per cell, and the cells
+// that change binade, cost more.  us per step of a Taylor-Green flow, RR / BGK / TRT,
+// with and without: 64^2 2.23 / 1.97 / 2.09 and 2.58 / 2.33 / 2.45, 128^2 2.44 / 2.19 /
+// 2.31 and 2.71 / 2.45 / 2.58, 192^2 3.23 / 2.98 / 2.97 and 3.09 / 2.83 / 2.88.
+constexpr long long kQuickCells = 1 << 14;
+
 template <int KIND>
-cudaError_t launch_hybrid(const Sweep& s, unsigned blocks, int bs, int ft, const HybridArgs& a) {
+cudaError_t launch_hybrid(const Sweep& s, const HybridArgs& a) {
+  const long long cells = (long long)s.nx * s.ny;
+  const int bs = block_for(cells, true);
+  const int ft = (s.ny + bs - 1) / bs;
+  const long long blocks = (long long)ft * s.nx;
+  if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+  const unsigned nb = (unsigned)blocks;
   const double* src = static_cast<const double*>(s.src);
   double* dst = static_cast<double*>(s.dst);
-  if ((unsigned long long)s.ld * (unsigned long long)s.nx * 9ull < (1ull << 32))
-    chained(k_step_hybrid<uint32_t, KIND>, blocks, bs, s.stream)(src, dst, s.nx, s.ny, s.ld, ft, a);
+  if ((unsigned long long)s.ld * (unsigned long long)s.nx * 9ull >= (1ull << 32))
+    chained(k_step_hybrid<size_t, KIND, false>, nb, bs, s.stream)(src, dst, s.nx, s.ny, s.ld, ft, a);
+  else if (cells > kQuickCells)
+    chained(k_step_hybrid<uint32_t, KIND, false>, nb, bs, s.stream)(src, dst, s.nx, s.ny, s.ld, ft, a);
   else
-    chained(k_step_hybrid<size_t, KIND>, blocks, bs, s.stream)(src, dst, s.nx, s.ny, s.ld, ft, a);
+    chained(k_step_hybrid<uint32_t, KIND, true>, nb, bs, s.stream)(src, dst, s.nx, s.ny, s.ld, ft, a);
   return cudaGetLastError();
 }
 
@@ -371,14 +475,10 @@ HybridArgs hybrid_args(const CollParams& cp, bool report) {
 
 cudaError_t step_pull_fixed(int kind, const Sweep& s, const CollParams& cp, bool report) {
   if (kind != K_BGK && kind != K_TRT && kind != K_RR) return cudaErrorNotSupported;
-  const int bs = block_for((long long)s.nx * s.ny, true);
-  const int ft = (s.ny + bs - 1) / bs;
-  const long long blocks = (long long)ft * s.nx;
-  if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   const HybridArgs a = hybrid_args(cp, report);
-  if (kind == K_TRT) return launch_hybrid<K_TRT>(s, (unsigned)blocks, bs, ft, a);
-  if (kind == K_RR) return launch_hybrid<K_RR>(s, (unsigned)blocks, bs, ft, a);
-  return launch_hybrid<K_BGK>(s, (unsigned)blocks, bs, ft, a);
+  if (kind == K_RR) return launch_hybrid<K_RR>(s, a);
+  if (takes_ahead(kind, s)) return kind == K_TRT ? launch_ahead<K_TRT>(s, a) : launch_ahead<K_BGK>(s, a);
+  return kind == K_TRT ? launch_hybrid<K_TRT>(s, a) : launch_hybrid<K_BGK>(s, a);
 }
 
 cudaError_t step_push_fixed(int kind, const Sweep& s, const CollParams& cp, bool report) {

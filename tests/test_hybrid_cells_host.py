@@ -25,6 +25,7 @@ def lib(tmp_path_factory):
                     "-o", str(so)], check=True)
     h = ctypes.CDLL(str(so))
     h.hc_collide.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_double, ctypes.c_double]
+    h.hc_collide_quick.argtypes = [ctypes.c_int, ctypes.c_void_p, ctypes.c_double, ctypes.c_double]
     h.hc_mulh64.restype = h.hc_recip.restype = ctypes.c_int64
     h.hc_mulh64.argtypes = [ctypes.c_int64, ctypes.c_int64]
     h.hc_recip.argtypes = [ctypes.c_int64]
@@ -151,3 +152,29 @@ def test_product_and_reciprocal(lib):
     lo, hi = (0x2000001 << 32), 2 ** 61 - 1
     for R in [lo, hi, 2 ** 59, 2 ** 59 - 1, 2 ** 60 + 1] + [int(v) for v in rng.integers(lo, hi, 2000)]:
         assert abs(Fr(lib.hc_recip(R)) * R / 2 ** 120 - 1) < Fr(1, 2 ** 59)
+
+
+@pytest.mark.parametrize("kind", list(KINDS))
+@pytest.mark.parametrize("case", ["calm", "noisy", "binade", "small"])
+def test_finish_in_the_populations_last_places(lib, kind, case):
+    """The branch-free last operations: the bounds of
+    test_collision_within_the_derived_error and the product's two units of 2^-59.
+    binade: populations a few spacings from a power of two, which the collision
+    moves across it; small: one below 2^-7, and one zero."""
+    states = list(cells(60, 0.05, 23, 1e-4) if case == "calm" else cells(60, 0.14, 29, 0.03))
+    for i, (f, omega) in enumerate(states):
+        if case == "binade":
+            f = [float(w) for w in W]
+            f[1 + i % 4] = 0.125 + (i - 30) * 2.0 ** -55
+            f[5 + i % 4] = 0.03125 + (30 - i) * 2.0 ** -57
+        elif case == "small":
+            f[5 + i % 4], f[1 + i % 4] = (2.0 ** -8 + i * 2.0 ** -60, 0.0)
+        ld = (4.0 - 2.0 * omega) / (4.0 * 0.25 * omega + 2.0 - omega)
+        a = np.array(f)
+        assert lib.hc_collide_quick(KINDS[kind], a.ctypes.data, omega, ld) == 0
+        ref, rho, jx, jy = exact_collide(kind, [Fr(v) for v in f], Fr(omega), Fr(ld))
+        for q in range(9):
+            drift = max(omega, ld, 1.0) * 2.0 ** -54 * float(rho if q == 0 else (abs(jx) + abs(jy) if q < 5 else 0))
+            tol = (0.5 * math.ulp(abs(a[q])) + 2.0 ** -57 + 2.0 ** -58 + drift + 2.0 ** -51 * abs(a[q] - f[q])
+                   + (2.0 ** -58 if case == "small" else 0))  # populations below 2^-7 are rounded by the load
+            assert abs(float(Fr(a[q]) - ref[q])) <= tol, (q, float(Fr(a[q]) - ref[q]), tol)
