@@ -275,7 +275,8 @@ int plbm_hybrid_range_flag(int *flag, int reset);
  * the grid's magic parameter).  Every grid keeps the layout f(ld,nx,0:8),
  * ld = pad16(ny), with two lattices packed in one allocation.
  *
- * Work is cut into tiles of ty rows (y) x threads/ty columns of one grid;
+ * A grid's rows are cut into strips of ty rows (the last one takes the
+ * remainder as well), a strip's cells, y fastest, into tiles of `threads`;
  * ty is chosen per grid from the bucket of its ny (<=48, <=96, <=192,
  * <=384, >384).  persistent = 1 runs all steps of a plbm_batch_run in ONE
  * cooperative launch with a grid-wide barrier between steps (bounded wait:
@@ -287,7 +288,7 @@ typedef struct plbm_batch_schedule {
     int threads;       /* threads per CTA, multiple of 32 in [64, 512]          */
     int ctas_per_sm;   /* resident CTAs per SM, 0 = occupancy maximum           */
     int persistent;    /* 1 = one cooperative launch for all steps              */
-    int ty[PLBM_BATCH_BUCKETS]; /* tile rows per ny bucket, power of 2 >= 32    */
+    int ty[PLBM_BATCH_BUCKETS]; /* strip rows per ny bucket, power of 2 >= 32   */
 } plbm_batch_schedule;
 typedef struct plbm_batch plbm_batch_t;
 

@@ -26,10 +26,9 @@ CollParams plbm_make_params(double omega, double trt_magic);
 
 struct plbm_batch {
   int ngrids = 0, storage = 0, device = 0, sms = 0, math = PLBM_MATH_FMA;
-  std::vector<BatchGrid> grids;   // host copy (off, sizes, params, ty)
+  std::vector<BatchGrid> grids;   // host copy (off, sizes, params)
   BatchGrid* d_grids = nullptr;
-  int2* d_tile_xy = nullptr;    // first cell of each tile (capacity tile_cap)
-  int* d_tile_grid = nullptr;   // grid index of each tile (capacity tile_cap)
+  BatchTile* d_tiles = nullptr;  // capacity tile_cap
   size_t tile_cap = 0;
   int small_index = 1;          // every lattice pair has < 2^32 elements
   int ntiles = 0, nt_bgk = 0;
@@ -80,47 +79,47 @@ void drop_graphs(plbm_batch_t* b) {
 
 // Tiles are numbered grid by grid, the BGK grids' first and the TRT grids'
 // after them, so that the per-step launch can run each kind with its own
-// kernel over a contiguous range; each tile records its grid and first cell.
+// kernel over a contiguous range.
 int apply_schedule(plbm_batch_t* b) {
-  std::vector<int> owner;
-  std::vector<int2> xy;
+  std::vector<BatchTile> tiles;
+  const int threads = b->sched.threads;
   b->nt_bgk = 0;
   for (int pass = 0; pass < 2; pass++) {
     for (int i = 0; i < b->ngrids; i++) {
-      BatchGrid& g = b->grids[i];
+      const BatchGrid& g = b->grids[i];
       if ((g.kind == PLBM_BGK) != (pass == 0)) continue;
-      g.ty = b->sched.ty[bucket_of(g.ny)];
-      g.lty = 0;
-      while ((1 << g.lty) < g.ty) g.lty++;
-      const int tx = b->sched.threads / g.ty;
-      const int tiles_y = (g.ny + g.ty - 1) / g.ty, tiles_x = (g.nx + tx - 1) / tx;
-      if ((long long)owner.size() + (long long)tiles_x * tiles_y > 0x7fffffffLL)
-        return fail(PLBM_E_INVALID, "too many tiles");
-      for (int a = 0; a < tiles_x; a++)
-        for (int c = 0; c < tiles_y; c++) {
-          owner.push_back(i);
-          xy.push_back(make_int2(a * tx, c * g.ty));
+      const int ty = b->sched.ty[bucket_of(g.ny)];
+      for (int y0 = 0; y0 < g.ny;) {
+        const int h = g.ny - y0 < 2 * ty ? g.ny - y0 : ty;
+        const long long cells = (long long)g.nx * h;
+        if ((long long)tiles.size() + (cells + threads - 1) / threads > 0x7fffffffLL)
+          return fail(PLBM_E_INVALID, "too many tiles");
+        BatchTile t{};
+        t.y0 = y0;
+        t.div = ((1u << kTileDivShift) + h - 1) / h;
+        t.grid = i;
+        for (long long k = 0; k < cells; k += threads) {
+          t.x0 = (int)(k / h);
+          t.r0_h = (unsigned)(k % h) | (unsigned)h << 16;
+          tiles.push_back(t);
         }
+        y0 += h;
+      }
     }
-    if (pass == 0) b->nt_bgk = (int)owner.size();
+    if (pass == 0) b->nt_bgk = (int)tiles.size();
   }
-  b->ntiles = (int)owner.size();
+  b->ntiles = (int)tiles.size();
   if ((size_t)b->ntiles > b->tile_cap) {
-    cudaFree(b->d_tile_grid);
-    cudaFree(b->d_tile_xy);
-    b->d_tile_grid = nullptr;
-    b->d_tile_xy = nullptr;
+    cudaFree(b->d_tiles);
+    b->d_tiles = nullptr;
     b->tile_cap = 0;
-    CUDA_TRY(cudaMalloc(&b->d_tile_grid, sizeof(int) * (size_t)b->ntiles), "cudaMalloc(tile table)");
-    CUDA_TRY(cudaMalloc(&b->d_tile_xy, sizeof(int2) * (size_t)b->ntiles), "cudaMalloc(tile table)");
-    b->tile_cap = (size_t)b->ntiles;
+    CUDA_TRY(cudaMalloc(&b->d_tiles, sizeof(BatchTile) * tiles.size()), "cudaMalloc(tile table)");
+    b->tile_cap = tiles.size();
   }
   CUDA_TRY(cudaMemcpy(b->d_grids, b->grids.data(), sizeof(BatchGrid) * b->ngrids, cudaMemcpyHostToDevice),
            "upload batch table");
-  CUDA_TRY(cudaMemcpy(b->d_tile_xy, xy.data(), sizeof(int2) * xy.size(), cudaMemcpyHostToDevice),
+  CUDA_TRY(cudaMemcpy(b->d_tiles, tiles.data(), sizeof(BatchTile) * tiles.size(), cudaMemcpyHostToDevice),
            "upload tile table");
-  CUDA_TRY(cudaMemcpy(b->d_tile_grid, owner.data(), sizeof(int) * owner.size(), cudaMemcpyHostToDevice),
-           "upload tile owners");
   int per_sm = 0;
   CUDA_TRY(batch_max_ctas(b->storage, b->sched.threads, b->small_index, &per_sm), "occupancy");
   if (per_sm < 1) return fail(PLBM_E_UNSUPPORTED, "batched kernel does not fit on an SM with %d threads", b->sched.threads);
@@ -133,8 +132,7 @@ int apply_schedule(plbm_batch_t* b) {
 BatchLaunch launch_of(const plbm_batch_t* b) {
   BatchLaunch L;
   L.grids = b->d_grids;
-  L.tile_xy = b->d_tile_xy;
-  L.tile_grid = b->d_tile_grid;
+  L.tiles = b->d_tiles;
   L.nt_bgk = b->nt_bgk;
   L.small_index = b->small_index;
   L.ngrids = b->ngrids;
@@ -257,8 +255,7 @@ extern "C" int plbm_batch_destroy(plbm_batch_t* b) {
   drop_graphs(b);
   cudaFree(b->base);
   cudaFree(b->d_grids);
-  cudaFree(b->d_tile_xy);
-  cudaFree(b->d_tile_grid);
+  cudaFree(b->d_tiles);
   cudaFree(b->ctrl);
   cudaFree(b->scratch);
   if (b->own) cudaStreamDestroy(b->own);

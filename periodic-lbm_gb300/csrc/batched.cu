@@ -3,11 +3,12 @@
 //
 // Layout: every grid keeps the reference layout f(ld,nx,0:8) (ld = pad16(ny))
 // with two lattices A and B, all grids packed into one device allocation.
-// Work unit: a tile of TY x TX cells of one grid (TY rows along the fast y
-// axis, TX = threads / TY columns), TY chosen per grid by the schedule.  The
-// tiles of all grids are numbered 0..T-1, the BGK grids' first; a table holds
-// each tile's grid and first cell.  Persistent CTA b takes tiles b, b + nCTA,
-// ...; the per-step launch gives each tile its own CTA.
+// Work unit: a tile of `threads` consecutive cells of a strip of one grid's rows
+// (y fastest), the strips cut by the schedule's ty.  The tiles of all grids are
+// numbered 0..T-1, the BGK grids' first; a table holds each tile's grid and first
+// cell.  Persistent CTA b takes tiles b, b + nCTA, ...; the per-step launch gives
+// each tile its own CTA.  (Tiles of ty rows by threads / ty columns left 28 % of
+// their threads past the edges of 48 grids of 32 to 512 cells a side.)
 //
 // Two launch modes, both capturable in a CUDA graph:
 //   * persistent: ONE cooperative launch runs all steps; the CTAs meet at a
@@ -18,9 +19,8 @@
 //     then holds those nodes); with 128-thread CTAs each kind runs a kernel
 //     compiled for it alone.
 //
-// Lattice loads use ld.global.cg (L2 only): in the persistent kernel a lattice
-// written in step s by other SMs is read in step s+1, and the non-coherent L1 /
-// read-only path could return lines cached before it was written.
+// Deviation-storage lattice loads of the persistent kernel use ld.global.cg (L2
+// only): a lattice written in step s by other SMs is read in step s+1.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -67,42 +67,56 @@ __device__ __noinline__ void fallback_cell(const double* __restrict__ src, doubl
   for (int q = 0; q < 9; q++) dst[YFast::off(x, y, q, nx, ny, ld)] = f[q];
 }
 
-// Process one tile of one grid for one step.  I: index type inside one grid's
-// lattice pair (32-bit when every grid's pair has fewer than 2^32 elements).
-// KIND: K_BGK or K_TRT, or (deviation storage) -1 for the grid's own, read at
-// run time.  Binary64 grids take the fixed-point collisions of
-// hybrid.cuh in either arithmetic (their error is no larger than the binary64
-// operator's).  gp is the grid's table entry; its relaxation constants are read
-// where they are used (through the read-only path) rather than held in
-// registers.  xy is the tile's first cell; its TY = 2^lty rows run along y.
+// The cell of this thread in tile t, one of `threads` consecutive cells of a strip of
+// rows (y fastest; see plbm_batched.h).
+struct Cell {
+  const BatchGrid* gp;
+  int x, y;  // x >= nx: past the strip's last cell
+};
+__device__ __forceinline__ Cell cell_of(const BatchGrid* __restrict__ grids, const BatchTile* __restrict__ tiles, int t) {
+  const int4 a = __ldg(reinterpret_cast<const int4*>(tiles + t));
+  const unsigned h = (unsigned)a.z >> 16, j = ((unsigned)a.z & 0xffffu) + threadIdx.x;
+  const unsigned c = (j * (unsigned)a.w) >> kTileDivShift;  // j / h
+  return {grids + __ldg(&tiles[t].grid), a.x + (int)c, a.y + (int)(j - c * h)};
+}
+
+// Offsets of the nine populations that stream into a cell.
+// I: index type inside one grid's lattice pair (32-bit when every grid's pair has
+// fewer than 2^32 elements).
+template <typename I>
+struct PullOff {
+  I q[9];
+  __device__ __forceinline__ PullOff(int x, int y, int nx, int ny, int ld) {
+    const I L = (I)ld, P = L * (I)nx;
+    const I c0 = (I)x * L, cm = (I)wrap_m(x, nx) * L, cp = (I)wrap_p(x, nx) * L;
+    const I y0 = (I)y, ym = (I)wrap_m(y, ny), yp = (I)wrap_p(y, ny);
+    q[0] = c0 + y0;
+    q[1] = P + cm + y0;
+    q[2] = 2 * P + c0 + ym;
+    q[3] = 3 * P + cp + y0;
+    q[4] = 4 * P + c0 + yp;
+    q[5] = 5 * P + cm + ym;
+    q[6] = 6 * P + cp + ym;
+    q[7] = 7 * P + cp + yp;
+    q[8] = 8 * P + cm + yp;
+  }
+};
+template <typename E>
+__device__ __forceinline__ E* lattice_of(const BatchGrid* gp, int which, E* base) {
+  const long long lat = 9LL * __ldg(&gp->ld) * __ldg(&gp->nx);
+  return base + __ldg(&gp->off) + (which ? lat : 0);
+}
+
+// Collide and store one cell.  KIND: K_BGK or K_TRT, or (deviation storage) -1 for
+// the grid's own, read at run time.  Binary64 grids take the fixed-point
+// collisions of hybrid.cuh in either arithmetic (their error is no larger than
+// the binary64 operator's).  The grid's relaxation constants are read where they
+// are used (through the read-only path) rather than held in registers.
 template <class S, bool CG, typename I, int KIND>
-__device__ __forceinline__ void do_tile(const BatchGrid* __restrict__ gp, int2 xy, int parity,
-                                        typename S::elem* __restrict__ base) {
-  const int nx = __ldg(&gp->nx), ny = __ldg(&gp->ny), ld = __ldg(&gp->ld);
-  const int lty = __ldg(&gp->lty);
-  const int y = xy.y + (int)(threadIdx.x & ((1u << lty) - 1u));
-  const int x = xy.x + (int)(threadIdx.x >> lty);
-  if (x >= nx || y >= ny) return;
-  const long long goff = __ldg(&gp->off);
-  const I L = (I)ld, P = (I)ld * (I)nx, lat = 9 * P;
-  const typename S::elem* src = base + goff + (parity ? lat : 0);
-  typename S::elem* dst = base + goff + (parity ? 0 : lat);
-  const I c0 = (I)x * L, cm = (I)wrap_m(x, nx) * L, cp = (I)wrap_p(x, nx) * L;
-  const I y0 = (I)y, ym = (I)wrap_m(y, ny), yp = (I)wrap_p(y, ny);
-  typedef typename S::elem E;
-  E e[9];
-  e[0] = load_pop<CG>(src + (c0 + y0));
-  e[1] = load_pop<CG>(src + (P + cm + y0));
-  e[2] = load_pop<CG>(src + (2 * P + c0 + ym));
-  e[3] = load_pop<CG>(src + (3 * P + cp + y0));
-  e[4] = load_pop<CG>(src + (4 * P + c0 + yp));
-  e[5] = load_pop<CG>(src + (5 * P + cm + ym));
-  e[6] = load_pop<CG>(src + (6 * P + cp + ym));
-  e[7] = load_pop<CG>(src + (7 * P + cp + yp));
-  e[8] = load_pop<CG>(src + (8 * P + cm + yp));
-  typename S::real f[9];
-#pragma unroll
-  for (int q = 0; q < 9; q++) f[q] = (typename S::real)e[q];
+__device__ __forceinline__ void collide_cell(typename S::real (&f)[9], const Cell& c, int parity,
+                                             typename S::elem* __restrict__ base) {
+  const BatchGrid* gp = c.gp;
+  typename S::elem* dst = lattice_of(gp, !parity, base);
   if constexpr (S::ddf) {
     if (KIND == K_TRT || (KIND < 0 && __ldg(&gp->kind) == K_TRT)) collide_shift<K_TRT, typename S::real>(f, gp->p);
     else collide_shift<K_BGK, typename S::real>(f, gp->p);
@@ -111,24 +125,32 @@ __device__ __forceinline__ void do_tile(const BatchGrid* __restrict__ gp, int2 x
     if constexpr (KIND == K_TRT) hy::trt_fma(f, gp->ht, bad);
     else hy::bgk_fma(f, gp->hp, bad);
     if (bad) {  // outside the fixed point's range: the binary64 operator on the same inputs
-      fallback_cell<CG>(src, dst, x, y, gp);
+      fallback_cell<CG>(lattice_of(gp, parity, base), dst, c.x, c.y, gp);
       return;
     }
   }
-  const I o = c0 + y0;
+  const I L = (I)__ldg(&gp->ld), P = L * (I)__ldg(&gp->nx), o = (I)c.x * L + (I)c.y;
 #pragma unroll
   for (int q = 0; q < 9; q++) S::store(dst, (size_t)((I)q * P + o), f[q]);
 }
 
-// Tiles t = first + blockIdx.x, + gridDim.x, ... below last, all of one
-// collision kind; the grid of tile t is tile_grid[t], its first cell
-// tile_xy[t] (both precomputed).
+// One tile for one step.
 template <class S, bool CG, typename I, int KIND>
-__device__ __forceinline__ void sweep(const BatchGrid* __restrict__ grids, const int2* __restrict__ tile_xy,
-                                      const int* __restrict__ tile_grid, int first, int last, int parity,
-                                      typename S::elem* base) {
-  for (int t = first; t < last; t += gridDim.x)
-    do_tile<S, CG, I, KIND>(grids + __ldg(tile_grid + t), __ldg(tile_xy + t), parity, base);
+__device__ __forceinline__ void do_tile(const BatchGrid* __restrict__ grids, const BatchTile* __restrict__ tiles, int t,
+                                        int parity, typename S::elem* __restrict__ base) {
+  const Cell c = cell_of(grids, tiles, t);
+  if (c.x >= __ldg(&c.gp->nx)) return;
+  const typename S::elem* src = lattice_of(c.gp, parity, base);
+  typename S::elem e[9];
+  {
+    const PullOff<I> off(c.x, c.y, __ldg(&c.gp->nx), __ldg(&c.gp->ny), __ldg(&c.gp->ld));
+#pragma unroll
+    for (int q = 0; q < 9; q++) e[q] = load_pop<CG>(src + off.q[q]);
+  }
+  typename S::real f[9];
+#pragma unroll
+  for (int q = 0; q < 9; q++) f[q] = (typename S::real)e[q];
+  collide_cell<S, CG, I, KIND>(f, c, parity, base);
 }
 
 // Grid-wide barrier with a bounded wait.  Returns false when the wait ran out
@@ -172,28 +194,133 @@ constexpr int batch_min_blocks(int max_threads) {
   return (S::ddf ? 1536 : 1024) / max_threads;
 }
 
-// Binary64: the BGK tiles (t < nt_bgk) and the TRT tiles run in loops of their own, each
-// compiled for its kind: with the kind read per tile inside one loop the
-// binary64 kernel took 114 registers, 2 CTAs of 256 per SM (48 grids, 4.0 M
-// cells: 0.204 ms per step against 0.163).  A CTA that ends its BGK
-// tiles early goes on with its share of the TRT tiles: tile t of either kind
-// belongs to CTA t mod gridDim.x.  Deviation storage reads the kind per tile:
-// both collisions fit in the registers of one, and the shared loads are the
-// faster form (0.0566 ms per step, 0.0571 in two loops).
+// A binary64 tile as the persistent kernel keeps it in shared memory: the tile, its
+// grid's sizes and the relaxation constants (a CTA has the same tiles in every step;
+// read from global memory for each tile, they put three dependent L2 latencies
+// before its loads and several before its collision).
+struct alignas(16) OwnTile {
+  int x0, y0;
+  unsigned r0_h, div;
+  int nx, ny, ld, grid;
+  long long off;  // of the lattice pair
+  union {
+    hy::BgkParams hp;
+    hy::TrtFmaParams ht;
+  };
+};
+constexpr int kOwnTiles = 32;  // CTAs with more read them in turns
+
+__device__ __forceinline__ void own_tile(OwnTile& o, const BatchGrid* __restrict__ grids,
+                                         const BatchTile* __restrict__ tiles, int t, int nt_bgk) {
+  const BatchTile b = tiles[t];
+  const BatchGrid* g = grids + b.grid;
+  o.x0 = b.x0, o.y0 = b.y0, o.r0_h = b.r0_h, o.div = b.div;
+  o.nx = g->nx, o.ny = g->ny, o.ld = g->ld, o.grid = b.grid, o.off = g->off;
+  if (t < nt_bgk) o.hp = g->hp;
+  else o.ht = g->ht;
+}
+
+__device__ __forceinline__ void own_cell(const OwnTile& o, int& x, int& y) {
+  const unsigned h = o.r0_h >> 16, j = (o.r0_h & 0xffffu) + threadIdx.x;
+  const unsigned c = (j * o.div) >> kTileDivShift;  // j / h
+  x = o.x0 + (int)c;
+  y = o.y0 + (int)(j - c * h);
+}
+
+// This thread's nine populations of a tile into a stage of shared memory.
+template <typename I>
+__device__ __forceinline__ void copy_tile(const OwnTile& o, int parity, const double* base, double* stage) {
+  int x, y;
+  own_cell(o, x, y);
+  if (x < o.nx) {
+    const double* src = base + o.off + (parity ? 9LL * o.ld * o.nx : 0);
+    const PullOff<I> off(x, y, o.nx, o.ny, o.ld);
+    const unsigned s0 = (unsigned)__cvta_generic_to_shared(stage + threadIdx.x);
+#pragma unroll
+    for (int q = 0; q < 9; q++)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(s0 + q * 8u * blockDim.x), "l"(src + off.q[q])
+                   : "memory");
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// Binary64 tiles [i, last) of a CTA's table (the copies end at n), of one kind: the BGK
+// grids' and the TRT grids' tiles in a loop each (with the kind read per tile the
+// kernel took 114 registers).  Each thread copies its own nine populations of the next
+// tile into shared memory (cp.async) while it collides the present ones.  The copies
+// go through L1: the fence of the grid barrier before them discards what an earlier
+// step left there.
+template <typename I, int KIND>
+__device__ __forceinline__ void sweep_ahead(const BatchGrid* __restrict__ grids, const OwnTile* own, int& i, int last,
+                                            int n, int parity, int& stage, double* sm, double* base) {
+  for (; i < last; i++) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    double f[9];
+    const double* mine = sm + stage * 9 * blockDim.x + threadIdx.x;
+#pragma unroll
+    for (int q = 0; q < 9; q++) f[q] = mine[q * blockDim.x];
+    stage ^= 1;
+    if (i + 1 < n) copy_tile<I>(own[i + 1], parity, base, sm + stage * 9 * blockDim.x);
+    const OwnTile& o = own[i];
+    int x, y;
+    own_cell(o, x, y);
+    if (x >= o.nx) continue;
+    bool bad = false;
+    if constexpr (KIND == K_TRT) hy::trt_fma(f, o.ht, bad);
+    else hy::bgk_fma(f, o.hp, bad);
+    const long long lat = 9LL * o.ld * o.nx;
+    double* pair = base + o.off;
+    double* dst = pair + (parity ? 0 : lat);
+    if (bad) {  // outside the fixed point's range: the binary64 operator on the same inputs
+      fallback_cell<true>(pair + (parity ? lat : 0), dst, x, y, grids + o.grid);
+      continue;
+    }
+    const I P = (I)o.ld * (I)o.nx;
+    dst += (I)x * (I)o.ld + (I)y;
+#pragma unroll
+    for (int q = 0; q < 9; q++) dst[(I)q * P] = f[q];
+  }
+}
+
+// All steps of a run.  Tile t belongs to CTA t mod gridDim.x.  Binary64: see
+// sweep_ahead.  Deviation storage reads the kind per tile: both collisions fit in the
+// registers of one (0.0566 ms per step of 48 grids, 4.0 M cells; 0.0571 in two loops).
+//
+// 48 grids of 32 to 512 cells a side, 1.42 M cells, us per step: tiles of ty by
+// threads / ty cells with loads for each 70; tiles of consecutive cells, columns copied
+// ahead 62; the tiles' table and constants in shared memory 53.  About a quarter
+// of it is the barrier and the memory's latency after it.  Waiting for chunks of
+// whole grids instead (each of which depends on itself alone) lost more to every
+// further release and acquire, 4 us each, than it gained: 2 chunks 53, 4 chunks 61.
+// 512 grids, 39 M cells: 1.94 -> 1.12 ms per step.
 template <class S, typename I, int MAXT>
 __global__ void __launch_bounds__(MAXT, batch_min_blocks<S>(MAXT))
-    k_batch_persistent(const BatchGrid* __restrict__ grids, const int2* __restrict__ tile_xy,
-                       const int* __restrict__ tile_grid, int nt_bgk, int ntiles, int nsteps, int parity0,
-                       typename S::elem* base, Ctrl* ctrl) {
-  const int r = nt_bgk % (int)gridDim.x;
-  const int trt0 = nt_bgk + ((int)blockIdx.x >= r ? (int)blockIdx.x - r : (int)blockIdx.x + (int)gridDim.x - r);
+    k_batch_persistent(const BatchGrid* __restrict__ grids, const BatchTile* __restrict__ tiles, int nt_bgk, int ntiles,
+                       int nsteps, int parity0, typename S::elem* base, Ctrl* ctrl) {
+  // own tiles below tile t
+  auto own_below = [](int t) { return t > (int)blockIdx.x ? (t - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0; };
+  const int count = own_below(ntiles), nb = own_below(nt_bgk);
+  int stage = 0;
   for (int s = 0; s < nsteps; s++) {
     const int parity = (parity0 + s) & 1;
     if constexpr (S::ddf) {
-      sweep<S, true, I, -1>(grids, tile_xy, tile_grid, blockIdx.x, ntiles, parity, base);
+      for (int t = blockIdx.x; t < ntiles; t += gridDim.x) do_tile<S, true, I, -1>(grids, tiles, t, parity, base);
     } else {
-      sweep<S, true, I, K_BGK>(grids, tile_xy, tile_grid, blockIdx.x, nt_bgk, parity, base);
-      sweep<S, true, I, K_TRT>(grids, tile_xy, tile_grid, trt0, ntiles, parity, base);
+      extern __shared__ double sm[];  // 2 x 9 x threads
+      __shared__ OwnTile own[kOwnTiles];
+      for (int i0 = 0; i0 < count; i0 += kOwnTiles) {
+        const int n = min(kOwnTiles, count - i0);
+        if (s == 0 || count > kOwnTiles) {
+          __syncthreads();
+          if ((int)threadIdx.x < n)
+            own_tile(own[threadIdx.x], grids, tiles, blockIdx.x + (i0 + threadIdx.x) * gridDim.x, nt_bgk);
+          __syncthreads();
+        }
+        int i = 0;
+        copy_tile<I>(own[0], parity, base, sm + stage * 9 * blockDim.x);
+        sweep_ahead<I, K_BGK>(grids, own, i, max(0, min(nb - i0, n)), n, parity, stage, sm, base);
+        sweep_ahead<I, K_TRT>(grids, own, i, n, n, parity, stage, sm, base);
+      }
     }
     if (s + 1 < nsteps && !barrier(ctrl, s)) return;
   }
@@ -203,15 +330,14 @@ __global__ void __launch_bounds__(MAXT, batch_min_blocks<S>(MAXT))
 // compiled for that kind alone: the binary64 BGK tiles take 64 registers and
 // the TRT tiles 72.  One kernel for both kinds needed far more registers than
 // either (97 for the earlier forms, 80 under a cap with spills, 20.9k MLUPS on
-// the 512-grid batch against 24.5k split by kind).
+// the 512-grid batch against 24.5k split by kind; 33.7k with tiles of consecutive
+// cells and the present collisions).
 template <class S, typename I, int KIND, int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB) k_batch_kind(const BatchGrid* __restrict__ grids,
-                                                          const int2* __restrict__ tile_xy,
-                                                          const int* __restrict__ tile_grid, int t0, int parity,
+                                                          const BatchTile* __restrict__ tiles, int t0, int parity,
                                                           typename S::elem* base) {
   chain_begin();
-  const int t = t0 + (int)blockIdx.x;
-  do_tile<S, false, I, KIND>(grids + __ldg(tile_grid + t), __ldg(tile_xy + t), parity, base);
+  do_tile<S, false, I, KIND>(grids, tiles, t0 + (int)blockIdx.x, parity, base);
 }
 
 // Per-step launch over all tiles, for deviation storage in CTAs other than 128
@@ -219,12 +345,10 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch_kind(const BatchGrid* __re
 // kind).
 template <class S, typename I>
 __global__ void __launch_bounds__(kBatchMaxThreads) k_batch_step(const BatchGrid* __restrict__ grids,
-                                                                const int2* __restrict__ tile_xy,
-                                                                const int* __restrict__ tile_grid, int parity,
+                                                                const BatchTile* __restrict__ tiles, int parity,
                                                                 typename S::elem* base) {
   chain_begin();
-  const int t = (int)blockIdx.x;
-  do_tile<S, false, I, -1>(grids + __ldg(tile_grid + t), __ldg(tile_xy + t), parity, base);
+  do_tile<S, false, I, -1>(grids, tiles, (int)blockIdx.x, parity, base);
 }
 
 template <class S, typename I, int MAXT>
@@ -235,10 +359,17 @@ cudaError_t launch_kinds(const BatchLaunch& L, int parity) {
   constexpr int bgk_blocks = MAXT == 128 ? 8 : batch_min_blocks<S>(MAXT);
   constexpr int trt_blocks = MAXT == 128 ? 7 : batch_min_blocks<S>(MAXT);
   if (L.nt_bgk > 0)
-    chained(k_batch_kind<S, I, K_BGK, MAXT, bgk_blocks>, L.nt_bgk, L.threads, L.stream)(L.grids, L.tile_xy, L.tile_grid, 0, parity, base);
+    chained(k_batch_kind<S, I, K_BGK, MAXT, bgk_blocks>, L.nt_bgk, L.threads, L.stream)(L.grids, L.tiles, 0, parity, base);
   if (ntrt > 0)
-    chained(k_batch_kind<S, I, K_TRT, MAXT, trt_blocks>, ntrt, L.threads, L.stream)(L.grids, L.tile_xy, L.tile_grid, L.nt_bgk, parity, base);
+    chained(k_batch_kind<S, I, K_TRT, MAXT, trt_blocks>, ntrt, L.threads, L.stream)(L.grids, L.tiles, L.nt_bgk, parity, base);
   return cudaGetLastError();
+}
+
+// Dynamic shared memory of the persistent kernel (raised past 48 KB where the
+// schedule is applied, in batch_max_ctas).
+template <class S>
+int persistent_smem(int threads) {
+  return S::ddf ? 0 : 2 * 9 * 8 * threads;
 }
 
 template <class S, typename I>
@@ -257,7 +388,8 @@ cudaError_t launch_batch(const BatchLaunch& L, int nsteps, int parity0) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     auto kernel = !S::ddf && L.threads <= 256 ? k_batch_persistent<S, I, 256> : k_batch_persistent<S, I, kBatchMaxThreads>;
-    return cudaLaunchKernelEx(&cfg, kernel, L.grids, L.tile_xy, L.tile_grid, L.nt_bgk, L.ntiles, nsteps, parity0,
+    cfg.dynamicSmemBytes = persistent_smem<S>(L.threads);
+    return cudaLaunchKernelEx(&cfg, kernel, L.grids, L.tiles, L.nt_bgk, L.ntiles, nsteps, parity0,
                               base, ctrl);
   }
   // one tile per CTA
@@ -267,7 +399,7 @@ cudaError_t launch_batch(const BatchLaunch& L, int nsteps, int parity0) {
     if (L.threads <= 128 && (!S::ddf || L.threads == 128)) {
       e = launch_kinds<S, I, 128>(L, parity);
     } else if constexpr (S::ddf) {
-      chained(k_batch_step<S, I>, L.ntiles, L.threads, L.stream)(L.grids, L.tile_xy, L.tile_grid, parity, base);
+      chained(k_batch_step<S, I>, L.ntiles, L.threads, L.stream)(L.grids, L.tiles, parity, base);
       e = cudaGetLastError();
     } else {
       e = L.threads <= 256 ? launch_kinds<S, I, 256>(L, parity) : launch_kinds<S, I, kBatchMaxThreads>(L, parity);
@@ -291,7 +423,10 @@ namespace {
 template <class S, typename I>
 cudaError_t persistent_ctas(int threads, int* per_sm) {
   auto kernel = !S::ddf && threads <= 256 ? k_batch_persistent<S, I, 256> : k_batch_persistent<S, I, kBatchMaxThreads>;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, threads, 0);
+  const int smem = persistent_smem<S>(threads);
+  if (smem > 48 * 1024)
+    if (cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) return e;
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, threads, smem);
 }
 }  // namespace
 

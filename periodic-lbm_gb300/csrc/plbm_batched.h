@@ -17,18 +17,28 @@ struct alignas(16) BatchGrid {
   long long off;      // element offset of lattice A; lattice B follows it
   int nx, ny, ld;
   int kind;           // K_BGK or K_TRT
-  int ty;             // tile rows along y; tile columns = threads / ty
-  int lty;            // log2(ty)
-  int pad[2];
 };
+
+// A tile: `threads` consecutive cells of a strip of h rows, column after column (y
+// fastest), the first one at (x0, y0 + r0).  A grid's rows are cut into strips of
+// ty rows, the last one taking the remainder as well: h < 2 ty <= 1024.
+struct alignas(16) BatchTile {
+  int x0, y0;
+  unsigned r0_h;  // r0 | h << 16
+  unsigned div;   // ceil(2^kTileDivShift / h): j / h = j div >> kTileDivShift for j < h + 512
+  int grid;
+  int pad[3];
+};
+// j div < 1536 2^21 < 2^32, and j times div's rounding (less than h / h) is below
+// 1536 x 1024 < 2^21: the quotient is exact.
+constexpr int kTileDivShift = 21;
 
 hy::BgkParams hybrid_bgk_params(double omega);
 hy::TrtFmaParams hybrid_trt_params(const CollParams& p);
 
 struct BatchLaunch {
   const BatchGrid* grids;  // device
-  const int2* tile_xy;     // device, first cell (x0, y0) of each tile
-  const int* tile_grid;    // device, grid index of each tile
+  const BatchTile* tiles;  // device
   int ngrids, ntiles;
   int nt_bgk;              // tiles [0, nt_bgk) belong to BGK grids, the rest to TRT grids
   int threads, ctas;       // ctas: persistent mode only (per-step: one CTA per tile)
