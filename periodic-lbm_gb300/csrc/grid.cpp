@@ -24,20 +24,56 @@
 
 using namespace plbm;
 
-int plbm::block_for(long long cells, bool binary64) {
-  static std::atomic<int> sms[64];  // SM count per device, 0 until first asked
-  const int most = binary64 ? (cells <= (1 << 18) ? 64 : 128)
-                            : (cells <= (1 << 17) ? 64 : (cells < (1 << 18) ? 128 : kBlock));
+namespace {
+// SMs of the current device (0: not known).
+int sm_count() {
+  static std::atomic<int> sms[64];  // by device, 0 until first asked
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return most;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
   int n = sms[dev].load(std::memory_order_relaxed);
   if (n < 1) {
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) return most;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) return 0;
     sms[dev].store(n, std::memory_order_relaxed);
   }
+  return n;
+}
+}  // namespace
+
+int plbm::block_for(long long cells, bool binary64) {
+  const int most = binary64 ? (cells <= (1 << 18) ? 64 : 128)
+                            : (cells <= (1 << 17) ? 64 : (cells < (1 << 18) ? 128 : kBlock));
+  const int n = sm_count();
+  if (n < 1) return most;
   const long long per_sm = (cells + n - 1) / n;
   if (per_sm >= most) return most;
   return (int)(per_sm < 32 ? 32 : (per_sm + 31) / 32 * 32);
+}
+
+bool plbm::rows_fit(int nfast, int nslow, bool binary64) {
+  const long long bs = block_for((long long)nfast * nslow, binary64);
+  return 32 * ((nfast + bs - 1) / bs * bs - nfast) <= nfast;
+}
+
+cudaError_t plbm::spread_cells(int nfast, int nslow, bool binary64, bool flat, int resident, Spread* w) {
+  const long long cells = (long long)nfast * nslow;
+  if (cells <= 0) return cudaErrorInvalidConfiguration;
+  w->threads = block_for(cells, binary64);
+  w->smem = 0;
+  w->rows = Rows{(unsigned)nfast, 0, 0};
+  const int per_row = (nfast + w->threads - 1) / w->threads;
+  long long blocks = (cells + w->threads - 1) / w->threads;
+  if (flat && blocks * w->threads < (1LL << 32))
+    w->rows.m = nfast == 1 ? 0xffffffffu : (unsigned)((1ull << 32) / (unsigned)nfast);
+  else
+    w->rows.tiles = (unsigned)per_row, blocks = (long long)nslow * per_row;
+  if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+  w->blocks = (unsigned)blocks;
+  const int n = sm_count();
+  if (n < 1) return cudaSuccess;
+  const long long per_sm = (blocks + n - 1) / n, fits = resident / w->threads;
+  // an SM's 228 KB, of which each CTA takes 1 KB for itself; more than 48 KB need leave
+  if (per_sm <= fits && 2 * per_sm > fits && per_sm >= 5) w->smem = (int)(((228 << 10) / per_sm - 1024) / 128 * 128);
+  return cudaSuccess;
 }
 
 // ---------------------------------------------------------------------------

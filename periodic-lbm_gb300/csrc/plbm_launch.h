@@ -1,6 +1,8 @@
 // plbm_launch.h -- internal launcher interface shared by the translation units
 // of libplbmgpu.so.  Not part of the public C ABI.
 #pragma once
+#include <algorithm>
+#include <atomic>
 #include <cuda_runtime.h>
 #include <stddef.h>
 #include "plbm_device.cuh"
@@ -32,6 +34,34 @@ constexpr int kReduceBlocks = 1216;
 // grid in 16 CTAs of 256 threads spent ~4.5 us per step in its collision.
 int block_for(long long cells, bool binary64);
 
+// Cells in flat order, rows one after the other: thread t of block b has cell
+// b blockDim + t, and no thread lies past a row's end.  (A row in blocks of its own left
+// 17 % of the threads of a 641 x 500 plugin grid without a cell.)
+struct Rows {
+  unsigned n;  // cells of a row
+  unsigned m;  // floor(2^32 / n); 0: blocks of one row each
+  unsigned tiles;  // blocks of a row (m == 0)
+};
+// A launch over such cells.  smem: shared memory that nothing uses, which limits the
+// CTAs an SM holds to its even share of the grid, where an SM holds that share but not
+// two.  Chained launches otherwise fill the rest of every SM with the next step's first
+// CTAs and give its last ones to whichever SM ends early, which then takes twice the
+// others' time (us per step, without flat cells and limit / with flat cells / with both:
+// 300^2 BGK 5.1 / 5.1 / 4.1, 256^2 RR 5.3 / 5.3 / 4.2, 1000 x 65 BGK 4.9 / 3.6 / 3.7,
+// 641 x 500 plugin BGK 11.1 / 10.0 / 10.0, 300^2 plugin RR 45.9 / 45.9 / 29.6).  The same limit
+// on grids of two waves and more: 400^2 BGK 5.6 -> 6.3, not taken.
+struct Spread {
+  unsigned blocks;
+  int threads, smem;
+  Rows rows;
+};
+// flat: rows cut into blocks of their own otherwise, and with 2^32 cells or more.
+// resident: threads of the kernel that an SM's registers hold.
+cudaError_t spread_cells(int nfast, int nslow, bool binary64, bool flat, int resident, Spread* out);
+// Whether rows cut into blocks of their own leave at most 1/32 of the threads without a
+// cell.
+bool rows_fit(int nfast, int nslow, bool binary64);
+
 // Launches of a time loop's kernels, chained by programmatic dependent launch:
 // the next kernel's CTAs are placed while this kernel still runs, and each waits
 // (chain_begin, the first statement of every such kernel) until the kernels
@@ -55,6 +85,7 @@ struct Chained {
   unsigned blocks;
   int threads;
   cudaStream_t stream;
+  int smem;
   // The launch error is returned, and kept for cudaGetLastError.
   template <typename... A>
   cudaError_t operator()(const A&... args) const {
@@ -62,6 +93,7 @@ struct Chained {
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3((unsigned)threads);
     cfg.stream = stream;
+    cfg.dynamicSmemBytes = (size_t)smem;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -71,8 +103,59 @@ struct Chained {
   }
 };
 template <typename... P>
-Chained<P...> chained(void (*kernel)(P...), unsigned blocks, int threads, cudaStream_t stream) {
-  return {kernel, blocks, threads, stream};
+Chained<P...> chained(void (*kernel)(P...), unsigned blocks, int threads, cudaStream_t stream, int smem = 0) {
+  return {kernel, blocks, threads, stream, smem};
+}
+template <typename... P>
+Chained<P...> chained(void (*kernel)(P...), const Spread& w, cudaStream_t stream) {
+  return {kernel, w.blocks, w.threads, stream, w.smem};
+}
+
+// Threads of kernel K that an SM's registers hold.
+template <auto K>
+int resident_threads() {
+  static std::atomic<int> threads{0};  // 0 until first asked
+  int n = threads.load(std::memory_order_relaxed);
+  if (n == 0) {
+    cudaFuncAttributes a;
+    if (cudaFuncGetAttributes(&a, K) != cudaSuccess || a.numRegs < 1) return 2048;
+    // 16,384 registers for each of the four schedulers, a warp's in multiples of 256
+    n = std::min(16, 16384 / (32 * ((a.numRegs + 7) / 8 * 8))) * 4 * 32;
+    threads.store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
+// Deviation storage takes flat cells but on grids larger than the L2 cache whose rows fit
+// their blocks and not their 128-byte lines: warps that straddle lines cost there
+// (binary32 RR 3001 x 2999 97.8 us per step in rows, 102.2 flat; 1000^2 10.6 and 10.0).
+inline bool dev_flat(int nfast, int nslow) {
+  return (long long)nfast * nslow <= (1 << 20) || nfast % 32 == 0 || !rows_fit(nfast, nslow, false);
+}
+
+// Kernel K(src, dst, nx, ny, ld, rows, p), a thread per cell of nslow rows of nfast.
+template <auto K, typename P>
+cudaError_t step_cells(const Sweep& s, int nfast, int nslow, bool binary64, bool flat, const P& p) {
+  Spread w;
+  if (cudaError_t e = spread_cells(nfast, nslow, binary64, flat, resident_threads<K>(), &w)) return e;
+  chained(K, w, s.stream)(s.src, s.dst, s.nx, s.ny, s.ld, w.rows, p);
+  return cudaGetLastError();
+}
+
+// The row and the place in it of this thread's cell; row >= its count: none.
+__device__ __forceinline__ void flat_cell(const Rows& r, int& row, int& place) {
+  if (r.m == 0) {
+    const unsigned s = blockIdx.x / r.tiles, f = (blockIdx.x - s * r.tiles) * blockDim.x + threadIdx.x;
+    row = f < r.n ? (int)s : 0x7fffffff;
+    place = (int)f;
+    return;
+  }
+  const unsigned j = blockIdx.x * blockDim.x;
+  unsigned s = __umulhi(j, r.m);  // j / n or one less
+  unsigned f = j - s * r.n + threadIdx.x;
+  while (f >= r.n) f -= r.n, s++;
+  row = (int)s;
+  place = (int)f;
 }
 #endif
 

@@ -29,10 +29,11 @@ __device__ __forceinline__ bool dev_cell(int ftiles, int nx, int ny, int& x, int
 template <class L, class S, int KIND, bool PUSH>
 __global__ void __launch_bounds__(kBlock) k_step_dev(const typename S::elem* __restrict__ src,
                                                     typename S::elem* __restrict__ dst, int nx, int ny,
-                                                    int ld, int ftiles, CollParams p) {
+                                                    int ld, Rows rows, CollParams p) {
   chain_begin();
   int x, y;
-  if (!dev_cell<L>(ftiles, nx, ny, x, y)) return;
+  flat_cell(rows, L::x_fast ? y : x, L::x_fast ? x : y);
+  if (L::x_fast ? y >= ny : x >= nx) return;
   float h[9];
 #pragma unroll
   for (int q = 0; q < 9; q++) {
@@ -64,14 +65,18 @@ ShiftParamsF shift_params(int kind, const CollParams& p) {
 // The pull step of the src/ layout (YFast) with explicit pull offsets: I is
 // the offset type, 32-bit when the lattice has fewer than 2^32 elements (one
 // multiply-add per address instead of 64-bit index arithmetic).
-template <class S, int KIND, typename I>
+template <class S, int KIND, typename I, bool FLAT>
 __global__ void __launch_bounds__(kBlock) k_step_dev_pull(const typename S::elem* __restrict__ src,
                                                          typename S::elem* __restrict__ dst, int nx, int ny,
-                                                         int ld, int ftiles, ShiftParamsF p) {
+                                                         int ld, Rows rows, ShiftParamsF p) {
   chain_begin();
-  const int x = blockIdx.x / ftiles;
-  const int y = (blockIdx.x - x * ftiles) * blockDim.x + threadIdx.x;
-  if (y >= ny) return;
+  int x, y;
+  if (FLAT) {
+    flat_cell(rows, x, y);
+    if (x >= nx) return;
+  } else if (!dev_cell<YFast>(rows.tiles, nx, ny, x, y)) {
+    return;
+  }
   const I L = (I)ld, P = (I)ld * (I)nx;
   const I c0 = (I)x * L, cm = (I)wrap_m(x, nx) * L, cp = (I)wrap_p(x, nx) * L;
   const I y0 = (I)y, ym = (I)wrap_m(y, ny), yp = (I)wrap_p(y, ny);
@@ -106,11 +111,12 @@ __global__ void __launch_bounds__(kBlock) k_step_dev_pull(const typename S::elem
 // and 4-byte aligned lattices, so that every half2 offset is even.
 template <int KIND, typename I>
 __global__ void __launch_bounds__(kBlock) k_step_f16_pull2(const __half* __restrict__ src, __half* __restrict__ dst,
-                                                          int nx, int ny, int ld, int ftiles, ShiftParamsF p) {
+                                                          int nx, int ny, int ld, Rows rows, ShiftParamsF p) {
   chain_begin();
-  const int x = blockIdx.x / ftiles;
-  const int y = 2 * ((blockIdx.x - x * ftiles) * blockDim.x + threadIdx.x);
-  if (y >= ny) return;
+  int x, y;
+  flat_cell(rows, x, y);
+  if (x >= nx) return;
+  y *= 2;
   const I L = (I)ld, P = (I)ld * (I)nx;
   const I c0 = (I)x * L, cm = (I)wrap_m(x, nx) * L, cp = (I)wrap_p(x, nx) * L;
   const I y0 = (I)y, y1 = (I)(y + 1), ym = (I)wrap_m(y, ny), yp = (I)wrap_p(y + 1, ny);
@@ -178,20 +184,14 @@ inline int tiles(int n) { return (n + kBlock - 1) / kBlock; }
 
 template <class L, class S, bool PUSH>
 cudaError_t launch_dev(int kind, const Sweep& s, const CollParams& p) {
-  const int bs = block_for((long long)s.nx * s.ny, false);
-  const int ft = ((L::x_fast ? s.nx : s.ny) + bs - 1) / bs;
-  const long long blocks = (long long)ft * (L::x_fast ? s.ny : s.nx);
-  if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-  typedef typename S::elem E;
-  const E* a = static_cast<const E*>(s.src);
-  E* b = static_cast<E*>(s.dst);
+  const int nfast = L::x_fast ? s.nx : s.ny, nslow = L::x_fast ? s.ny : s.nx;
+  const bool flat = dev_flat(nfast, nslow);
   switch (kind) {
-    case K_BGK: chained(k_step_dev<L, S, K_BGK, PUSH>, (unsigned)blocks, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p); break;
-    case K_TRT: chained(k_step_dev<L, S, K_TRT, PUSH>, (unsigned)blocks, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p); break;
-    case K_RR: chained(k_step_dev<L, S, K_RR, PUSH>, (unsigned)blocks, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p); break;
+    case K_BGK: return step_cells<k_step_dev<L, S, K_BGK, PUSH>>(s, nfast, nslow, false, flat, p);
+    case K_TRT: return step_cells<k_step_dev<L, S, K_TRT, PUSH>>(s, nfast, nslow, false, flat, p);
+    case K_RR: return step_cells<k_step_dev<L, S, K_RR, PUSH>>(s, nfast, nslow, false, flat, p);
     default: return cudaErrorNotSupported;
   }
-  return cudaGetLastError();
 }
 
 template <class S>
@@ -210,43 +210,27 @@ cudaError_t launch_collide_dev(int kind, const Sweep& s, const CollParams& p) {
   return cudaGetLastError();
 }
 
-template <class S, typename I>
+template <class S, typename I, bool FLAT>
 cudaError_t launch_pull_dev(int kind, const Sweep& s, const CollParams& cp) {
-  const int bs = block_for((long long)s.nx * s.ny, false);
-  const int ft = (s.ny + bs - 1) / bs;
-  const long long blocks = (long long)ft * s.nx;
-  if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-  typedef typename S::elem E;
-  const E* a = static_cast<const E*>(s.src);
-  E* b = static_cast<E*>(s.dst);
   const ShiftParamsF p = shift_params(kind, cp);
-  const unsigned nb = (unsigned)blocks;
   switch (kind) {
-    case K_BGK: chained(k_step_dev_pull<S, K_BGK, I>, nb, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p); break;
-    case K_TRT: chained(k_step_dev_pull<S, K_TRT, I>, nb, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p); break;
-    case K_RR: chained(k_step_dev_pull<S, K_RR, I>, nb, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p); break;
+    case K_BGK: return step_cells<k_step_dev_pull<S, K_BGK, I, FLAT>>(s, s.ny, s.nx, false, FLAT, p);
+    case K_TRT: return step_cells<k_step_dev_pull<S, K_TRT, I, FLAT>>(s, s.ny, s.nx, false, FLAT, p);
+    case K_RR: return step_cells<k_step_dev_pull<S, K_RR, I, FLAT>>(s, s.ny, s.nx, false, FLAT, p);
     default: return cudaErrorNotSupported;
   }
-  return cudaGetLastError();
 }
 
 template <typename I>
 cudaError_t launch_f16_pull2(int kind, const Sweep& s, const CollParams& cp) {
-  const int bs = block_for((long long)s.nx * (s.ny / 2), false);
-  const int ft = (s.ny / 2 + bs - 1) / bs;
-  const long long blocks = (long long)ft * s.nx;
-  if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-  const __half* a = static_cast<const __half*>(s.src);
-  __half* b = static_cast<__half*>(s.dst);
+  const bool flat = dev_flat(s.ny / 2, s.nx);
   const ShiftParamsF p = shift_params(kind, cp);
-  const unsigned nb = (unsigned)blocks;
   switch (kind) {
-    case K_BGK: chained(k_step_f16_pull2<K_BGK, I>, nb, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p); break;
-    case K_TRT: chained(k_step_f16_pull2<K_TRT, I>, nb, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p); break;
-    case K_RR: chained(k_step_f16_pull2<K_RR, I>, nb, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p); break;
+    case K_BGK: return step_cells<k_step_f16_pull2<K_BGK, I>>(s, s.ny / 2, s.nx, false, flat, p);
+    case K_TRT: return step_cells<k_step_f16_pull2<K_TRT, I>>(s, s.ny / 2, s.nx, false, flat, p);
+    case K_RR: return step_cells<k_step_f16_pull2<K_RR, I>>(s, s.ny / 2, s.nx, false, flat, p);
     default: return cudaErrorNotSupported;
   }
-  return cudaGetLastError();
 }
 
 }  // namespace
@@ -257,10 +241,13 @@ cudaError_t step_pull_dev(int storage, int kind, const Sweep& s, const CollParam
                      (((uintptr_t)s.src | (uintptr_t)s.dst) & 3) == 0;
   if (storage == ST_F16DEV && pairs)
     return small ? launch_f16_pull2<uint32_t>(kind, s, p) : launch_f16_pull2<size_t>(kind, s, p);
-  if (storage == ST_F32DEV)
-    return small ? launch_pull_dev<StoreF32Dev, uint32_t>(kind, s, p) : launch_pull_dev<StoreF32Dev, size_t>(kind, s, p);
-  if (storage == ST_F16DEV)
-    return small ? launch_pull_dev<StoreF16Dev, uint32_t>(kind, s, p) : launch_pull_dev<StoreF16Dev, size_t>(kind, s, p);
+  const bool flat = dev_flat(s.ny, s.nx);
+#define PLBM_PULL(S)                                                                                          \
+  return small ? (flat ? launch_pull_dev<S, uint32_t, true>(kind, s, p) : launch_pull_dev<S, uint32_t, false>(kind, s, p)) \
+               : (flat ? launch_pull_dev<S, size_t, true>(kind, s, p) : launch_pull_dev<S, size_t, false>(kind, s, p))
+  if (storage == ST_F32DEV) PLBM_PULL(StoreF32Dev);
+  if (storage == ST_F16DEV) PLBM_PULL(StoreF16Dev);
+#undef PLBM_PULL
   return cudaErrorInvalidValue;
 }
 

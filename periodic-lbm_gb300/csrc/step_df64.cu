@@ -41,11 +41,12 @@ __global__ void __launch_bounds__(kBlock) k_step_dev_df(const typename S::elem* 
 template <class S, typename I>
 __global__ void __launch_bounds__(kBlock) k_step_dev_comp(const typename S::elem* __restrict__ src,
                                                          typename S::elem* __restrict__ dst, int nx, int ny, int ld,
-                                                         int ftiles, df::DevParams p) {
+                                                         Rows rows, df::DevParams p) {
   chain_begin();
-  const int xb = blockIdx.x / ftiles, x = 2 * xb;
-  const int y = (blockIdx.x - xb * ftiles) * blockDim.x + threadIdx.x;
-  if (y >= ny) return;
+  int x, y;
+  flat_cell(rows, x, y);
+  if (x >= (nx + 1) / 2) return;
+  x *= 2;
   const I L = (I)ld, P = (I)ld * (I)nx;
   const int x2 = wrap_p(x, nx);  // the second column (column 0 again after an odd last one)
   const I ca = (I)x * L, cb = (I)x2 * L, cm = (I)wrap_m(x, nx) * L, cp = (I)wrap_p(x2, nx) * L;
@@ -105,24 +106,16 @@ cudaError_t step_pull_dev_hi(int storage, int math, int kind, const Sweep& s, co
   if (math == 2) {  // compensated binary32
     if (kind != K_BGK) return cudaErrorNotSupported;
     const df::DevParams p = df::dev_params(cp.omega);
-    const int bs = block_for((long long)s.nx * s.ny / 2, false);
-    const int ftc = (s.ny + bs - 1) / bs;
-    const unsigned nbc = (unsigned)((long long)ftc * ((s.nx + 1) / 2));
+    const int pairs = s.nx / 2 + (s.nx & 1);
+    const bool flat = dev_flat(s.ny, pairs);
     const bool small = (unsigned long long)s.ld * (unsigned long long)s.nx * 9ull < (1ull << 32);
-    if (storage == ST_F32DEV) {
-      const float* a = static_cast<const float*>(s.src);
-      float* b = static_cast<float*>(s.dst);
-      if (small) chained(k_step_dev_comp<StoreF32Dev, uint32_t>, nbc, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ftc, p);
-      else chained(k_step_dev_comp<StoreF32Dev, size_t>, nbc, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ftc, p);
-    } else if (storage == ST_F16DEV) {
-      const __half* a = static_cast<const __half*>(s.src);
-      __half* b = static_cast<__half*>(s.dst);
-      if (small) chained(k_step_dev_comp<StoreF16Dev, uint32_t>, nbc, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ftc, p);
-      else chained(k_step_dev_comp<StoreF16Dev, size_t>, nbc, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ftc, p);
-    } else {
-      return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
+    if (storage == ST_F32DEV)
+      return small ? step_cells<k_step_dev_comp<StoreF32Dev, uint32_t>>(s, s.ny, pairs, false, flat, p)
+                   : step_cells<k_step_dev_comp<StoreF32Dev, size_t>>(s, s.ny, pairs, false, flat, p);
+    if (storage == ST_F16DEV)
+      return small ? step_cells<k_step_dev_comp<StoreF16Dev, uint32_t>>(s, s.ny, pairs, false, flat, p)
+                   : step_cells<k_step_dev_comp<StoreF16Dev, size_t>>(s, s.ny, pairs, false, flat, p);
+    return cudaErrorInvalidValue;
   }
   if (math == 3) {  // double-float
     if (kind != K_BGK) return cudaErrorNotSupported;

@@ -49,12 +49,19 @@ __device__ __forceinline__ bool cell_of<XFast>(int ftiles, int nx, int ny, int& 
 
 // Fused step.  PUSH=false: pull-stream then collide at the destination cell
 // (src/ semantics).  PUSH=true: collide at the source cell, then push.
-template <class L, int KIND, bool SHIFT, bool PUSH>
+// FLAT: flat cells; rows otherwise (rows_fit), where their arithmetic is 1.5 % of the RR
+// plugin step (2048^2 1.193 and 1.209 ms).
+template <class L, int KIND, bool SHIFT, bool PUSH, bool FLAT>
 __global__ void __launch_bounds__(kBlock) k_step(const double* __restrict__ src, double* __restrict__ dst,
-                                                int nx, int ny, int ld, int ftiles, CollParams p) {
+                                                int nx, int ny, int ld, Rows rows, CollParams p) {
   chain_begin();
   int x, y;
-  if (!cell_of<L>(ftiles, nx, ny, x, y)) return;
+  if (FLAT) {
+    flat_cell(rows, L::x_fast ? y : x, L::x_fast ? x : y);
+    if (L::x_fast ? y >= ny : x >= nx) return;
+  } else if (!cell_of<L>(rows.tiles, nx, ny, x, y)) {
+    return;
+  }
   double f[9];
 #pragma unroll
   for (int q = 0; q < 9; q++) {
@@ -178,24 +185,19 @@ inline int tiles(int n) { return (n + kBlock - 1) / kBlock; }
 
 template <class L, bool SHIFT, bool PUSH>
 cudaError_t launch_step(int kind, const Sweep& s, const CollParams& p) {
-  const int bs = block_for((long long)s.nx * s.ny, true);
-  const int nfast = L::x_fast ? s.nx : s.ny;
-  const int ft = (nfast + bs - 1) / bs;
-  const int nslow = L::x_fast ? s.ny : s.nx;
-  const long long blocks = (long long)ft * nslow;
-  if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-  const double* a = static_cast<const double*>(s.src);
-  double* b = static_cast<double*>(s.dst);
-#define PLBM_STEP(K) chained(k_step<L, K, SHIFT, PUSH>, (unsigned)blocks, bs, s.stream)(a, b, s.nx, s.ny, s.ld, ft, p)
+  const int nfast = L::x_fast ? s.nx : s.ny, nslow = L::x_fast ? s.ny : s.nx;
+  const bool flat = !rows_fit(nfast, nslow, true);
+#define PLBM_STEP(K)                                                                               \
+  return flat ? step_cells<k_step<L, K, SHIFT, PUSH, true>>(s, nfast, nslow, true, true, p)      \
+              : step_cells<k_step<L, K, SHIFT, PUSH, false>>(s, nfast, nslow, true, false, p)
 #ifdef PLBM_STRICT
   switch (kind) {
-    case K_BGK: PLBM_STEP(K_BGK); break;
-    case K_TRT: PLBM_STEP(K_TRT); break;
-    case K_RR: PLBM_STEP(K_RR); break;
+    case K_BGK: PLBM_STEP(K_BGK);
+    case K_TRT: PLBM_STEP(K_TRT);
+    case K_RR: PLBM_STEP(K_RR);
     case K_BGKI:
       if constexpr (SHIFT) return cudaErrorNotSupported;
       else PLBM_STEP(K_BGKI);
-      break;
     default: return cudaErrorInvalidValue;
   }
 #else
@@ -203,15 +205,14 @@ cudaError_t launch_step(int kind, const Sweep& s, const CollParams& p) {
   // point (step_hybrid.cu)
   if constexpr (SHIFT) {
     if (kind == K_TRT) PLBM_STEP(K_TRT);
-    else if (kind == K_RR) PLBM_STEP(K_RR);
-    else return cudaErrorNotSupported;
+    if (kind == K_RR) PLBM_STEP(K_RR);
+    return cudaErrorNotSupported;
   } else {
     if (kind != K_BGKI) return cudaErrorInvalidValue;
     PLBM_STEP(K_BGKI);
   }
 #endif
 #undef PLBM_STEP
-  return cudaGetLastError();
 }
 
 }  // namespace

@@ -58,12 +58,12 @@ constexpr int hybrid_min_blocks(int kind) { return kind == K_RR ? 3 : 4; }
 template <typename I, int KIND, bool QUICK>
 __global__ void __launch_bounds__(kBlock, hybrid_min_blocks(KIND)) k_step_hybrid(const double* __restrict__ src,
                                                                                 double* __restrict__ dst, int nx,
-                                                                                int ny, int ld, int ftiles,
+                                                                                int ny, int ld, Rows rows,
                                                                                 HybridArgs a) {
   chain_begin();
-  const int x = blockIdx.x / ftiles;
-  const int y = (blockIdx.x - x * ftiles) * blockDim.x + threadIdx.x;
-  if (y >= ny) return;
+  int x, y;
+  flat_cell(rows, x, y);
+  if (x >= nx) return;
   const I L = (I)ld, P = (I)ld * (I)nx;
   const I c0 = (I)x * L, cm = (I)wrap_m(x, nx) * L, cp = (I)wrap_p(x, nx) * L;
   const I y0 = (I)y, ym = (I)wrap_m(y, ny), yp = (I)wrap_p(y, ny);
@@ -386,12 +386,12 @@ __device__ __noinline__ void push_fallback_cell(const double* __restrict__ src, 
 template <typename I, int KIND>
 __global__ void __launch_bounds__(kBlock, hybrid_min_blocks(KIND)) k_push_hybrid(const double* __restrict__ src,
                                                                                 double* __restrict__ dst, int nx,
-                                                                                int ny, int ld, int ftiles,
+                                                                                int ny, int ld, Rows rows,
                                                                                 HybridArgs a) {
   chain_begin();
-  const int y = blockIdx.x / ftiles;
-  const int x = (blockIdx.x - y * ftiles) * blockDim.x + threadIdx.x;
-  if (x >= nx) return;
+  int x, y;
+  flat_cell(rows, y, x);
+  if (y >= ny) return;
   const I L = (I)ld, P = (I)ld * (I)ny;
   const I o = (I)y * L + (I)x;
   double f[9];
@@ -429,21 +429,20 @@ constexpr long long kQuickCells = 1 << 14;
 
 template <int KIND>
 cudaError_t launch_hybrid(const Sweep& s, const HybridArgs& a) {
-  const long long cells = (long long)s.nx * s.ny;
-  const int bs = block_for(cells, true);
-  const int ft = (s.ny + bs - 1) / bs;
-  const long long blocks = (long long)ft * s.nx;
-  if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-  const unsigned nb = (unsigned)blocks;
-  const double* src = static_cast<const double*>(s.src);
-  double* dst = static_cast<double*>(s.dst);
   if ((unsigned long long)s.ld * (unsigned long long)s.nx * 9ull >= (1ull << 32))
-    chained(k_step_hybrid<size_t, KIND, false>, nb, bs, s.stream)(src, dst, s.nx, s.ny, s.ld, ft, a);
-  else if (cells > kQuickCells)
-    chained(k_step_hybrid<uint32_t, KIND, false>, nb, bs, s.stream)(src, dst, s.nx, s.ny, s.ld, ft, a);
-  else
-    chained(k_step_hybrid<uint32_t, KIND, true>, nb, bs, s.stream)(src, dst, s.nx, s.ny, s.ld, ft, a);
-  return cudaGetLastError();
+    return step_cells<k_step_hybrid<size_t, KIND, false>>(s, s.ny, s.nx, true, true, a);
+  if ((long long)s.nx * s.ny > kQuickCells)
+    return step_cells<k_step_hybrid<uint32_t, KIND, false>>(s, s.ny, s.nx, true, true, a);
+  // rows that fill their blocks: the same cells, 0.1 us (of 2) sooner
+  const bool flat = s.ny % block_for((long long)s.nx * s.ny, true) != 0;
+  return step_cells<k_step_hybrid<uint32_t, KIND, true>>(s, s.ny, s.nx, true, flat, a);
+}
+
+template <int KIND>
+cudaError_t launch_push(const Sweep& s, const HybridArgs& a) {
+  if ((unsigned long long)s.ld * (unsigned long long)s.ny * 9ull < (1ull << 32))
+    return step_cells<k_push_hybrid<uint32_t, KIND>>(s, s.nx, s.ny, true, true, a);
+  return step_cells<k_push_hybrid<size_t, KIND>>(s, s.nx, s.ny, true, true, a);
 }
 
 }  // namespace
@@ -483,28 +482,8 @@ cudaError_t step_pull_fixed(int kind, const Sweep& s, const CollParams& cp, bool
 
 cudaError_t step_push_fixed(int kind, const Sweep& s, const CollParams& cp, bool report) {
   if (kind != K_BGK && kind != K_TRT && kind != K_RR) return cudaErrorNotSupported;
-  const int bs = block_for((long long)s.nx * s.ny, true);
-  const int ft = (s.nx + bs - 1) / bs;
-  const long long blocks = (long long)ft * s.ny;
-  if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   const HybridArgs a = hybrid_args(cp, report);
-  const double* src = static_cast<const double*>(s.src);
-  double* dst = static_cast<double*>(s.dst);
-  const unsigned nb = (unsigned)blocks;
-  const bool small = (unsigned long long)s.ld * (unsigned long long)s.ny * 9ull < (1ull << 32);
-#define PLBM_PUSH_HY(I)                                                                                      \
-  switch (kind) {                                                                                            \
-    case K_BGK: chained(k_push_hybrid<I, K_BGK>, nb, bs, s.stream)(src, dst, s.nx, s.ny, s.ld, ft, a); break; \
-    case K_TRT: chained(k_push_hybrid<I, K_TRT>, nb, bs, s.stream)(src, dst, s.nx, s.ny, s.ld, ft, a); break; \
-    default: chained(k_push_hybrid<I, K_RR>, nb, bs, s.stream)(src, dst, s.nx, s.ny, s.ld, ft, a); break;     \
-  }
-  if (small) {
-    PLBM_PUSH_HY(uint32_t)
-  } else {
-    PLBM_PUSH_HY(size_t)
-  }
-#undef PLBM_PUSH_HY
-  return cudaGetLastError();
+  return kind == K_TRT ? launch_push<K_TRT>(s, a) : (kind == K_RR ? launch_push<K_RR>(s, a) : launch_push<K_BGK>(s, a));
 }
 
 namespace {
