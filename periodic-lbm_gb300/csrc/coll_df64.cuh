@@ -122,7 +122,60 @@ DF_HD float relax(float h, float d, float om_hi, float om_lo) {
   return t + c;
 }
 
-// The same operations on values of type V (one cell or a pair of cells).
+// The update of a pair (q, qbar = -q): heq = a +- b with a = w (drho + rho nl_q)
+// (nl_q = 4.5 (c_q.u)^2 - 1.5 u^2) and b = 3 w c_q.j.  With the pair's exact
+// sum S = h_q + h_qbar and difference D = h_q - h_qbar (the error-free sums
+// the moments are built from),
+//   heq_q - h_q = (a - S/2) + (b - D/2),  heq_qbar - h_qbar = (a - S/2) - (b - D/2):
+// a - S/2 and b - D/2 are the symmetric and antisymmetric non-equilibrium
+// parts, small against a and b, so their high parts subtract exactly (the
+// operands are within a factor two; the FMA with -1/2 forms S/2 exactly) and
+// their low parts add in binary32.  This replaces the double-float sums
+// a + b, a - b of the two equilibria and 12 binary32 operations per pair.
+DF_HD void bgk_dev_comp_one(float (&h)[9], const DevParams& p) {
+  // exact pairwise sums and differences of the stored values
+  const df64 s13 = two_sum(h[1], h[3]), s24 = two_sum(h[2], h[4]);
+  const df64 s57 = two_sum(h[5], h[7]), s68 = two_sum(h[6], h[8]);
+  const df64 d13 = two_sum(h[1], -h[3]), d24 = two_sum(h[2], -h[4]);
+  const df64 d57 = two_sum(h[5], -h[7]), d86 = two_sum(h[8], -h[6]);
+  const df64 drho = add_lazy(add_lazy(add_lazy(s57, s68), add_lazy(s13, s24)), make(h[0], 0.0f));
+  const df64 jx = add_lazy(add_lazy(d57, d86), d13);
+  const df64 jy = add_lazy(add_lazy(d57, neg(d86)), d24);
+  // nonlinear part in binary32: u = j / (1 + drho)
+  const float dr = drho.hi + drho.lo;
+  const float inv = 1.0f / (1.0f + dr);
+  const float jxf = jx.hi + jx.lo, jyf = jy.hi + jy.lo;
+  const float ux = jxf * inv, uy = jyf * inv;
+  const float rho = 1.0f + dr;
+  const float u2 = 1.5f * (ux * ux + uy * uy);
+  // h' = h + omega (heq - h), heq = w (drho + rho (4.5 (c.u)^2 - 1.5 u^2)) + 3 w c.j.
+  // The equilibrium's O(h) part is formed in double-float, the nonlinear term
+  // (binary32) joining the exact drho before the product with w (binary32
+  // weights in that product biased the relaxation rate by ~1e-8); heq - h is a
+  // small difference of nearby values and takes binary32; relax() adds
+  // omega (heq - h) with one rounding, to the storage format.
+  {
+    const df64 e = mul_lazy(p.w[0], add_lazy(drho, make(rho * -u2, 0.0f)));
+    h[0] = relax(h[0], (e.hi - h[0]) + e.lo, p.om_hi, p.om_lo);
+  }
+#define PLBM_COMP_ONE(QP, QM, CUF, CJ, S, D, WI)                                                       \
+  {                                                                                                    \
+    const float cu = (CUF);                                                                            \
+    const df64 a = mul_lazy(p.w[WI], add_lazy(drho, make(rho * fmaf_(4.5f * cu, cu, -u2), 0.0f)));    \
+    const df64 b = mul_lazy(p.w3[WI], CJ);                                                             \
+    const float sym = fmaf_(-0.5f, S.hi, a.hi) + fmaf_(-0.5f, S.lo, a.lo);                             \
+    const float asym = fmaf_(-0.5f, D.hi, b.hi) + fmaf_(-0.5f, D.lo, b.lo);                            \
+    h[QP] = relax(h[QP], sym + asym, p.om_hi, p.om_lo);                                                \
+    h[QM] = relax(h[QM], sym - asym, p.om_hi, p.om_lo);                                                \
+  }
+  PLBM_COMP_ONE(1, 3, ux, jx, s13, d13, 1)
+  PLBM_COMP_ONE(2, 4, uy, jy, s24, d24, 1)
+  PLBM_COMP_ONE(5, 7, ux + uy, add_lazy(jx, jy), s57, d57, 2)
+  PLBM_COMP_ONE(8, 6, ux - uy, add_lazy(jx, neg(jy)), s68, d86, 2)
+#undef PLBM_COMP_ONE
+}
+
+// The same in fewer operations, on values of type V (one cell or a pair of cells).
 template <typename V>
 struct dfv {
   V hi, lo;
@@ -170,8 +223,7 @@ DF_HD V relax_v(V h, V d, V om_hi, V om_lo) {
   return vadd(t, vfma(om_lo, d, vfma(om_hi, d, vsub(h, t))));
 }
 
-// The update of a pair (q, qbar = -q): heq = a +- b with a = w (drho + nl_q)
-// (nl_q = 4.5 (c_q.j)(c_q.u) - 1.5 j.u) and b = 3 w c_q.j.  With the pair's exact
+// As bgk_dev_comp_one, with nl_q = 4.5 (c_q.j)(c_q.u) - 1.5 j.u for rho nl_q.  With the pair's exact
 // sum S = h_q + h_qbar and difference D = h_q - h_qbar (the error-free sums
 // the moments are built from),
 //   heq_q - h_q = (a - S/2) + (b - D/2),  heq_qbar - h_qbar = (a - S/2) - (b - D/2):

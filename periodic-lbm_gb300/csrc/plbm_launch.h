@@ -126,6 +126,10 @@ int resident_threads() {
   return n;
 }
 
+// Deviation-storage BGK: the packed operations (bgk_dev, bgk_dev_comp) on grids of at least
+// 2^20 cells, the smallest that a pass of several steps is taken on, in single steps too.
+inline bool packed_bgk(int nx, int ny) { return (long long)nx * ny >= 1 << 20; }
+
 // Deviation storage takes flat cells but on grids larger than the L2 cache whose rows fit
 // their blocks and not their 128-byte lines: warps that straddle lines cost there
 // (binary32 RR 3001 x 2999 97.8 us per step in rows, 102.2 flat; 1000^2 10.6 and 10.0).

@@ -32,6 +32,35 @@ __global__ void __launch_bounds__(kBlock) k_step_dev_df(const typename S::elem* 
   for (int q = 0; q < 9; q++) S::store(dst, YFast::off(x, y, q, nx, ny, ld), h[q].hi + h[q].lo);
 }
 
+// Deviation storage, BGK with the compensated binary32 operator on grids below
+// packed_bgk's line, a cell per thread.
+template <class S, typename I>
+__global__ void __launch_bounds__(kBlock) k_step_dev_comp_one(const typename S::elem* __restrict__ src,
+                                                             typename S::elem* __restrict__ dst, int nx, int ny,
+                                                             int ld, Rows rows, df::DevParams p) {
+  chain_begin();
+  int x, y;
+  flat_cell(rows, x, y);
+  if (x >= nx) return;
+  const I L = (I)ld, P = (I)ld * (I)nx;
+  const I c0 = (I)x * L, cm = (I)wrap_m(x, nx) * L, cp = (I)wrap_p(x, nx) * L;
+  const I y0 = (I)y, ym = (I)wrap_m(y, ny), yp = (I)wrap_p(y, ny);
+  float h[9];
+  h[0] = S::load(src, c0 + y0);
+  h[1] = S::load(src, P + cm + y0);
+  h[2] = S::load(src, 2 * P + c0 + ym);
+  h[3] = S::load(src, 3 * P + cp + y0);
+  h[4] = S::load(src, 4 * P + c0 + yp);
+  h[5] = S::load(src, 5 * P + cm + ym);
+  h[6] = S::load(src, 6 * P + cp + ym);
+  h[7] = S::load(src, 7 * P + cp + yp);
+  h[8] = S::load(src, 8 * P + cm + yp);
+  df::bgk_dev_comp_one(h, p);
+  const I o = c0 + y0;
+#pragma unroll
+  for (int q = 0; q < 9; q++) S::store(dst, (I)q * P + o, h[q]);
+}
+
 // Deviation storage, BGK with the compensated binary32 operator, two cells of
 // adjacent columns per thread in packed binary32 registers: the operator's 350
 // operations per cell bound the one-cell kernel by issue (437 instructions per
@@ -106,9 +135,19 @@ cudaError_t step_pull_dev_hi(int storage, int math, int kind, const Sweep& s, co
   if (math == 2) {  // compensated binary32
     if (kind != K_BGK) return cudaErrorNotSupported;
     const df::DevParams p = df::dev_params(cp.omega);
+    const bool small = (unsigned long long)s.ld * (unsigned long long)s.nx * 9ull < (1ull << 32);
+    if (!packed_bgk(s.nx, s.ny)) {
+      // fewer than 2^32 elements unless the rows are mostly padding
+      if (storage == ST_F32DEV)
+        return small ? step_cells<k_step_dev_comp_one<StoreF32Dev, uint32_t>>(s, s.ny, s.nx, false, true, p)
+                     : step_cells<k_step_dev_comp_one<StoreF32Dev, size_t>>(s, s.ny, s.nx, false, true, p);
+      if (storage == ST_F16DEV)
+        return small ? step_cells<k_step_dev_comp_one<StoreF16Dev, uint32_t>>(s, s.ny, s.nx, false, true, p)
+                     : step_cells<k_step_dev_comp_one<StoreF16Dev, size_t>>(s, s.ny, s.nx, false, true, p);
+      return cudaErrorInvalidValue;
+    }
     const int pairs = s.nx / 2 + (s.nx & 1);
     const bool flat = dev_flat(s.ny, pairs);
-    const bool small = (unsigned long long)s.ld * (unsigned long long)s.nx * 9ull < (1ull << 32);
     if (storage == ST_F32DEV)
       return small ? step_cells<k_step_dev_comp<StoreF32Dev, uint32_t>>(s, s.ny, pairs, false, flat, p)
                    : step_cells<k_step_dev_comp<StoreF32Dev, size_t>>(s, s.ny, pairs, false, flat, p);
