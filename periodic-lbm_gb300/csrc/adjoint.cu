@@ -250,12 +250,13 @@ template <int ST, typename I>
 __global__ void __launch_bounds__(kBlock) k_adj_step(const void* __restrict__ f, const void* __restrict__ lam_in,
                                                     void* __restrict__ lam_out, double* __restrict__ dom,
                                                     typename AdjTraits<ST>::real om, int nx, int ny, int ld,
-                                                    int ftiles) {
+                                                    Rows rows) {
   chain_begin();
   typedef typename AdjTraits<ST>::real R;
   typedef typename AdjTraits<ST>::elem E;
   int x, y;
-  const bool in = yfast_cell(ftiles, ny, x, y);
+  flat_cell(rows, x, y);
+  const bool in = x < nx;
   R part = R(0);
   if (in) {
     const E* fe = static_cast<const E*>(f);
@@ -277,7 +278,7 @@ __global__ void __launch_bounds__(kBlock) k_adj_step(const void* __restrict__ f,
     for (int p = 0; p < 9; p++) lo[off[p]] = (E)mu[p];
   }
   const double t = warp_sum((double)part);
-  if ((threadIdx.x & 31) == 0) dom[(size_t)blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5)] += t;
+  if ((threadIdx.x & 31) == 0) dom[(size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)] += t;
 }
 
 // The reverse step in compensated binary32 (binary32 storage; df::adj_step_comp
@@ -288,10 +289,11 @@ template <typename I>
 __global__ void __launch_bounds__(kBlock, 4) k_adj_step_comp(const float* __restrict__ fe, const float* __restrict__ li,
                                                          float* __restrict__ lo, double* __restrict__ dom,
                                                          df::AdjDevParams cpar, int nx, int ny, int ld,
-                                                         int ftiles) {
+                                                         Rows rows) {
   chain_begin();
   int x, y;
-  const bool in = yfast_cell(ftiles, ny, x, y);
+  flat_cell(rows, x, y);
+  const bool in = x < nx;
   float part = 0.0f;
   if (in) {
     const I L = (I)ld, P = (I)ld * (I)nx;
@@ -310,7 +312,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_adj_step_comp(const float* __rest
     for (int q = 0; q < 9; q++) lo[off[q]] = mu[q];
   }
   const double t = warp_sum((double)part);
-  if ((threadIdx.x & 31) == 0) dom[(size_t)blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5)] += t;
+  if ((threadIdx.x & 31) == 0) dom[(size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)] += t;
 }
 
 // dL/du0 from lambda_0 and u0.
@@ -337,8 +339,30 @@ __global__ void __launch_bounds__(kBlock) k_adj_u0(const void* __restrict__ lam,
 
 inline int tiles(int n) { return (n + kBlock - 1) / kBlock; }
 
+// The reverse step's threads: rows of 256 where those fit, flat cells otherwise (64
+// threads: ragged rows of 300^2 19.9 -> 14.9 us per step with its recomputation, 257^2
+// 18.6 -> 12.5; 256^2 16.0 in rows and 16.2 flat).  No limit on an SM's CTAs: it would
+// keep the recomputation, on another stream, off the SMs (256^2: 18.1).
+cudaError_t reverse_spread(int nx, int ny, Spread* w) {
+  const long long tl = tiles(ny), blocks = tl * nx;
+  if (32 * (tl * kBlock - ny) > ny) return spread_cells(ny, nx, true, true, 0, w);
+  if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+  *w = Spread{(unsigned)blocks, kBlock, 0, Rows{(unsigned)ny, 0, (unsigned)tl}};
+  return cudaSuccess;
+}
+
+// Kernel K(f, lam_in, lam_out, dom, p, nx, ny, ld, rows).
+template <auto K, typename P>
+cudaError_t reverse_step(const AdjLaunch& a, const P& p) {
+  Spread w;
+  if (cudaError_t e = reverse_spread(a.nx, a.ny, &w)) return e;
+  chained(K, w, a.stream)(a.f, a.lam_in, a.lam_out, a.dom, p, a.nx, a.ny, a.ld, w.rows);
+  return cudaGetLastError();
+}
+
 template <int ST>
 cudaError_t dispatch(int what, const AdjLaunch& a) {
+  const bool small = (unsigned long long)a.ld * (unsigned long long)a.nx * 9ull < (1ull << 32);
   const int ft = tiles(a.ny);
   const long long blocks = (long long)ft * a.nx;
   if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
@@ -357,24 +381,11 @@ cudaError_t dispatch(int what, const AdjLaunch& a) {
         }
         cpar.om_hi = (float)a.omega;
         cpar.om_lo = (float)(a.omega - (double)cpar.om_hi);
-        const float* fa = static_cast<const float*>(a.f);
-        const float* la = static_cast<const float*>(a.lam_in);
-        float* lb = static_cast<float*>(a.lam_out);
-        if ((unsigned long long)a.ld * (unsigned long long)a.nx * 9ull < (1ull << 32))
-          chained(k_adj_step_comp<uint32_t>, nb, kBlock, a.stream)(fa, la, lb, a.dom, cpar, a.nx, a.ny, a.ld, ft);
-        else
-          chained(k_adj_step_comp<size_t>, nb, kBlock, a.stream)(fa, la, lb, a.dom, cpar, a.nx, a.ny, a.ld, ft);
-        break;
+        if (small) return reverse_step<k_adj_step_comp<uint32_t>>(a, cpar);
+        return reverse_step<k_adj_step_comp<size_t>>(a, cpar);
       }
-      if ((unsigned long long)a.ld * (unsigned long long)a.nx * 9ull < (1ull << 32))
-        chained(k_adj_step<ST, uint32_t>, nb, kBlock, a.stream)(a.f, a.lam_in, a.lam_out, a.dom,
-                                                              (typename AdjTraits<ST>::real)a.omega, a.nx, a.ny,
-                                                              a.ld, ft);
-      else
-        chained(k_adj_step<ST, size_t>, nb, kBlock, a.stream)(a.f, a.lam_in, a.lam_out, a.dom,
-                                                            (typename AdjTraits<ST>::real)a.omega, a.nx, a.ny, a.ld,
-                                                            ft);
-      break;
+      if (small) return reverse_step<k_adj_step<ST, uint32_t>>(a, (typename AdjTraits<ST>::real)a.omega);
+      return reverse_step<k_adj_step<ST, size_t>>(a, (typename AdjTraits<ST>::real)a.omega);
     case 3: k_adj_u0<ST><<<nb, kBlock, 0, a.stream>>>(a.lam_in, a.u, a.out, a.nx, a.ny, a.ld, ft); break;
     default: return cudaErrorInvalidValue;
   }
@@ -383,7 +394,11 @@ cudaError_t dispatch(int what, const AdjLaunch& a) {
 
 }  // namespace
 
-int adjoint_blocks(int nx, int ny) { return tiles(ny) * nx * (kBlock / 32); }
+// The reverse step's warps: one dL/domega slot each.
+int adjoint_blocks(int nx, int ny) {
+  Spread w;
+  return reverse_spread(nx, ny, &w) == cudaSuccess ? (int)(w.blocks * (unsigned)(w.threads / 32)) : 0;
+}
 
 cudaError_t adjoint_launch(int storage, int what, const AdjLaunch& a) {
   if (storage == ST_F64) return dispatch<ST_F64>(what, a);

@@ -39,40 +39,45 @@ int sm_count() {
 }
 }  // namespace
 
-int plbm::block_for(long long cells, bool binary64) {
+namespace {
+int block_of(long long cells, bool binary64, int sms) {
   const int most = binary64 ? (cells <= (1 << 18) ? 64 : 128)
                             : (cells <= (1 << 17) ? 64 : (cells < (1 << 18) ? 128 : kBlock));
-  const int n = sm_count();
-  if (n < 1) return most;
-  const long long per_sm = (cells + n - 1) / n;
-  if (per_sm >= most) return most;
-  return (int)(per_sm < 32 ? 32 : (per_sm + 31) / 32 * 32);
+  if (sms < 1 || cells > (long long)most * (sms - 1)) return most;
+  const int per_sm = ((int)cells + sms - 1) / sms;
+  return per_sm < 32 ? 32 : (per_sm + 31) / 32 * 32;
 }
+}  // namespace
+
+int plbm::block_for(long long cells, bool binary64) { return block_of(cells, binary64, sm_count()); }
 
 bool plbm::rows_fit(int nfast, int nslow, bool binary64) {
-  const long long bs = block_for((long long)nfast * nslow, binary64);
-  return 32 * ((nfast + bs - 1) / bs * bs - nfast) <= nfast;
+  const int bs = block_for((long long)nfast * nslow, binary64);
+  return 32LL * ((nfast + bs - 1) / bs * bs - nfast) <= nfast;
 }
 
 cudaError_t plbm::spread_cells(int nfast, int nslow, bool binary64, bool flat, int resident, Spread* w) {
   const long long cells = (long long)nfast * nslow;
   if (cells <= 0) return cudaErrorInvalidConfiguration;
-  w->threads = block_for(cells, binary64);
+  const int sms = sm_count();
+  w->threads = block_of(cells, binary64, sms);
   w->smem = 0;
   w->rows = Rows{(unsigned)nfast, 0, 0};
-  const int per_row = (nfast + w->threads - 1) / w->threads;
-  long long blocks = (cells + w->threads - 1) / w->threads;
-  if (flat && blocks * w->threads < (1LL << 32))
+  long long blocks;
+  if (flat && cells < (1LL << 32) - w->threads) {
     w->rows.m = nfast == 1 ? 0xffffffffu : (unsigned)((1ull << 32) / (unsigned)nfast);
-  else
-    w->rows.tiles = (unsigned)per_row, blocks = (long long)nslow * per_row;
+    blocks = ((unsigned)cells + (unsigned)w->threads - 1) / (unsigned)w->threads;
+  } else {
+    w->rows.tiles = ((unsigned)nfast + (unsigned)w->threads - 1) / (unsigned)w->threads;
+    blocks = (long long)nslow * w->rows.tiles;
+  }
   if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   w->blocks = (unsigned)blocks;
-  const int n = sm_count();
-  if (n < 1) return cudaSuccess;
-  const long long per_sm = (blocks + n - 1) / n, fits = resident / w->threads;
+  // more than the 2,048 threads that an SM holds at most: no limit
+  if (sms < 1 || blocks * w->threads > 2048LL * sms) return cudaSuccess;
+  const int per_sm = ((int)blocks + sms - 1) / sms, fits = resident / w->threads;
   // an SM's 228 KB, of which each CTA takes 1 KB for itself; more than 48 KB need leave
-  if (per_sm <= fits && 2 * per_sm > fits && per_sm >= 5) w->smem = (int)(((228 << 10) / per_sm - 1024) / 128 * 128);
+  if (per_sm <= fits && 2 * per_sm > fits && per_sm >= 5) w->smem = ((228 << 10) / per_sm - 1024) / 128 * 128;
   return cudaSuccess;
 }
 

@@ -56,7 +56,7 @@ struct Spread {
   Rows rows;
 };
 // flat: rows cut into blocks of their own otherwise, and with 2^32 cells or more.
-// resident: threads of the kernel that an SM's registers hold.
+// resident: threads of the kernel that an SM's registers hold; 0: no limit.
 cudaError_t spread_cells(int nfast, int nslow, bool binary64, bool flat, int resident, Spread* out);
 // Whether rows cut into blocks of their own leave at most 1/32 of the threads without a
 // cell.

@@ -67,3 +67,24 @@ def test_plugin_rolled(gpu_lib, kind, storage, math, nx, ny):
         out.append([np.array(v) for v in sim.vars()])
     for a, b in zip(*out):
         assert np.array_equal(np.roll(a, (nx // 2, ny // 3), axis=(0, 1)), b)
+
+
+@pytest.mark.parametrize("storage,math", [("f64", "fma"), ("f32dev", "fma"), ("f32dev", "hybrid")])
+@pytest.mark.parametrize("nx,ny,copies", [(3, 128, 2), (5, 85, 3), (2, 51, 5), (40, 150, 2)])
+def test_reverse_steps_of_copies(gpu_lib, storage, math, nx, ny, copies):
+    """The reverse step in rows (256, 255 rows) and over flat cells: the gradient of
+    copies is the copies of the gradient, dL/domega their sum (binary64 sums of equal
+    terms in another order: 1e-12 of the terms' size, at most 40 x 300 of them)."""
+    import torch
+    from plbm.autograd import Adjoint
+    rng = np.random.default_rng(nx + ny)
+    u, g = 0.03 * rng.standard_normal((2, nx, ny)), rng.standard_normal((2, nx, ny))
+    out = []
+    for k in (1, copies):
+        a = Adjoint(nx, ny * k, 4, checkpoint_every=2, storage=storage, math=math)
+        a.forward(torch.tensor(np.tile(u, (1, 1, k)), device="cuda"), 1.4)
+        gu, dom = a.backward(torch.tensor(np.tile(g, (1, 1, k)), device="cuda"))
+        out.append((gu.cpu().numpy(), dom / k))
+        a.close()
+    assert np.array_equal(np.tile(out[0][0], (1, 1, copies)), out[1][0])
+    assert abs(out[0][1] - out[1][1]) <= 1e-12 * nx * ny
