@@ -230,8 +230,8 @@ __global__ void __launch_bounds__(kBlock) k_step_scheme_hybrid(const double* __r
 // FDM), ISO and WLS, while a1 and a2 are below 2^(shift - 4) (time steps up to
 // about 1, the scheme's own stability limit); other schemes and steps keep the
 // stencil form.  512^2, central FDM, BGK, dt = 0.3: 68 us per step in the stencil
-// form with the binary64 collision, 33 us with the fixed-point collision, 20.5 us
-// here (12.7 GLUPS; 2048^2 17.0 against 4.2 and 8.0); error against binary64
+// form with the binary64 collision, 33 us with the fixed-point collision, 16.8 us
+// here (15.6 GLUPS; 2048^2 17.0 against 4.2 and 8.0); error against binary64
 // arithmetic of the reference's expressions 4.4e-16 (stencil form 2.1e-15).
 // Bound by issue: about 1,500 instructions per cell, the ALU pipe 67 % busy.
 enum { FORM_LINE = 0, FORM_CENTRAL = 1, FORM_ISO = 2, FORM_WLS = 3 };
@@ -523,14 +523,15 @@ bool scheme_fixed_constants(int scheme, int kind, double dt, double omega, int& 
   return true;
 }
 
-// Tile columns of k_step_scheme_fixed: two for grids whose wider tiles would not
+// Tile columns of k_step_scheme_fixed: four for grids whose wider tiles would not
 // give every SM a CTA, 16 (two cells per thread, the smaller halo) where every SM
-// gets several.  BGK, central FDM, MLUPS with 2 / 8 / 16 columns: 64^2 1,205 / 885 / 525,
-// 128^2 3,849 / 3,538 / 2,084, 256^2 7,966 / 9,788 / 8,206, 512^2 8,510 / 12,742 /
-// 11,587, 1024^2 - / 10,019 / 10,011 (an earlier form), 2048^2 9,895 / 16,486 / 17,019.
+// gets several.  BGK, central FDM, us per step with 2 / 4 / 8 / 16 columns: 64^2 3.2 / 3.3 /
+// 4.4 / -, 128^2 4.0 / 3.3 / 4.3 / -, 180^2 6.2 / 5.2 / 5.9 / -, 256^2 - / 6.4 / 6.1 / 7.7,
+// 512^2 - / 18.5 / 16.9 / 19.6, 1000^2 - / 70.8 / 64.3 / 66.5; 6, 10, 12 and 14 columns lie
+// between or above, and so do 3 and 5 CTAs per SM.
 int scheme_tile(const Sweep& s) {
   const long long cells = (long long)s.nx * s.ny;
-  return cells > (1 << 20) ? 16 : (cells > 40000 ? 8 : 2);
+  return cells > (1 << 20) ? 16 : (cells > 40000 ? 8 : 4);
 }
 
 template <int FORM, int TX>
@@ -560,7 +561,7 @@ cudaError_t step_scheme_fixed(int scheme, int kind, const Sweep& s, double dt, c
 #define PLBM_SCH_FX(F)                                             \
   if (tx == 16) launch_scheme_fixed<F, 16>(kind, s, c, st, a);     \
   else if (tx == 8) launch_scheme_fixed<F, 8>(kind, s, c, st, a);  \
-  else launch_scheme_fixed<F, 2>(kind, s, c, st, a)
+  else launch_scheme_fixed<F, 4>(kind, s, c, st, a)
     switch (form) {
       case FORM_LINE: PLBM_SCH_FX(FORM_LINE); break;
       case FORM_CENTRAL: PLBM_SCH_FX(FORM_CENTRAL); break;

@@ -1,5 +1,5 @@
 """The finite-difference schemes' fixed-point kernel (k_step_scheme_fixed) at the
-edges of its tiles (32 rows by 2, 8 or 16 columns), its range and its rule."""
+edges of its tiles (32 rows by 4, 8 or 16 columns), its range and its rule."""
 import numpy as np
 import pytest
 
