@@ -8,7 +8,8 @@ N(0, 1e-4^2) velocity noise, f at equilibrium.  A step is one
 perform_lbm_step (one fused pull-stream + collide kernel) over the grid.
 The headline arithmetic is PLBM_MATH_HYBRID (binary64 storage, one binary64
 FMA per population on an exact integer bracket, exact integer moments); the
-straight binary64 kernel is measured beside it ("variants.fp64_native").
+same workload in PLBM_MATH_FMA, the library's default, is measured beside it
+("variants.fp64_native").
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
                     [--n 8192] [--kind bgk|trt|rr] [--storage f64|f32dev|f16dev]
@@ -52,9 +53,10 @@ import numpy as np  # noqa: E402
 BYTES_PER_CELL = {"f64": 144, "f32dev": 72, "f16dev": 36}
 # DRAM bytes per cell update measured by ncu (dram__bytes_read.sum +
 # dram__bytes_write.sum of one launch / cells) on a 2048^2 capture of the same
-# kernel, scaled by the cell count: profiles/k_step_*_2048_fullset.md.
-NCU_TRAFFIC_PER_CELL = {("f64", "bgk", "hybrid"): 132.6, ("f64", "trt", "hybrid"): 132.4,
-                        ("f64", "rr", "hybrid"): 133.0, ("f64", "bgk", "fma"): 132.4}
+# kernel, scaled by the cell count: profiles/step_kernels_pipes.md (BGK),
+# profiles/k_step_*_2048_fullset.md.
+NCU_TRAFFIC_PER_CELL = {("f64", "bgk", "hybrid"): 131.4, ("f64", "trt", "hybrid"): 132.4,
+                        ("f64", "rr", "hybrid"): 133.0, ("f64", "bgk", "fma"): 131.4}
 FALLBACK_HBM_GBS = 6800.0
 
 

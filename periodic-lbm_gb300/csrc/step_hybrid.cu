@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(kBlock) k_step_scheme_hybrid(const double* __r
 // form with the binary64 collision, 33 us with the fixed-point collision, 16.8 us
 // here (15.6 GLUPS; 2048^2 17.0 against 4.2 and 8.0); error against binary64
 // arithmetic of the reference's expressions 4.4e-16 (stencil form 2.1e-15).
-// Bound by issue: about 1,500 instructions per cell, the ALU pipe 67 % busy.
+// Bound by the integer pipe: about 1,450 instructions per cell, the ALU pipe 70 % busy.
 enum { FORM_LINE = 0, FORM_CENTRAL = 1, FORM_ISO = 2, FORM_WLS = 3 };
 // Left shift of D1, D2 before the product: the largest for which |D| 2^shift stays
 // below 2^63 for axis populations below 1/4 and diagonal ones below 1/8.
