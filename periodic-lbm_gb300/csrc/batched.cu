@@ -194,6 +194,14 @@ constexpr int batch_min_blocks(int max_threads) {
   return (S::ddf ? 1536 : 1024) / max_threads;
 }
 
+// The persistent binary64 kernel at 256 threads: three CTAs (80 registers, no spill) hide
+// the copies as well as four (64, 84 bytes spilled), and fewer meet at the barrier: 512
+// grids 1.117 -> 1.091 ms per step, 8 grids 17.6 -> 16.6 us; two CTAs 1.162 and 15.3.
+template <class S>
+constexpr int persistent_min_blocks(int max_threads) {
+  return !S::ddf && max_threads == 256 ? 3 : batch_min_blocks<S>(max_threads);
+}
+
 // A binary64 tile as the persistent kernel keeps it in shared memory: the tile, its
 // grid's sizes and the relaxation constants (a CTA has the same tiles in every step;
 // read from global memory for each tile, they put three dependent L2 latencies
@@ -288,13 +296,13 @@ __device__ __forceinline__ void sweep_ahead(const BatchGrid* __restrict__ grids,
 //
 // 48 grids of 32 to 512 cells a side, 1.42 M cells, us per step: tiles of ty by
 // threads / ty cells with loads for each 70; tiles of consecutive cells, columns copied
-// ahead 62; the tiles' table and constants in shared memory 53.  About a quarter
+// ahead 62; the tiles' table and constants in shared memory 53; three CTAs per SM 49.  A quarter
 // of it is the barrier and the memory's latency after it.  Waiting for chunks of
 // whole grids instead (each of which depends on itself alone) lost more to every
 // further release and acquire, 4 us each, than it gained: 2 chunks 53, 4 chunks 61.
-// 512 grids, 39 M cells: 1.94 -> 1.12 ms per step.
+// 512 grids, 39 M cells: 1.94 -> 1.09 ms per step.
 template <class S, typename I, int MAXT>
-__global__ void __launch_bounds__(MAXT, batch_min_blocks<S>(MAXT))
+__global__ void __launch_bounds__(MAXT, persistent_min_blocks<S>(MAXT))
     k_batch_persistent(const BatchGrid* __restrict__ grids, const BatchTile* __restrict__ tiles, int nt_bgk, int ntiles,
                        int nsteps, int parity0, typename S::elem* base, Ctrl* ctrl) {
   // own tiles below tile t
