@@ -46,6 +46,11 @@ __device__ __forceinline__ f32x2 vfma(f32x2 a, f32x2 b, f32x2 c) {
 }
 template <>
 DF_HD f32x2 vset<f32x2>(float c) { return pack2(c, c); }
+// a b, not to be contracted into a sum that follows: ptxas fuses a packed product and
+// sum, .rn or not; a fused product and sum of its own is left alone (+ -0 changes no
+// product, not even the sign of a zero).
+__device__ __forceinline__ float vprod(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ f32x2 vprod(f32x2 a, f32x2 b) { return vfma(a, b, vset<f32x2>(-0.0f)); }
 __device__ __forceinline__ f32x2 rcp_seed(f32x2 x) { return pack2(rcp_seed(lo2(x)), rcp_seed(hi2(x))); }
 
 // a / x with r = vrcp(x): the product and its exact residual added back
@@ -63,9 +68,7 @@ __device__ __forceinline__ V vquot(V a, V x, V r) {
 // the even part of a pair (q, -q) once, the odd part added and subtracted; 66
 // operations.  The O(h) terms come from dr and j themselves, not from rho - 1 and
 // rho u, which lose dr's low bits to the rounding of rho = 1 + dr.
-// SC: populations held scaled by S = 2^15 (binary16 storage): dr, j and heq scale
-// with them, rho = 1 + dr / S and u = (j / S) / rho.
-template <typename V, bool SC>
+template <typename V>
 __device__ __forceinline__ void bgk_dev(V (&h)[9], float omega) {
   // the three binary32 weights share one relative error, 7e-9, with which mass and
   // momentum drift; 3 w c.j with a rounded 3 w would drift four times as fast
@@ -74,19 +77,9 @@ __device__ __forceinline__ void bgk_dev(V (&h)[9], float omega) {
   const V d13 = vsub(h[1], h[3]), d24 = vsub(h[2], h[4]), d57 = vsub(h[5], h[7]), d86 = vsub(h[8], h[6]);
   const V dr = vadd(vadd(vadd(s57, s68), vadd(s13, s24)), h[0]);
   const V jx = vadd(vadd(d57, d86), d13), jy = vadd(vsub(d57, d86), d24);
-  V rho, ux, uy;
-  if constexpr (SC) {
-    const V is = vset<V>(1.0f / 32768.0f);
-    rho = vfma(dr, is, vset<V>(1.0f));
-    const V r = vrcp(rho);
-    ux = vquot(vmul(jx, is), rho, r);
-    uy = vquot(vmul(jy, is), rho, r);
-  } else {
-    rho = vadd(dr, vset<V>(1.0f));
-    const V r = vrcp(rho);
-    ux = vquot(jx, rho, r);
-    uy = vquot(jy, rho, r);
-  }
+  const V rho = vadd(dr, vset<V>(1.0f));
+  const V r = vrcp(rho);
+  const V ux = vquot(jx, rho, r), uy = vquot(jy, rho, r);
   const V base = vfma(vset<V>(-1.5f), vfma(jy, uy, vmul(jx, ux)), dr);
   // h' = h - omega (h - w heq'), all fused: no plain product feeds a sum or a
   // difference (ptxas contracts a packed product and difference, .rn or not).
@@ -102,6 +95,45 @@ __device__ __forceinline__ void bgk_dev(V (&h)[9], float omega) {
   pair(2, 4, uy, jy, ws);
   pair(5, 7, vadd(ux, uy), vadd(jx, jy), wd);
   pair(8, 6, vsub(ux, uy), vsub(jx, jy), wd);
+}
+
+// BGK on binary16 deviations kept in their stored scale, H = 2^15 h: the scale
+// enters the constants instead of 18 multiplies per cell.  rho = 1 + 2^-15 sum H,
+// u = j / rho, and H' = (1 - omega) H + omega Heq with Heq = w (sum H + 2^15 rho P),
+// P = -1.5 u^2 + 3 c.u + 4.5 (c.u)^2 -- the shifted equilibrium of coll_bgk_shift,
+// scaled, with omega w folded into the two per-cell factors; 64 operations and the
+// division.  u takes the approximate division (2 ulp): binary16 storage rounds the
+// populations to 2^-11 relative, far above it.  Each operation rounds on its own, so
+// that one cell per thread, two per thread and a pass of several steps give the same
+// bits: an operator that rounds otherwise lands on another binary16 value now and
+// then, 2^-11 of h apart.
+__device__ __forceinline__ float f16_inv_rho(float rho) { return __fdividef(1.0f / 32768.0f, rho); }
+__device__ __forceinline__ f32x2 f16_inv_rho(f32x2 rho) { return pack2(f16_inv_rho(lo2(rho)), f16_inv_rho(hi2(rho))); }
+template <typename V>
+__device__ __forceinline__ void bgk_f16(V (&H)[9], float omega) {
+  const V s13 = vadd(H[1], H[3]), s24 = vadd(H[2], H[4]), s57 = vadd(H[5], H[7]), s68 = vadd(H[6], H[8]);
+  const V d13 = vsub(H[1], H[3]), d24 = vsub(H[2], H[4]), d57 = vsub(H[5], H[7]), d86 = vsub(H[8], H[6]);
+  const V dh = vadd(vadd(vadd(s57, s68), vadd(s13, s24)), H[0]);
+  const V rho = vfma(dh, vset<V>(1.0f / 32768.0f), vset<V>(1.0f));
+  const V r = f16_inv_rho(rho);
+  const V ux = vprod(vadd(vadd(d57, d86), d13), r), uy = vprod(vadd(vsub(d57, d86), d24), r);
+  const V uxx = vprod(ux, ux), uyy = vprod(uy, uy);
+  const V indp = vmul(vset<V>(-1.5f), vadd(uxx, uyy));
+  const V sr = vmul(vset<V>(32768.0f), rho), omb = vset<V>(vsub(1.0f, omega));
+  const V three = vset<V>(3.0f), mthree = vset<V>(-3.0f);
+  const V a0 = vset<V>(vmul(omega, 4.0f / 9.0f));
+  H[0] = vfma(omb, H[0], vfma(vmul(a0, sr), indp, vmul(a0, dh)));
+  auto pair = [&](int a, int b, V u, V even, V k1, V k0) {
+    H[a] = vfma(omb, H[a], vfma(k1, vfma(three, u, even), k0));
+    H[b] = vfma(omb, H[b], vfma(k1, vfma(mthree, u, even), k0));
+  };
+  const V as = vset<V>(vmul(omega, 1.0f / 9.0f)), k1s = vmul(as, sr), k0s = vmul(as, dh);
+  pair(1, 3, ux, vfma(vset<V>(4.5f), uxx, indp), k1s, k0s);
+  pair(2, 4, uy, vfma(vset<V>(4.5f), uyy, indp), k1s, k0s);
+  const V ad = vset<V>(vmul(omega, 1.0f / 36.0f)), k1d = vmul(ad, sr), k0d = vmul(ad, dh);
+  const V up = vadd(ux, uy), um = vsub(ux, uy);
+  pair(5, 7, up, vfma(vmul(vset<V>(4.5f), up), up, indp), k1d, k0d);
+  pair(8, 6, um, vfma(vmul(vset<V>(4.5f), um), um, indp), k1d, k0d);
 }
 
 }  // namespace plbm

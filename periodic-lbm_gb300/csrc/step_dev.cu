@@ -62,42 +62,8 @@ ShiftParamsF shift_params(int kind, const CollParams& p) {
   return {(float)p.omega, 0.0f, 0.0f};
 }
 
-// BGK on binary16 deviations kept in their stored scale, H = 2^15 h: the
-// scale enters the constants instead of 18 multiplies per cell.  rho = 1 +
-// 2^-15 sum H, u = j / rho, and H' = (1 - omega) H + omega Heq with Heq =
-// w (sum H + 2^15 rho P), P = -1.5 u^2 + 3 c.u + 4.5 (c.u)^2 -- the shifted
-// equilibrium of coll_bgk_shift, scaled, with omega w folded into the two
-// per-cell factors.  u takes the approximate division (2 ulp): binary16
-// storage rounds the populations to 2^-11 relative, far above it.
-__device__ __forceinline__ void coll_bgk_shift_f16scaled(float (&H)[9], float omega) {
-  const float dh = (((H[5] + H[7]) + (H[6] + H[8])) + ((H[1] + H[3]) + (H[2] + H[4]))) + H[0];
-  const float rho = fmaf(dh, F16_INV_SCALE, 1.0f);
-  const float r = __fdividef(F16_INV_SCALE, rho);
-  const float ux = (((H[5] - H[7]) + (H[8] - H[6])) + (H[1] - H[3])) * r;
-  const float uy = (((H[5] - H[7]) + (H[6] - H[8])) + (H[2] - H[4])) * r;
-  const float uxx = ux * ux, uyy = uy * uy;
-  const float indp = -1.5f * (uxx + uyy);
-  const float sr = F16_SCALE * rho, omb = 1.0f - omega;
-  const float a0 = omega * (4.0f / 9.0f), as = omega * (1.0f / 9.0f), ad = omega * (1.0f / 36.0f);
-  const float k00 = a0 * dh, k10 = a0 * sr, k0s = as * dh, k1s = as * sr, k0d = ad * dh, k1d = ad * sr;
-  H[0] = fmaf(omb, H[0], fmaf(k10, indp, k00));
-  const float bx = fmaf(4.5f, uxx, indp), by = fmaf(4.5f, uyy, indp);
-  H[1] = fmaf(omb, H[1], fmaf(k1s, fmaf(3.0f, ux, bx), k0s));
-  H[3] = fmaf(omb, H[3], fmaf(k1s, fmaf(-3.0f, ux, bx), k0s));
-  H[2] = fmaf(omb, H[2], fmaf(k1s, fmaf(3.0f, uy, by), k0s));
-  H[4] = fmaf(omb, H[4], fmaf(k1s, fmaf(-3.0f, uy, by), k0s));
-  const float uxpy = ux + uy, uxmy = ux - uy;
-  const float bp = fmaf(4.5f * uxpy, uxpy, indp), bm = fmaf(4.5f * uxmy, uxmy, indp);
-  H[5] = fmaf(omb, H[5], fmaf(k1d, fmaf(3.0f, uxpy, bp), k0d));
-  H[7] = fmaf(omb, H[7], fmaf(k1d, fmaf(-3.0f, uxpy, bp), k0d));
-  H[6] = fmaf(omb, H[6], fmaf(k1d, fmaf(-3.0f, uxmy, bm), k0d));
-  H[8] = fmaf(omb, H[8], fmaf(k1d, fmaf(3.0f, uxmy, bm), k0d));
-}
-
-// BGK in the operations of bgk_dev (f32x2.cuh), which the marched passes of large
-// grids take: a kind of these kernels beside the operator's own.  Grids below
-// kPackedCells keep coll_bgk_shift and its scaled form to the last bit (their moments
-// are read in binary64); their steps wait for launches and memory, not for arithmetic.
+// binary32 BGK in the operations of bgk_dev (f32x2.cuh), which the marched passes of
+// large grids take: a kind of these kernels beside the operator's own (packed_bgk).
 constexpr int kBgkPacked = 100;
 
 // The pull step of the src/ layout (YFast) with explicit pull offsets: I is
@@ -127,8 +93,7 @@ __global__ void __launch_bounds__(kBlock) k_step_dev_pull(const typename S::elem
     for (int q = 0; q < 9; q++) H[q] = __half2float(ld_chain(src + offs[q]));
     if constexpr (KIND == K_TRT) coll_trt_shift<float, true>(H, p.a, p.b, p.c);
     else if constexpr (KIND == K_RR) coll_rr_shift<float, true>(H, p.a, p.b, p.c);
-    else if constexpr (KIND == K_BGK) coll_bgk_shift_f16scaled(H, p.a);
-    else bgk_dev<float, true>(H, p.a);
+    else bgk_f16(H, p.a);
 #pragma unroll
     for (int q = 0; q < 9; q++) dst[(I)q * P + o] = __float2half_rn(H[q]);
     return;
@@ -139,7 +104,7 @@ __global__ void __launch_bounds__(kBlock) k_step_dev_pull(const typename S::elem
   if (KIND == K_TRT) coll_trt_shift<float>(h, p.a, p.b, p.c);
   else if (KIND == K_RR) coll_rr_shift<float>(h, p.a, p.b, p.c);
   else if (KIND == K_BGK) coll_bgk_shift<float>(h, p.a);
-  else bgk_dev<float, false>(h, p.a);
+  else bgk_dev(h, p.a);
 #pragma unroll
   for (int q = 0; q < 9; q++) S::store(dst, (I)q * P + o, h[q]);
 }
@@ -178,14 +143,11 @@ __global__ void __launch_bounds__(kBlock) k_step_f16_pull2(const __half* __restr
   } else if constexpr (KIND == K_RR) {
     coll_rr_shift<float, true>(A, p.a, p.b, p.c);
     coll_rr_shift<float, true>(B, p.a, p.b, p.c);
-  } else if constexpr (KIND == K_BGK) {
-    coll_bgk_shift_f16scaled(A, p.a);
-    coll_bgk_shift_f16scaled(B, p.a);
   } else {
     f32x2 H[9];
 #pragma unroll
     for (int q = 0; q < 9; q++) H[q] = pack2(A[q], B[q]);
-    bgk_dev<f32x2, true>(H, p.a);
+    bgk_f16(H, p.a);
 #pragma unroll
     for (int q = 0; q < 9; q++) A[q] = lo2(H[q]), B[q] = hi2(H[q]);
   }
@@ -258,8 +220,9 @@ cudaError_t launch_pull_dev(int kind, const Sweep& s, const CollParams& cp) {
   const ShiftParamsF p = shift_params(kind, cp);
   switch (kind) {
     case K_BGK:
-      if (!packed_bgk(s.nx, s.ny)) return step_cells<k_step_dev_pull<S, K_BGK, I, FLAT>>(s, s.ny, s.nx, false, FLAT, p);
-      return step_cells<k_step_dev_pull<S, kBgkPacked, I, FLAT>>(s, s.ny, s.nx, false, FLAT, p);
+      if constexpr (std::is_same<S, StoreF32Dev>::value)
+        if (packed_bgk(s.nx, s.ny)) return step_cells<k_step_dev_pull<S, kBgkPacked, I, FLAT>>(s, s.ny, s.nx, false, FLAT, p);
+      return step_cells<k_step_dev_pull<S, K_BGK, I, FLAT>>(s, s.ny, s.nx, false, FLAT, p);
     case K_TRT: return step_cells<k_step_dev_pull<S, K_TRT, I, FLAT>>(s, s.ny, s.nx, false, FLAT, p);
     case K_RR: return step_cells<k_step_dev_pull<S, K_RR, I, FLAT>>(s, s.ny, s.nx, false, FLAT, p);
     default: return cudaErrorNotSupported;
@@ -271,9 +234,7 @@ cudaError_t launch_f16_pull2(int kind, const Sweep& s, const CollParams& cp) {
   const bool flat = dev_flat(s.ny / 2, s.nx);
   const ShiftParamsF p = shift_params(kind, cp);
   switch (kind) {
-    case K_BGK:
-      if (!packed_bgk(s.nx, s.ny)) return step_cells<k_step_f16_pull2<K_BGK, I>>(s, s.ny / 2, s.nx, false, flat, p);
-      return step_cells<k_step_f16_pull2<kBgkPacked, I>>(s, s.ny / 2, s.nx, false, flat, p);
+    case K_BGK: return step_cells<k_step_f16_pull2<K_BGK, I>>(s, s.ny / 2, s.nx, false, flat, p);
     case K_TRT: return step_cells<k_step_f16_pull2<K_TRT, I>>(s, s.ny / 2, s.nx, false, flat, p);
     case K_RR: return step_cells<k_step_f16_pull2<K_RR, I>>(s, s.ny / 2, s.nx, false, flat, p);
     default: return cudaErrorNotSupported;

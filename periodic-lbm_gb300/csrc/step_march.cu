@@ -76,10 +76,13 @@ struct MarchF16 {
 };
 
 // Collisions.
-template <bool SC>
+template <class S>
 struct MarchBgk {
   typedef float Params;  // omega
-  __device__ __forceinline__ static void collide(f32x2 (&h)[9], Params omega) { bgk_dev<f32x2, SC>(h, omega); }
+  __device__ __forceinline__ static void collide(f32x2 (&h)[9], Params omega) {
+    if constexpr (S::sc) bgk_f16(h, omega);
+    else bgk_dev(h, omega);
+  }
 };
 
 struct MarchComp {
@@ -273,8 +276,8 @@ cudaError_t march_dev(int storage, bool comp, int steps, const Sweep& s, double 
   if (comp)
     return steps == 2 ? launch_march<MarchF32, MarchComp, 2>(s, df::dev_params(omega))
                       : launch_march<MarchF32, MarchComp, 3>(s, df::dev_params(omega));
-  if (storage == ST_F32DEV) return launch_march<MarchF32, MarchBgk<false>, 3>(s, (float)omega);
-  return launch_march<MarchF16, MarchBgk<true>, 3>(s, (float)omega);
+  if (storage == ST_F32DEV) return launch_march<MarchF32, MarchBgk<MarchF32>, 3>(s, (float)omega);
+  return launch_march<MarchF16, MarchBgk<MarchF16>, 3>(s, (float)omega);
 }
 
 }  // namespace plbm
