@@ -126,8 +126,14 @@ int resident_threads() {
   return n;
 }
 
-// Deviation-storage BGK: the packed operations (bgk_dev, bgk_dev_comp) on grids of at least
-// 2^20 cells, the smallest that a pass of several steps is taken on, in single steps too.
+// binary32 deviation-storage BGK: the packed operators (bgk_dev, bgk_dev_comp) on grids of at
+// least 2^20 cells, the smallest that a pass of several steps is taken on, in single steps too,
+// and the former ones (coll_bgk_shift, bgk_dev_comp_one) below.  The line is not one of speed:
+// small grids' moments are read in binary64, and keep every bit they had; the packed operator
+// errs less (velocities 3e-7 against 3e-6 after the same steps) and rounds otherwise.  binary16
+// has one operator at every size: its stores are 2^-11 of h apart, so that another rounding
+// before them shows (compensated, one cell per thread against pairs: 2048^2 59.4 and 57.2 us
+// per step, 3001 x 2999 123.6 and 127.5).
 inline bool packed_bgk(int nx, int ny) { return (long long)nx * ny >= 1 << 20; }
 
 // Deviation storage takes flat cells but on grids larger than the L2 cache whose rows fit

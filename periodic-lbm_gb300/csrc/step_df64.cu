@@ -32,8 +32,8 @@ __global__ void __launch_bounds__(kBlock) k_step_dev_df(const typename S::elem* 
   for (int q = 0; q < 9; q++) S::store(dst, YFast::off(x, y, q, nx, ny, ld), h[q].hi + h[q].lo);
 }
 
-// Deviation storage, BGK with the compensated binary32 operator on grids below
-// packed_bgk's line, a cell per thread.
+// Deviation storage, BGK with the compensated binary32 operator, a cell per thread:
+// binary16, and binary32 below packed_bgk's line.
 template <class S, typename I>
 __global__ void __launch_bounds__(kBlock) k_step_dev_comp_one(const typename S::elem* __restrict__ src,
                                                              typename S::elem* __restrict__ dst, int nx, int ny,
@@ -136,25 +136,18 @@ cudaError_t step_pull_dev_hi(int storage, int math, int kind, const Sweep& s, co
     if (kind != K_BGK) return cudaErrorNotSupported;
     const df::DevParams p = df::dev_params(cp.omega);
     const bool small = (unsigned long long)s.ld * (unsigned long long)s.nx * 9ull < (1ull << 32);
-    if (!packed_bgk(s.nx, s.ny)) {
-      // fewer than 2^32 elements unless the rows are mostly padding
-      if (storage == ST_F32DEV)
-        return small ? step_cells<k_step_dev_comp_one<StoreF32Dev, uint32_t>>(s, s.ny, s.nx, false, true, p)
-                     : step_cells<k_step_dev_comp_one<StoreF32Dev, size_t>>(s, s.ny, s.nx, false, true, p);
-      if (storage == ST_F16DEV)
-        return small ? step_cells<k_step_dev_comp_one<StoreF16Dev, uint32_t>>(s, s.ny, s.nx, false, true, p)
-                     : step_cells<k_step_dev_comp_one<StoreF16Dev, size_t>>(s, s.ny, s.nx, false, true, p);
-      return cudaErrorInvalidValue;
-    }
+    // binary16: the one-cell kernel at every size (packed_bgk)
+    if (storage == ST_F16DEV)
+      return small ? step_cells<k_step_dev_comp_one<StoreF16Dev, uint32_t>>(s, s.ny, s.nx, false, true, p)
+                   : step_cells<k_step_dev_comp_one<StoreF16Dev, size_t>>(s, s.ny, s.nx, false, true, p);
+    if (storage != ST_F32DEV) return cudaErrorInvalidValue;
+    if (!packed_bgk(s.nx, s.ny))  // fewer than 2^32 elements unless the rows are mostly padding
+      return small ? step_cells<k_step_dev_comp_one<StoreF32Dev, uint32_t>>(s, s.ny, s.nx, false, true, p)
+                   : step_cells<k_step_dev_comp_one<StoreF32Dev, size_t>>(s, s.ny, s.nx, false, true, p);
     const int pairs = s.nx / 2 + (s.nx & 1);
     const bool flat = dev_flat(s.ny, pairs);
-    if (storage == ST_F32DEV)
-      return small ? step_cells<k_step_dev_comp<StoreF32Dev, uint32_t>>(s, s.ny, pairs, false, flat, p)
-                   : step_cells<k_step_dev_comp<StoreF32Dev, size_t>>(s, s.ny, pairs, false, flat, p);
-    if (storage == ST_F16DEV)
-      return small ? step_cells<k_step_dev_comp<StoreF16Dev, uint32_t>>(s, s.ny, pairs, false, flat, p)
-                   : step_cells<k_step_dev_comp<StoreF16Dev, size_t>>(s, s.ny, pairs, false, flat, p);
-    return cudaErrorInvalidValue;
+    return small ? step_cells<k_step_dev_comp<StoreF32Dev, uint32_t>>(s, s.ny, pairs, false, flat, p)
+                 : step_cells<k_step_dev_comp<StoreF32Dev, size_t>>(s, s.ny, pairs, false, flat, p);
   }
   if (math == 3) {  // double-float
     if (kind != K_BGK) return cudaErrorNotSupported;
