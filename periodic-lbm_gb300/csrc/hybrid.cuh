@@ -540,13 +540,16 @@ DF_HD void bgk_fma(double (&f)[9], const BgkParams& p, bool& bad) {
   }
 }
 
-// Recursive-regularized constant (rr_fma): 1 - omega at scale 2^63.
+// Recursive-regularized constant (rr_fma): 1 - omega at scale 2^63, for omega in [0, 2]
+// (the ends 2^-63 inside it).  Another omega, or none, has no place in that scale: every
+// cell is then out of range.
 struct RrParams {
   int64_t omb;
+  bool out;
 };
 inline RrParams rr_fma_params(double omega) {
-  RrParams r;
-  const double b = ldexp(1.0 - omega, 63);
+  RrParams r = {0, !(omega >= 0.0 && omega <= 2.0)};
+  const double b = r.out ? 0.0 : ldexp(1.0 - omega, 63);
   r.omb = b >= 0x1p63 ? INT64_MAX : (b <= -0x1p63 ? INT64_MIN + 1 : (int64_t)llrint(b));
   return r;
 }
@@ -573,7 +576,7 @@ inline RrParams rr_fma_params(double omega) {
 // brackets sum to zero with the weights exactly, as T_q - 36 w_q F_q does; the
 // reference's binary64 weights (sums 1 - 2^-54) take 2^-54 of the mass and
 // momentum each step, restored by p.mass_k / p.mom_k (bgk_fma_params at
-// omega = 1).  Range as bgk_fma, q_xx + q_yy < 0.2 and sum |M / 2| < 0.1: then the Hermite parts
+// omega = 1).  Range: omega in [0, 2], as bgk_fma, q_xx + q_yy < 0.2 and sum |M / 2| < 0.1: then the Hermite parts
 // add at most 3, 0.9 and 1.8 (units of 2^59) to the rest, axis and diagonal
 // brackets, which stay below 13 x 2^59, and no product's operand leaves int64.
 template <bool SHIFTED>
@@ -606,7 +609,7 @@ DF_HD void rr_brackets(const int64_t (&F)[9], const RrParams& r, const BgkParams
   // sum |M / 2| < 0.1, on the leading words
   const uint32_t sum2 = uabs_hi(mxx) + uabs_hi(myy) + 3 * uabs_hi(mxy);  // scale 6 2^28
   const uint32_t sum3 = uabs_hi(mxxy) + uabs_hi(myyx) + uabs_hi(mxxyy);  // scale 6 2^30
-  bad |= rho_out_of_range(Rrho) | ((int32_t)((qxx + qyy) >> 34) >= kTurn02) | (sum2 >= kTurn06 / 4) |
+  bad |= r.out | rho_out_of_range(Rrho) | ((int32_t)((qxx + qyy) >> 34) >= kTurn02) | (sum2 >= kTurn06 / 4) |
          (4 * sum2 + sum3 >= kTurn06);
   const int64_t X3 = round_shr(mxx, 2), Y3 = round_shr(myy, 2), K = round_shr(9 * mxy, 1);
   const int64_t GY = round_shr(3 * mxxy, 4), GX = round_shr(3 * myyx, 4), G = round_shr(3 * mxxyy, 4);
