@@ -270,6 +270,9 @@ DF_HD double fixed_to_double_tr(int64_t T) {
 // (diagonal) or 2^-59 (axis, rest; places of 2^-56 and 2^-54).  Norm-wise error
 // against 113-bit arithmetic as with the FMAs: BGK 1.31e-16 / 1.33e-16, TRT
 // 1.31e-16 / 1.32e-16, RR 1.16e-16 / 1.17e-16.
+// Rate: omega (TRT: lambda_e) in [0, 2], where c fits 2^66 and every new population of a
+// cell in range 2^61; a launch with another rate takes the binary64 FMAs.
+inline bool finish_takes(double omega) { return omega >= 0.0 && omega <= 2.0; }
 PLBM_NOINLINE void finish_slow(double* f, const int64_t* Y, double c0, double cs, double cd) {
   for (int q = 0; q < 9; q++) f[q] = fma_d(q == 0 ? c0 : (q < 5 ? cs : cd), fixed_to_double_tr(Y[q]), f[q]);
 }
@@ -389,7 +392,7 @@ inline BgkParams bgk_fma_params(double omega, const double (&w)[3]) {
   const double km = ldexp(omega * eps_m / p.c4, 64), kj = ldexp(0.5 * omega * eps_j / p.c4, 64);
   p.mass_k = fabs(km) < 0x1p30 ? (int32_t)llrint(km) : 0;
   p.mom_k = fabs(kj) < 0x1p30 ? (int32_t)llrint(kj) : 0;
-  p.c_fx = llrint(ldexp(p.c1, 66));
+  p.c_fx = finish_takes(omega) ? llrint(ldexp(p.c1, 66)) : 0;
   return p;
 }
 
@@ -711,7 +714,7 @@ inline TrtFmaParams trt_fma_params(double lambda_e, double lambda_d, const doubl
   const double kj = ldexp(lambda_d * first_moment_error(w) / p.c2, 64);
   p.mass_k = fabs(km) < 0x1p30 ? (int32_t)llrint(km) : 0;
   p.mom_k = fabs(kj) < 0x1p30 ? (int32_t)llrint(kj) : 0;
-  p.c_fx = llrint(ldexp(p.ch, 66));
+  p.c_fx = finish_takes(lambda_e) ? llrint(ldexp(p.ch, 66)) : 0;
   return p;
 }
 

@@ -431,7 +431,7 @@ template <int KIND>
 cudaError_t launch_hybrid(const Sweep& s, const HybridArgs& a) {
   if ((unsigned long long)s.ld * (unsigned long long)s.nx * 9ull >= (1ull << 32))
     return step_cells<k_step_hybrid<size_t, KIND, false>>(s, s.ny, s.nx, true, true, a);
-  if ((long long)s.nx * s.ny > kQuickCells)
+  if ((long long)s.nx * s.ny > kQuickCells || !hy::finish_takes(a.ref.omega))
     return step_cells<k_step_hybrid<uint32_t, KIND, false>>(s, s.ny, s.nx, true, true, a);
   // rows that fill their blocks: the same cells, 0.1 us (of 2) sooner
   const bool flat = s.ny % block_for((long long)s.nx * s.ny, true) != 0;
@@ -490,6 +490,7 @@ namespace {
 // The fixed-point constants of a scheme, or false where it keeps the stencil
 // form (see k_step_scheme_fixed).
 bool scheme_fixed_constants(int scheme, int kind, double dt, double omega, int& form, SchemeFx& c) {
+  if (!hy::finish_takes(omega)) return false;
   double a1s, a2s, a1d, a2d;
   switch (scheme) {
     case sch::SOFONEA:

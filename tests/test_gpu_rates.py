@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
-KINDS = {"rr": 2}
+KINDS = {"bgk": 0, "trt": 1, "rr": 2}
 W = np.array((4 / 9,) + (1 / 9,) * 4 + (1 / 36,) * 4)
 RATES = [-1.0, 0.0, 1.9, 2.0, 2.05, 2.5, 4.6, 5.0, 100.0, math.nan]
 
