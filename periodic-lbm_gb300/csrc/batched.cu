@@ -373,8 +373,7 @@ cudaError_t launch_kinds(const BatchLaunch& L, int parity) {
   return cudaGetLastError();
 }
 
-// Dynamic shared memory of the persistent kernel (raised past 48 KB where the
-// schedule is applied, in batch_max_ctas).
+// Dynamic shared memory of the persistent kernel.
 template <class S>
 int persistent_smem(int threads) {
   return S::ddf ? 0 : 2 * 9 * 8 * threads;
@@ -431,10 +430,14 @@ namespace {
 template <class S, typename I>
 cudaError_t persistent_ctas(int threads, int* per_sm) {
   auto kernel = !S::ddf && threads <= 256 ? k_batch_persistent<S, I, 256> : k_batch_persistent<S, I, kBatchMaxThreads>;
-  const int smem = persistent_smem<S>(threads);
-  if (smem > 48 * 1024)
-    if (cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, threads, smem);
+  // With its static tables the kernel for more than 256 threads passes 48 KB, from 320
+  // threads on.  The limit belongs to the kernel, which every batch shares: the most that
+  // any schedule asks for, whichever schedule this is.
+  if (!S::ddf && threads > 256)
+    if (cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             persistent_smem<S>(kBatchMaxThreads)))
+      return e;
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, threads, persistent_smem<S>(threads));
 }
 }  // namespace
 
