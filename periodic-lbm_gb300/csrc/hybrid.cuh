@@ -479,7 +479,6 @@ DF_HD void load_fixed(const double (&f)[9], int64_t (&F)[9], bool& bad, bool& sm
 // rho outside [2^-2 + 2^-27, 4): the reciprocal's range.
 DF_HD bool rho_out_of_range(int64_t R) { return (uint32_t)((uint64_t)R >> 32) - 0x2000001u > 0x1dfffffeu; }
 constexpr int32_t kTurn02 = 26843545;    // 0.2 2^27
-constexpr uint32_t kTurn06 = 644245094;  // 0.6 2^30
 
 // SHIFTED: f holds h = f - w (the plugin's storage, sim/sim.F90:131).  The
 // linear brackets then take DH = sum h = rho - 1 in place of R (the w terms
@@ -548,11 +547,12 @@ DF_HD void bgk_fma(double (&f)[9], const BgkParams& p, bool& bad) {
 // cell is then out of range.
 struct RrParams {
   int64_t omb;
-  bool out;
+  uint32_t limit;  // of 6 sum |M / 2| 2^30; 0: every cell
 };
+constexpr uint32_t kTurn06 = 644245094;  // 0.6 2^30
 inline RrParams rr_fma_params(double omega) {
-  RrParams r = {0, !(omega >= 0.0 && omega <= 2.0)};
-  const double b = r.out ? 0.0 : ldexp(1.0 - omega, 63);
+  RrParams r = {0, omega >= 0.0 && omega <= 2.0 ? kTurn06 : 0};
+  const double b = r.limit ? ldexp(1.0 - omega, 63) : 0.0;
   r.omb = b >= 0x1p63 ? INT64_MAX : (b <= -0x1p63 ? INT64_MIN + 1 : (int64_t)llrint(b));
   return r;
 }
@@ -612,8 +612,8 @@ DF_HD void rr_brackets(const int64_t (&F)[9], const RrParams& r, const BgkParams
   // sum |M / 2| < 0.1, on the leading words
   const uint32_t sum2 = uabs_hi(mxx) + uabs_hi(myy) + 3 * uabs_hi(mxy);  // scale 6 2^28
   const uint32_t sum3 = uabs_hi(mxxy) + uabs_hi(myyx) + uabs_hi(mxxyy);  // scale 6 2^30
-  bad |= r.out | rho_out_of_range(Rrho) | ((int32_t)((qxx + qyy) >> 34) >= kTurn02) | (sum2 >= kTurn06 / 4) |
-         (4 * sum2 + sum3 >= kTurn06);
+  bad |= rho_out_of_range(Rrho) | ((int32_t)((qxx + qyy) >> 34) >= kTurn02) | (sum2 >= kTurn06 / 4) |
+         (4 * sum2 + sum3 >= r.limit);
   const int64_t X3 = round_shr(mxx, 2), Y3 = round_shr(myy, 2), K = round_shr(9 * mxy, 1);
   const int64_t GY = round_shr(3 * mxxy, 4), GX = round_shr(3 * myyx, 4), G = round_shr(3 * mxxyy, 4);
   Y[0] = 4 * (R - X3 - Y3) - 9 * F[0] + 2 * G + scale_2m64(R, p.mass_k);
