@@ -23,6 +23,8 @@
 // lambda_0 in binary64 (k_adj_u0).
 #include <cuda_runtime.h>
 
+#include <cmath>
+
 #include "../../include/plbm_gpu.h"
 #include "coll_df64.cuh"
 #include "hybrid.cuh"
@@ -80,11 +82,23 @@ __device__ __forceinline__ void cell_state(const R (&g)[9], R& rho, R& ux, R& uy
   }
 }
 
+// Constants of a reverse step: omega, and in binary64 1 - omega and 3 omega = om3 + om3_lo.
+template <typename R>
+struct Rates {
+  R om, omb, om3, om3_lo;
+};
+template <typename R>
+inline Rates<R> rates(double omega) {
+  return {(R)omega, (R)(1.0 - omega), (R)(3.0 * omega), (R)std::fma(3.0, omega, -(3.0 * omega))};
+}
+
 // One cell of the reverse step, binary32: mu = J_C(g)^T lambda and the dL/domega
 // term sum_q l_q (feq_q - g_q).  (The binary64 form's pair sums would not run
 // faster here, where the loads bind, and round otherwise.)
-__device__ __forceinline__ float reverse_cell(const float (&g)[9], const float (&l)[9], float om, float (&mu)[9]) {
+__device__ __forceinline__ float reverse_cell(const float (&g)[9], const float (&l)[9], const Rates<float>& p,
+                                              float (&mu)[9]) {
   typedef float R;
+  const R om = p.om;
   R neq[9], rho, ux, uy;
   cell_state<R, true>(g, rho, ux, uy, neq);
   const R u2 = ux * ux + uy * uy;
@@ -137,11 +151,12 @@ __device__ __forceinline__ double forward_state(const double (&g)[9], const doub
   }
   ux = hy::fixed_to_double_tr<61>(U);
   uy = hy::fixed_to_double_tr<61>(V);
-  double ds = l[0] * hy::fixed_to_double_tr(Y[0]), dd = l[5] * hy::fixed_to_double_tr(Y[5]);
+  auto y = [&](int q) { return hy::fixed_to_double_tr<hy::kScale>(Y[q]); };
+  double ds = l[0] * y(0), dd = l[5] * y(5);
 #pragma unroll
-  for (int q = 1; q < 5; q++) ds += l[q] * hy::fixed_to_double_tr(Y[q]);
+  for (int q = 1; q < 5; q++) ds += l[q] * y(q);
 #pragma unroll
-  for (int q = 6; q < 9; q++) dd += l[q] * hy::fixed_to_double_tr(Y[q]);
+  for (int q = 6; q < 9; q++) dd += l[q] * y(q);
   return (4.0 * ds + dd) * (1.0 / 36.0);
 }
 
@@ -156,7 +171,11 @@ __device__ __forceinline__ double forward_state(const double (&g)[9], const doub
 // not drop, two divisions and the equilibria took more than three times as many.
 // 256^2: 46.8 us per reverse step (with its share of the recomputation) before,
 // 19.0 now; 1024^2 618 and 187.
-__device__ __forceinline__ double reverse_cell(const double (&g)[9], const double (&l)[9], double om,
+// 3 omega is exact in two parts: rounded to one, it changes lambda's momentum by up to 1.5e-16
+// in every step alike (300 x 257, tau = 0.52, 120 steps: dL/du0 1.7e-14 from the exact one in
+// the mean square, 1.1e-15 now, 2.6e-15 with the sums over nine populations; 256^2, tau = 0.6,
+// 200 steps: 1.3e-14, 2.7e-15 and 1.2e-14).
+__device__ __forceinline__ double reverse_cell(const double (&g)[9], const double (&l)[9], const Rates<double>& p,
                                                double (&mu)[9]) {
   double ux, uy;
   const double d = forward_state(g, l, ux, uy);
@@ -168,9 +187,9 @@ __device__ __forceinline__ double reverse_cell(const double (&g)[9], const doubl
   const double mx = WD * (m57 + m86) + WS * (l[1] - l[3]), my = WD * (m57 - m86) + WS * (l[2] - l[4]);
   const double qx = ux * kxx + uy * kxy, qy = uy * kyy + ux * kxy;
   const double n = 4.5 * (ux * qx + uy * qy) - (1.5 * s0) * (ux * ux + uy * uy);
-  const double omb = 1.0 - om, om3 = 3.0 * om;
-  const double a = om * (s0 - n);
-  const double ex = om3 * ((mx + 3.0 * qx) - s0 * ux), ey = om3 * ((my + 3.0 * qy) - s0 * uy);
+  const double omb = p.omb, a = p.om * (s0 - n);
+  const double tx = (mx + 3.0 * qx) - s0 * ux, ty = (my + 3.0 * qy) - s0 * uy;
+  const double ex = __fma_rn(p.om3, tx, p.om3_lo * tx), ey = __fma_rn(p.om3, ty, p.om3_lo * ty);
   const double ep = ex + ey, em = ex - ey;
   mu[0] = omb * l[0] + a;
   mu[1] = omb * l[1] + (a + ex);
@@ -249,7 +268,7 @@ __global__ void __launch_bounds__(kBlock) k_adj_final(const void* __restrict__ f
 template <int ST, typename I>
 __global__ void __launch_bounds__(kBlock) k_adj_step(const void* __restrict__ f, const void* __restrict__ lam_in,
                                                     void* __restrict__ lam_out, double* __restrict__ dom,
-                                                    typename AdjTraits<ST>::real om, int nx, int ny, int ld,
+                                                    Rates<typename AdjTraits<ST>::real> p, int nx, int ny, int ld,
                                                     Rows rows) {
   chain_begin();
   typedef typename AdjTraits<ST>::real R;
@@ -273,7 +292,7 @@ __global__ void __launch_bounds__(kBlock) k_adj_step(const void* __restrict__ f,
       g[q] = (R)ld_chain(fe + off[q]);
       l[q] = (R)ld_chain(li + ((I)q * P + c0 + y0));
     }
-    part = reverse_cell(g, l, om, mu);
+    part = reverse_cell(g, l, p, mu);
 #pragma unroll
     for (int p = 0; p < 9; p++) lo[off[p]] = (E)mu[p];
   }
@@ -384,8 +403,8 @@ cudaError_t dispatch(int what, const AdjLaunch& a) {
         if (small) return reverse_step<k_adj_step_comp<uint32_t>>(a, cpar);
         return reverse_step<k_adj_step_comp<size_t>>(a, cpar);
       }
-      if (small) return reverse_step<k_adj_step<ST, uint32_t>>(a, (typename AdjTraits<ST>::real)a.omega);
-      return reverse_step<k_adj_step<ST, size_t>>(a, (typename AdjTraits<ST>::real)a.omega);
+      if (small) return reverse_step<k_adj_step<ST, uint32_t>>(a, rates<typename AdjTraits<ST>::real>(a.omega));
+      return reverse_step<k_adj_step<ST, size_t>>(a, rates<typename AdjTraits<ST>::real>(a.omega));
     case 3: k_adj_u0<ST><<<nb, kBlock, 0, a.stream>>>(a.lam_in, a.u, a.out, a.nx, a.ny, a.ld, ft); break;
     default: return cudaErrorInvalidValue;
   }
