@@ -151,7 +151,7 @@ __device__ __forceinline__ double forward_state(const double (&g)[9], const doub
   }
   ux = hy::fixed_to_double_tr<61>(U);
   uy = hy::fixed_to_double_tr<61>(V);
-  auto y = [&](int q) { return hy::fixed_to_double_tr<hy::kScale>(Y[q]); };
+  auto y = [&](int q) { return hy::fixed_to_double_tr<hy::kScale, true>(Y[q]); };
   double ds = l[0] * y(0), dd = l[5] * y(5);
 #pragma unroll
   for (int q = 1; q < 5; q++) ds += l[q] * y(q);

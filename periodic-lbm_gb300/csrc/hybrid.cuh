@@ -241,11 +241,16 @@ DF_HD double pos_fixed_to_double(int64_t v) {
 // 2^-52 relative plus 2^-59 absolute -- for the non-equilibrium brackets it
 // converts, negligible against the binary64 rounding of the populations.  (Selecting the
 // words without a branch put more on the ALU pipe, which binds: 8192^2 TRT 33.3
-// GLUPS against 36.)
-template <int SCALE = kScale>
+// GLUPS against 36.)  EXACT: a negative T's own magnitude, for sums over many T, in which
+// half of a unit on average adds up.
+template <int SCALE = kScale, bool EXACT = false>
 DF_HD double fixed_to_double_tr(int64_t T) {
-  const uint32_t hi = (uint32_t)((uint64_t)T >> 32), lo = (uint32_t)(uint64_t)T;
+  uint32_t hi = (uint32_t)((uint64_t)T >> 32), lo = (uint32_t)(uint64_t)T;
   const uint32_t s = (uint32_t)((int32_t)hi >> 31);  // 0 or ~0
+  if (EXACT) {
+    const uint64_t m = (uint64_t)T + (((uint64_t)s << 32) | s);  // -T = ~(T - 1)
+    hi = (uint32_t)(m >> 32), lo = (uint32_t)m;
+  }
   const uint32_t ah = hi ^ s, al = lo ^ s;
   if (ah == 0u) return fixed_to_double_any_slow(T) * pow2_const(kScale - SCALE);
   const uint32_t lz = clz32(ah);  // 0..31
