@@ -10,9 +10,9 @@
 // registers: populations moving in +x for two columns, resting in x for one,
 // moving in -x none; the shift by one row within the strip is one shuffle of half
 // a pair.  No shared memory and no barrier: the warps are independent.  Each step
-// after the first loses one row at either end of the strip, so 60 of 64 rows are
-// stored for T <= 3 (the pulls of the first step read outside the strip), and the
-// T - 1 columns before and after a segment of columns are computed twice.
+// loses one row at either end of the strip, so that, in whole lanes, 60 of its 64 rows are
+// stored for T <= 2 and 56 for T = 3, and the T - 1 columns before and after a segment of
+// columns are computed twice.
 // Binary16 values are rounded to storage between the steps, so that the result has
 // the bits of T single steps.
 //
@@ -214,16 +214,18 @@ cudaError_t launch_march(const Sweep& s, const typename C::Params& p) {
   const int gx = (strips + kMarchWarps - 1) / kMarchWarps;
   // One wave of CTAs, in segments of at least 16 columns; on grids long enough
   // for segments of 160 columns all the same, up to four waves, which even out the
-  // strips at the grid's edge; three on grids of an odd ny, whose edge strips load row by
-  // row (8192^2, 1 / 2 / 4 waves: binary32 215 / 218 / 220 GLUPS,
-  // binary16 224 / 232 / 240; 2048^2 binary32 186 / 174 / 166;
-  // 3001 x 2999 binary32, 1 / 2 / 3 waves: 156 / 159 / 168).
+  // strips at the grid's edge (8192^2, 1 / 2 / 4 waves: binary32 215 / 218 / 220 GLUPS,
+  // binary16 224 / 232 / 240; 2048^2 binary32 186 / 174 / 166).  Binary16 with an odd ny,
+  // whose edge strips load row by row, from 32 columns on (1 / 2 / 3 / 4 waves: 3001 x 2999
+  // 180 / 194 / 196 / 195, 2999 x 5001 178 / 199 / 203 / 206, 5121^2 178 / 205 / 215 / 217, but 1500 x
+  // 1401 157 / 135, 700 x 2999 165 / 154).  Binary32 with an odd ny is no different from
+  // an even one (3001 x 2999 226 / 218 / 212, compensated 88.6 / 88.0 / 85.6, 1500 x 1401 185 /
+  // 140 and 80 / 69).
   int segs = cap / gx;
   if (segs > s.nx / 16) segs = s.nx / 16;
   if (segs < 1) segs = 1;
-  int waves = s.nx / (160 * segs);
+  int waves = s.nx / ((S::sc && s.ny % 2 != 0 ? 32 : 160) * segs);
   if (waves > 4) waves = 4;
-  if (s.ny % 2 != 0 && waves < 3) waves = 3;
   if (waves > 1) segs = segs * waves < s.nx / 16 ? segs * waves : s.nx / 16;
   const int seg = (s.nx + segs - 1) / segs;
   segs = (s.nx + seg - 1) / seg;
