@@ -194,7 +194,7 @@ constexpr int batch_min_blocks(int max_threads) {
   return (S::ddf ? 1536 : 1024) / max_threads;
 }
 
-// The persistent binary64 kernel at 256 threads: three CTAs (80 registers, no spill) hide
+// The persistent binary64 kernel at 256 threads: three CTAs (80 registers, 16 bytes spilled) hide
 // the copies as well as four (64, 84 bytes spilled), and fewer meet at the barrier: 512
 // grids 1.117 -> 1.091 ms per step, 8 grids 17.6 -> 16.6 us; two CTAs 1.162 and 15.3.
 template <class S>

@@ -63,13 +63,18 @@ DF_HD float vfma(float a, float b, float c) {
   return fmaf(a, b, c);
 #endif
 }
+// 1 / x within 1 ulp (the bound that is documented for it; a host build may define
+// PLBM_HOST_SEED to try other values within it).
+#ifndef PLBM_HOST_SEED
+#define PLBM_HOST_SEED(x) (1.0f / (x))
+#endif
 DF_HD float rcp_seed(float x) {
 #ifdef __CUDA_ARCH__
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 #else
-  return 1.0f / x;
+  return PLBM_HOST_SEED(x);
 #endif
 }
 // The constant c in a value of type V.

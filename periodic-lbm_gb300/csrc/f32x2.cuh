@@ -5,7 +5,9 @@
 // the same bits in both.  GB300 retires the packed operations at half the issue
 // slots of the scalar ones and the same 128 values per clock and SM (measured).
 #pragma once
+#ifdef __CUDACC__
 #include <cuda_runtime.h>
+#endif
 #include <stdint.h>
 #include "df64.cuh"
 
@@ -17,6 +19,9 @@ struct f32x2 {
 DF_HD f32x2 pack2(float lo, float hi) {
   return {((unsigned long long)df::f2u(hi) << 32) | (unsigned long long)df::f2u(lo)};
 }
+template <>
+DF_HD f32x2 vset<f32x2>(float c) { return pack2(c, c); }
+#ifdef __CUDACC__
 __device__ __forceinline__ float lo2(f32x2 a) {
   return __uint_as_float((unsigned)a.v);
 }
@@ -44,19 +49,18 @@ __device__ __forceinline__ f32x2 vfma(f32x2 a, f32x2 b, f32x2 c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
   return r;
 }
-template <>
-DF_HD f32x2 vset<f32x2>(float c) { return pack2(c, c); }
 // a b, not to be contracted into a sum that follows: ptxas fuses a packed product and
 // sum, .rn or not; a fused product and sum of its own is left alone (+ -0 changes no
 // product, not even the sign of a zero).
-__device__ __forceinline__ float vprod(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ f32x2 vprod(f32x2 a, f32x2 b) { return vfma(a, b, vset<f32x2>(-0.0f)); }
 __device__ __forceinline__ f32x2 rcp_seed(f32x2 x) { return pack2(rcp_seed(lo2(x)), rcp_seed(hi2(x))); }
+#endif
+DF_HD float vprod(float a, float b) { return vmul(a, b); }
 
 // a / x with r = vrcp(x): the product and its exact residual added back
 // (Markstein 1990), within half an ulp and a hair.
 template <typename V>
-__device__ __forceinline__ V vquot(V a, V x, V r) {
+DF_HD V vquot(V a, V x, V r) {
   const V q = vmul(a, r);
   const V e = vfma(vsub(vset<V>(0.0f), x), q, a);
   return vfma(e, r, q);
@@ -69,7 +73,7 @@ __device__ __forceinline__ V vquot(V a, V x, V r) {
 // operations.  The O(h) terms come from dr and j themselves, not from rho - 1 and
 // rho u, which lose dr's low bits to the rounding of rho = 1 + dr.
 template <typename V>
-__device__ __forceinline__ void bgk_dev(V (&h)[9], float omega) {
+DF_HD void bgk_dev(V (&h)[9], float omega) {
   // the three binary32 weights share one relative error, 7e-9, with which mass and
   // momentum drift; 3 w c.j with a rounded 3 w would drift four times as fast
   const float w0 = 4.0f / 9.0f, ws = 1.0f / 9.0f, wd = 1.0f / 36.0f;
@@ -107,10 +111,18 @@ __device__ __forceinline__ void bgk_dev(V (&h)[9], float omega) {
 // that one cell per thread, two per thread and a pass of several steps give the same
 // bits: an operator that rounds otherwise lands on another binary16 value now and
 // then, 2^-11 of h apart.
-__device__ __forceinline__ float f16_inv_rho(float rho) { return __fdividef(1.0f / 32768.0f, rho); }
+DF_HD float f16_inv_rho(float rho) {
+#ifdef __CUDA_ARCH__
+  return __fdividef(1.0f / 32768.0f, rho);
+#else
+  return 1.0f / 32768.0f / rho;
+#endif
+}
+#ifdef __CUDACC__
 __device__ __forceinline__ f32x2 f16_inv_rho(f32x2 rho) { return pack2(f16_inv_rho(lo2(rho)), f16_inv_rho(hi2(rho))); }
+#endif
 template <typename V>
-__device__ __forceinline__ void bgk_f16(V (&H)[9], float omega) {
+DF_HD void bgk_f16(V (&H)[9], float omega) {
   const V s13 = vadd(H[1], H[3]), s24 = vadd(H[2], H[4]), s57 = vadd(H[5], H[7]), s68 = vadd(H[6], H[8]);
   const V d13 = vsub(H[1], H[3]), d24 = vsub(H[2], H[4]), d57 = vsub(H[5], H[7]), d86 = vsub(H[8], H[6]);
   const V dh = vadd(vadd(vadd(s57, s68), vadd(s13, s24)), H[0]);

@@ -52,12 +52,10 @@ DF_HD int64_t mulh64(int64_t a, int64_t b) {
 // meaningless value (the callers report such cells as out of range).
 DF_HD int64_t recip_fixed(int64_t R) {
   // rho 2^30 and 2^26 / rho
+  const float y = rcp_seed((float)(uint32_t)(R >> 29));
 #ifdef __CUDA_ARCH__
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint2float_rn((uint32_t)(R >> 29))));
   const uint32_t Y = __float2uint_rz(y * 0x1p56f);
 #else
-  const float y = 1.0f / (float)(uint32_t)(R >> 29);
   const float yf = y * 0x1p56f;
   const uint32_t Y = yf < 0x1p31f ? (uint32_t)yf : 0x7fffffffu;
 #endif
