@@ -53,10 +53,10 @@ import numpy as np  # noqa: E402
 BYTES_PER_CELL = {"f64": 144, "f32dev": 72, "f16dev": 36}
 # DRAM bytes per cell update measured by ncu (dram__bytes_read.sum +
 # dram__bytes_write.sum of one launch / cells) on a 2048^2 capture of the same
-# kernel, scaled by the cell count: profiles/step_kernels_pipes.md (BGK),
-# profiles/k_step_*_2048_fullset.md.
-NCU_TRAFFIC_PER_CELL = {("f64", "bgk", "hybrid"): 131.4, ("f64", "trt", "hybrid"): 132.4,
-                        ("f64", "rr", "hybrid"): 133.0, ("f64", "bgk", "fma"): 131.4}
+# kernel (profiles/step_kernels_pipes.md), scaled by the cell count; FMA and
+# hybrid arithmetic run the same kernels.
+NCU_TRAFFIC_PER_CELL = {("f64", kind, math): b for kind, b in (("bgk", 131.4), ("trt", 133.1), ("rr", 132.3))
+                        for math in ("hybrid", "fma")}
 FALLBACK_HBM_GBS = 6800.0
 
 
