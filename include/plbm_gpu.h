@@ -53,16 +53,23 @@ extern "C" {
  *          moments, fixed-point products, one binary64 FMA per population; the
  *          error per step is no larger than that of the binary64 operators
  *          with FMA contraction, which a cell outside the fixed point's range
- *          (as for HYBRID) and the improved BGK take
+ *          (as for HYBRID) and the improved BGK take.  This is the fused step
+ *          (plbm_perform_lbm_step, plbm_launch_step, batches);
+ *          plbm_collide and plbm_perform_triple_step evaluate the binary64
+ *          operators, so that the same step rounds differently by route
  *   STRICT binary64, no contraction: the Fortran's operations in its order,
  *          bit-identical to it
  *   HYBRID BGK, TRT and RR: the same step, and integer forms of the moments
  *          and equilibria (plbm_update_macros below).  A cell out of range
  *          (f_0 outside [0, 1), f_axis [0, 1/4), f_diagonal [0, 1/8), density
- *          <= 1/4, or too fast) is evaluated with the binary64 operator
- *          instead (see plbm_hybrid_range_flag)
+ *          <= 1/4, or too fast; RR: any cell, at a rate outside [0, 2]) is
+ *          evaluated with the binary64 operator instead (see
+ *          plbm_hybrid_range_flag)
  * Deviation storage (PLBM_F32DEV / PLBM_F16DEV):
- *   FMA    binary32 collision (default)
+ *   FMA    binary32 collision (default).  PLBM_F32DEV BGK, FMA and HYBRID,
+ *          has one operator below 2^20 cells and another, which rounds
+ *          otherwise and in FMA less, from there on: the result of a
+ *          lattice's step depends on its size in the last binary32 places
  *   STRICT binary64 collision on the stored deviations
  *   HYBRID BGK only: compensated binary32 collision (exact pairwise sums,
  *          hi+lo pairs for the O(h) linear terms, binary32 nonlinear term)

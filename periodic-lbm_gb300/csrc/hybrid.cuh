@@ -12,8 +12,7 @@
 //   R, JX, JY = sum F_q, sum cx F_q, sum cy F_q          exact integer sums
 //   f'_q      = fma(c_q, Y_q 2^-59, f_q)                  ONE binary64 FMA
 // where Y_q is an integer bracket holding the whole update of population q
-// (the linear part exact, the nonlinear part from double-float or exact
-// 128-bit products taken to the fixed point once), c_q a power-of-two multiple
+// (the linear part exact, the nonlinear part from fixed-point products), c_q a power-of-two multiple
 // of one rounded relaxation constant, so that the brackets of the nine
 // populations sum to zero with the weights exactly: mass and momentum change
 // only by the nine final roundings, plus the drift the reference's own

@@ -49,7 +49,10 @@ struct Rows {
 // others' time (us per step, without flat cells and limit / with flat cells / with both:
 // 300^2 BGK 5.1 / 5.1 / 4.1, 256^2 RR 5.3 / 5.3 / 4.2, 1000 x 65 BGK 4.9 / 3.6 / 3.7,
 // 641 x 500 plugin BGK 11.1 / 10.0 / 10.0, 300^2 plugin RR 45.9 / 45.9 / 29.6).  The same limit
-// on grids of two waves and more: 400^2 BGK 5.6 -> 6.3, not taken.
+// on grids of two waves and more: 400^2 BGK 5.6 -> 6.3, not taken.  A kernel of another stream
+// that needs shared memory or more warps than the limit leaves waits for the limited CTAs: a
+// 300^2 BGK grid beside a 2048^2 binary32 one, 25.3 us per pair of steps without the limit
+// and 31.6 with it; two 300^2 BGK grids 5.8 and 4.8, 256^2 RR beside 128^2 BGK 5.4 and 4.8.
 struct Spread {
   unsigned blocks;
   int threads, smem;
