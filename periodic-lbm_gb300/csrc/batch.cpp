@@ -79,16 +79,19 @@ void drop_graphs(plbm_batch_t* b) {
 
 // Tiles are numbered grid by grid, the BGK grids' first and the TRT grids'
 // after them, so that the per-step launch can run each kind with its own
-// kernel over a contiguous range.
-int apply_schedule(plbm_batch_t* b) {
+// kernel over a contiguous range.  A schedule that cannot be applied leaves the batch
+// with the one it had.
+int apply_schedule(plbm_batch_t* b, const plbm_batch_schedule& sched) {
   std::vector<BatchTile> tiles;
-  const int threads = b->sched.threads;
-  b->nt_bgk = 0;
+  const int threads = sched.threads;
+  int nt_bgk = 0, per_sm = 0;
+  CUDA_TRY(batch_max_ctas(b->storage, threads, b->small_index, &per_sm), "occupancy");
+  if (per_sm < 1) return fail(PLBM_E_UNSUPPORTED, "batched kernel does not fit on an SM with %d threads", threads);
   for (int pass = 0; pass < 2; pass++) {
     for (int i = 0; i < b->ngrids; i++) {
       const BatchGrid& g = b->grids[i];
       if ((g.kind == PLBM_BGK) != (pass == 0)) continue;
-      const int ty = b->sched.ty[bucket_of(g.ny)];
+      const int ty = sched.ty[bucket_of(g.ny)];
       for (int y0 = 0; y0 < g.ny;) {
         const int h = g.ny - y0 < 2 * ty ? g.ny - y0 : ty;
         const long long cells = (long long)g.nx * h;
@@ -106,26 +109,25 @@ int apply_schedule(plbm_batch_t* b) {
         y0 += h;
       }
     }
-    if (pass == 0) b->nt_bgk = (int)tiles.size();
+    if (pass == 0) nt_bgk = (int)tiles.size();
   }
-  b->ntiles = (int)tiles.size();
-  if ((size_t)b->ntiles > b->tile_cap) {
+  if (tiles.size() > b->tile_cap) {
+    BatchTile* table = nullptr;
+    CUDA_TRY(cudaMalloc(&table, sizeof(BatchTile) * tiles.size()), "cudaMalloc(tile table)");
     cudaFree(b->d_tiles);
-    b->d_tiles = nullptr;
-    b->tile_cap = 0;
-    CUDA_TRY(cudaMalloc(&b->d_tiles, sizeof(BatchTile) * tiles.size()), "cudaMalloc(tile table)");
+    b->d_tiles = table;
     b->tile_cap = tiles.size();
   }
+  drop_graphs(b);
+  b->sched = sched;
+  b->nt_bgk = nt_bgk;
+  b->ntiles = (int)tiles.size();
+  const int want = sched.ctas_per_sm > 0 ? std::min(sched.ctas_per_sm, per_sm) : per_sm;
+  b->ctas = std::max(1, std::min(b->ntiles, want * b->sms));
   CUDA_TRY(cudaMemcpy(b->d_grids, b->grids.data(), sizeof(BatchGrid) * b->ngrids, cudaMemcpyHostToDevice),
            "upload batch table");
   CUDA_TRY(cudaMemcpy(b->d_tiles, tiles.data(), sizeof(BatchTile) * tiles.size(), cudaMemcpyHostToDevice),
            "upload tile table");
-  int per_sm = 0;
-  CUDA_TRY(batch_max_ctas(b->storage, b->sched.threads, b->small_index, &per_sm), "occupancy");
-  if (per_sm < 1) return fail(PLBM_E_UNSUPPORTED, "batched kernel does not fit on an SM with %d threads", b->sched.threads);
-  const int want = b->sched.ctas_per_sm > 0 ? std::min(b->sched.ctas_per_sm, per_sm) : per_sm;
-  b->ctas = std::max(1, std::min(b->ntiles, want * b->sms));
-  drop_graphs(b);
   return PLBM_OK;
 }
 
@@ -240,7 +242,7 @@ extern "C" int plbm_batch_create(int ngrids, const int* nx, const int* ny, const
   }
   b->stream = b->own;
   plbm_batch_default_schedule(&b->sched);
-  if (int r = apply_schedule(b)) {
+  if (int r = apply_schedule(b, b->sched)) {
     plbm_batch_destroy(b);
     return r;
   }
@@ -277,8 +279,7 @@ extern "C" int plbm_batch_set_schedule(plbm_batch_t* b, const plbm_batch_schedul
   if (int r = check_schedule(*s)) return r;
   CUDA_TRY(cudaSetDevice(b->device), "cudaSetDevice");
   CUDA_TRY(cudaStreamSynchronize(b->stream), "synchronize");
-  b->sched = *s;
-  return apply_schedule(b);
+  return apply_schedule(b, *s);
 }
 
 extern "C" int plbm_batch_get_schedule(const plbm_batch_t* b, plbm_batch_schedule* s) {
@@ -303,7 +304,7 @@ extern "C" int plbm_batch_set_math(plbm_batch_t* b, int math) {
   CUDA_TRY(cudaSetDevice(b->device), "cudaSetDevice");
   CUDA_TRY(cudaStreamSynchronize(b->stream), "synchronize");
   b->math = math;
-  return apply_schedule(b);
+  return apply_schedule(b, b->sched);
 }
 
 extern "C" int plbm_batch_set_equilibrium(plbm_batch_t* b, int grid, const double* rho, const double* ux,
