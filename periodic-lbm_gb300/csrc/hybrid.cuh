@@ -433,14 +433,19 @@ DF_HD int64_t to_fixed_nonneg(double d, bool& bad) {
 // an error whose mean does not depend on the sign of h.  (Rounded toward zero,
 // h of the sign of c.u shrinks and |J| is damped by ~1e-16 per step, 2e-12 in u
 // over 10,000 plugin steps; rounded toward -infinity, one instruction pair
-// fewer, the error of one step is 1.4 times as large.)
+// fewer, the error of one step is 1.4 times as large.)  The half unit is a 32-bit one, so that
+// |h| < 2^-28 is rounded toward -infinity, unless NEAREST: then to the nearest as well, which costs
+// TRT and RR 1.1 to 2.4 % (641 x 500 10.95 -> 11.08 us per step and 12.82 -> 13.01) and shows in flows of
+// 1e-11 and less (40 x 36 vortex with noise of 1e-13, velocity after 400 steps: TRT 4.5e-4 off without and
+// 1.6e-4 with it, RR 5.8e-3 and 2.2e-4).  BGK takes such cells out of line instead (bgk_tiny; 1 %
+// rather than 1.9).
 PLBM_NOINLINE void load_fixed_slow(const double* f, int64_t* F) {
   bool b = false;  // stays false: the caller has checked the limits
   F[0] = to_fixed_nonneg<1022>(f[0], b);
   for (int q = 1; q < 5; q++) F[q] = to_fixed_nonneg<1020>(f[q], b);
   for (int q = 5; q < 9; q++) F[q] = to_fixed_nonneg<1019>(f[q], b);
 }
-template <bool SHIFTED>
+template <bool SHIFTED, bool NEAREST = false>
 DF_HD void load_fixed(const double (&f)[9], int64_t (&F)[9], bool& bad, bool& small) {
   bool odd = false;
 #pragma unroll
@@ -451,10 +456,14 @@ DF_HD void load_fixed(const double (&f)[9], int64_t (&F)[9], bool& bad, bool& sm
     if constexpr (SHIFTED) {
       const uint32_t e = (H >> 20) & 0x7FFu;
       odd |= e > (q == 0 ? 1021u : (q < 5 ? 1019u : 1018u));
-      const uint32_t rs = 1026u - e < 63u ? 1026u - e : 63u;
       const uint64_t n = ((((uint64_t)mh << 32) | L) << 10) ^ (uint64_t)((int64_t)u >> 63);
-      // (rs > 32, |h| < 2^-28: rounded toward -infinity)
-      F[q] = (int64_t)(n + (1u << ((rs - 1u) & 31u))) >> rs;
+      if constexpr (NEAREST) {
+        const uint32_t rs = 1025u - e < 63u ? 1025u - e : 63u;  // to half units
+        F[q] = (((int64_t)n >> rs) + 1) >> 1;
+      } else {
+        const uint32_t rs = 1026u - e < 63u ? 1026u - e : 63u;
+        F[q] = (int64_t)(n + (1u << ((rs - 1u) & 31u))) >> rs;
+      }
     } else {
       const uint32_t sh = (H >> 20) - 1016u;  // a set sign bit makes this large
       odd |= sh > (q == 0 ? 6u : (q < 5 ? 4u : 3u));
@@ -689,7 +698,7 @@ template <bool SHIFTED = false, bool QUICK = false>
 DF_HD void rr_fma(double (&f)[9], const RrParams& r, const BgkParams& p, bool& bad) {
   int64_t F[9], Y[9];
   bool small;
-  load_fixed<SHIFTED>(f, F, bad, small);
+  load_fixed<SHIFTED, SHIFTED>(f, F, bad, small);
   if (bad) return;
   rr_brackets<SHIFTED>(F, r, p, Y, bad);
   if constexpr (SHIFTED || !QUICK) {
@@ -817,7 +826,7 @@ template <bool SHIFTED = false, bool QUICK = false>
 DF_HD void trt_fma(double (&f)[9], const TrtFmaParams& p, bool& bad) {
   int64_t F[9], Y[9];
   bool small;
-  load_fixed<SHIFTED>(f, F, bad, small);
+  load_fixed<SHIFTED, SHIFTED>(f, F, bad, small);
   if (bad) return;
   trt_brackets(F, p, Y, bad);
   if constexpr (SHIFTED || !QUICK) {

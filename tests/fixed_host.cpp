@@ -23,3 +23,13 @@ extern "C" int fx_bgk_shifted(double* f, double omega) {
   for (int q = 0; q < 9; q++) f[q] = v[q];
   return bad;
 }
+// The nine shifted populations in units of 2^-59, as TRT and RR load them; 0 where one is out of range.
+extern "C" int fx_load_shifted(const double* f, int64_t* F) {
+  double v[9];
+  int64_t G[9];
+  bool bad = false, small;
+  for (int q = 0; q < 9; q++) v[q] = f[q];
+  hy::load_fixed<true, true>(v, G, bad, small);
+  for (int q = 0; q < 9; q++) F[q] = G[q];
+  return !bad;
+}

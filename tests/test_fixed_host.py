@@ -19,6 +19,7 @@ def lib(tmp_path_factory):
     h = ctypes.CDLL(str(so))
     h.fx_to_double.restype = ctypes.c_double
     h.fx_bgk_shifted.argtypes = [ctypes.c_void_p, ctypes.c_double]
+    h.fx_load_shifted.argtypes = [ctypes.c_void_p, ctypes.c_void_p]
     h.fx_to_double.argtypes = [ctypes.c_int64, ctypes.c_int]
     return h
 
@@ -88,3 +89,17 @@ def test_cells_at_rest_and_false_hints(lib):
     assert max(abs(Fr(float(x)) - y) for x, y in zip(a, want)) <= 2.0 ** -55
     h[3] = 0.2  # past the limit
     assert lib.fx_bgk_shifted(h.ctypes.data, 1.3) == 2
+
+
+@pytest.mark.parametrize("top", [-5, -20, -27, -28, -29, -45, -57, -58, -59, -60, -61, -62, -100, -1022])
+def test_shifted_load_rounds_to_nearest(lib, top):
+    """Every deviation that the fixed point takes, of either sign and of every size: within half a
+    unit of 2^-59, zeros of either sign zero."""
+    rng = np.random.default_rng(-top)
+    F = np.zeros(9, np.int64)
+    for _ in range(60):
+        h = np.ldexp(rng.choice([-1, 1], 9) * rng.uniform(0.5, 1.0, 9), top)
+        h[rng.integers(0, 9)] = rng.choice([0.0, -0.0])
+        assert lib.fx_load_shifted(h.ctypes.data, F.ctypes.data)
+        for q in range(9):
+            assert abs(Fr(float(h[q])) * 2 ** 59 - int(F[q])) <= Fr(1, 2), (q, h[q])
