@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(kBlock) k_stream_scheme(const double* __restri
 #pragma unroll
   for (int q = 1; q < 9; q++) {
     double v[9];
-    sch::gather<YFast>(src, q, x, y, xp, xm, yp, ym, nx, ny, ld, v);
+    sch::gather<YFast, false>(src, q, x, y, xp, xm, yp, ym, nx, ny, ld, v);
     dst[YFast::off(x, y, q, nx, ny, ld)] = sch::scheme_value(SCHEME, v, q, dt);
   }
 }
