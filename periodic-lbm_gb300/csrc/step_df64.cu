@@ -16,11 +16,11 @@ namespace {
 template <class S>
 __global__ void __launch_bounds__(kBlock) k_step_dev_df(const typename S::elem* __restrict__ src,
                                                        typename S::elem* __restrict__ dst, int nx, int ny, int ld,
-                                                       int ftiles, df::DfParams p) {
+                                                       Rows rows, df::DfParams p) {
   chain_begin();
-  const int x = blockIdx.x / ftiles;
-  const int y = (blockIdx.x - x * ftiles) * blockDim.x + threadIdx.x;
-  if (y >= ny) return;
+  int x, y;
+  flat_cell(rows, x, y);
+  if (x >= nx) return;
   df::df64 h[9];
 #pragma unroll
   for (int q = 0; q < 9; q++) {
@@ -104,11 +104,11 @@ __global__ void __launch_bounds__(kBlock) k_step_dev_comp(const typename S::elem
 template <class S, int KIND>
 __global__ void __launch_bounds__(kBlock) k_step_dev_d(const typename S::elem* __restrict__ src,
                                                       typename S::elem* __restrict__ dst, int nx, int ny, int ld,
-                                                      int ftiles, CollParams p) {
+                                                      Rows rows, CollParams p) {
   chain_begin();
-  const int x = blockIdx.x / ftiles;
-  const int y = (blockIdx.x - x * ftiles) * blockDim.x + threadIdx.x;
-  if (y >= ny) return;
+  int x, y;
+  flat_cell(rows, x, y);
+  if (x >= nx) return;
   double h[9];
 #pragma unroll
   for (int q = 0; q < 9; q++) {
@@ -128,10 +128,6 @@ df::df64 split_const(double d) {
 }  // namespace
 
 cudaError_t step_pull_dev_hi(int storage, int math, int kind, const Sweep& s, const CollParams& cp) {
-  const int ft = (s.ny + kBlock - 1) / kBlock;
-  const long long blocks = (long long)ft * s.nx;
-  if (blocks <= 0 || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-  const unsigned nb = (unsigned)blocks;
   if (math == 2) {  // compensated binary32
     if (kind != K_BGK) return cudaErrorNotSupported;
     const df::DevParams p = df::dev_params(cp.omega);
@@ -149,6 +145,11 @@ cudaError_t step_pull_dev_hi(int storage, int math, int kind, const Sweep& s, co
     return small ? step_cells<k_step_dev_comp<StoreF32Dev, uint32_t>>(s, s.ny, pairs, false, flat, p)
                  : step_cells<k_step_dev_comp<StoreF32Dev, size_t>>(s, s.ny, pairs, false, flat, p);
   }
+  // As the straight binary64 kernels, blocks by the grid's size and an even share for each SM.  Rows in
+  // chained blocks of 256: 300 x 257 strict BGK 50.6 us per binary16 step (42.2 with launches apart; 21.3 now),
+  // double-float 7.9 (6.4; 3.9); 513 x 700 strict BGK 106.8 and 95.3; rows that fill such blocks lose at
+  // most 0.4 us in double-float (256^2 3.6 and 3.9, 4.1 with launches apart) and gain elsewhere.
+  const bool flat = !rows_fit(s.ny, s.nx, true);
   if (math == 3) {  // double-float
     if (kind != K_BGK) return cudaErrorNotSupported;
     df::DfParams p;
@@ -159,38 +160,21 @@ cudaError_t step_pull_dev_hi(int storage, int math, int kind, const Sweep& s, co
     p.wd = split_const(WD);
     p.ws3 = split_const(3.0 * WS);
     p.wd3 = split_const(3.0 * WD);
-    if (storage == ST_F32DEV)
-      chained(k_step_dev_df<StoreF32Dev>, nb, kBlock, s.stream)(static_cast<const float*>(s.src),
-                                                              static_cast<float*>(s.dst), s.nx, s.ny, s.ld, ft, p);
-    else if (storage == ST_F16DEV)
-      chained(k_step_dev_df<StoreF16Dev>, nb, kBlock, s.stream)(static_cast<const __half*>(s.src),
-                                                              static_cast<__half*>(s.dst), s.nx, s.ny, s.ld, ft, p);
-    else
-      return cudaErrorInvalidValue;
-    return cudaGetLastError();
-  }
-#define PLBM_DEVD(S, E)                                                                                      \
-  switch (kind) {                                                                                            \
-    case K_BGK: chained(k_step_dev_d<S, K_BGK>, nb, kBlock, s.stream)(static_cast<const E*>(s.src),            \
-                                                                    static_cast<E*>(s.dst), s.nx, s.ny, s.ld, \
-                                                                    ft, cp); break;                           \
-    case K_TRT: chained(k_step_dev_d<S, K_TRT>, nb, kBlock, s.stream)(static_cast<const E*>(s.src),            \
-                                                                    static_cast<E*>(s.dst), s.nx, s.ny, s.ld, \
-                                                                    ft, cp); break;                           \
-    case K_RR: chained(k_step_dev_d<S, K_RR>, nb, kBlock, s.stream)(static_cast<const E*>(s.src),              \
-                                                                  static_cast<E*>(s.dst), s.nx, s.ny, s.ld,   \
-                                                                  ft, cp); break;                             \
-    default: return cudaErrorNotSupported;                                                                   \
-  }
-  if (storage == ST_F32DEV) {
-    PLBM_DEVD(StoreF32Dev, float)
-  } else if (storage == ST_F16DEV) {
-    PLBM_DEVD(StoreF16Dev, __half)
-  } else {
+    if (storage == ST_F32DEV) return step_cells<k_step_dev_df<StoreF32Dev>>(s, s.ny, s.nx, true, flat, p);
+    if (storage == ST_F16DEV) return step_cells<k_step_dev_df<StoreF16Dev>>(s, s.ny, s.nx, true, flat, p);
     return cudaErrorInvalidValue;
   }
+#define PLBM_DEVD(S)                                                                           \
+  switch (kind) {                                                                              \
+    case K_BGK: return step_cells<k_step_dev_d<S, K_BGK>>(s, s.ny, s.nx, true, flat, cp);      \
+    case K_TRT: return step_cells<k_step_dev_d<S, K_TRT>>(s, s.ny, s.nx, true, flat, cp);      \
+    case K_RR: return step_cells<k_step_dev_d<S, K_RR>>(s, s.ny, s.nx, true, flat, cp);        \
+    default: return cudaErrorNotSupported;                                                     \
+  }
+  if (storage == ST_F32DEV) PLBM_DEVD(StoreF32Dev)
+  if (storage == ST_F16DEV) PLBM_DEVD(StoreF16Dev)
 #undef PLBM_DEVD
-  return cudaGetLastError();
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace plbm

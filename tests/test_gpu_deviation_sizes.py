@@ -62,3 +62,16 @@ def test_either_side_of_the_line_against_binary64(gpu_lib, storage, math, nx, ny
     want = run(nx, ny, "f64", "strict", state, 12)
     store = (2.0 ** -24 if storage == "f32dev" else 2.0 ** -11) / 16
     assert np.max(np.abs(got - want)) <= 2 * 12 * (store + 4 * 2.0 ** -24 / 2)
+
+
+@pytest.mark.parametrize("storage,math", [("f32dev", "strict"), ("f16dev", "strict"), ("f32dev", "df64"), ("f16dev", "df64")])
+@pytest.mark.parametrize("nx,ny,cx,cy", [(1, 1, 3, 5), (5, 3, 7, 11), (3, 32, 17, 8), (10, 257, 30, 1), (31, 33, 33, 31)])
+def test_binary64_collisions_of_copies(gpu_lib, nx, ny, cx, cy, storage, math):
+    """Collisions in binary64 and double-float: a lattice of copies evolves as its copies bit for bit, in
+    blocks of every size, rows that fill them and rows that do not."""
+    rng = np.random.default_rng(nx + ny)
+    state = [1 + 0.01 * rng.standard_normal((nx, ny)), 0.05 * rng.standard_normal((nx, ny)),
+             0.05 * rng.standard_normal((nx, ny))]
+    small = run(nx, ny, storage, math, state, 6)
+    large = run(nx * cx, ny * cy, storage, math, [np.tile(s, (cx, cy)) for s in state], 6)
+    assert np.array_equal(large, np.tile(small, (1, cx, cy)))
